@@ -525,9 +525,11 @@ plk_status run_prune(plk_handle* h, int precision, void** store, cudaEvent_t* af
     }
     const size_t tsz = precision == PLK_FP64 ? sizeof(double) : sizeof(float);
     const size_t vec_bytes = (size_t)h->post.size() * h->C * h->n_sites * h->S * tsz;
-    const int blocks = (h->n_sites + 63) / 64;  // the smallest tile: 64 sites (prune4p, two threads per site)
+    const int any_blocks = prune_any_blocks(prune_args(h, precision), h->S, precision, store != nullptr);
+    // the smallest tile elsewhere: 64 sites (prune4p, two threads per site)
+    const int blocks = std::max((h->n_sites + 63) / 64, any_blocks);
     PLK_CUDA(h, h->d_site_lnl.ensure(sizeof(double) * h->n_sites), "allocate site lnL");
-    PLK_CUDA(h, h->d_block.ensure(sizeof(double) * 2 * blocks), "allocate block sums");
+    PLK_CUDA(h, h->d_block.ensure(sizeof(double) * 2 * (size_t)blocks), "allocate block sums");
     PLK_CUDA(h, h->d_lnl.ensure(sizeof(double)), "allocate lnL");
     // arrival counters, zero between launches: the grid's, then one per
     // 128-site tile (the 20-state compact form's in-kernel combine)
@@ -545,6 +547,7 @@ plk_status run_prune(plk_handle* h, int precision, void** store, cudaEvent_t* af
     a.paired_ready = (precision == PLK_FP32S && h->paired_written) ? 1 : 0;
     a.withhold_first_stage = (precision == PLK_FP32S && h->withhold_stage) ? 1 : 0;
     if (precision == PLK_FP32S) h->withhold_stage = false;
+    a.use_any = any_blocks > 0 ? 1 : 0;
     const bool fused = fused_kernel_applies(h, precision);
     std::vector<int> cands20;
     if (!store && precision == PLK_FP32S && h->S == 20)
@@ -562,6 +565,11 @@ plk_status run_prune(plk_handle* h, int precision, void** store, cudaEvent_t* af
             if (s != PLK_OK) return s;
         }
         a.variant = h->variant;
+    } else if (a.use_any) {
+        if (store) {
+            PLK_CUDA(h, h->d_cond.ensure(vec_bytes), "allocate node vectors");
+            a.cond = h->d_cond.p;
+        }
     } else if (!fused) {
         PLK_CUDA(h, h->d_work.ensure(vec_bytes), "allocate work vectors");
         a.work = h->d_work.p;

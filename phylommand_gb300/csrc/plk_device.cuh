@@ -191,57 +191,13 @@ __device__ __forceinline__ void store_site_record(double* bs, size_t slot, const
     reinterpret_cast<float4*>(bs)[slot] = make_float4(t.hi, t.lo, __int_as_float(t.ee), 0.0f);
 }
 
-// Compensated sum of the n (sum, compensation) pairs of bs by one CTA:
-// thread i folds pairs i, i + blockDim.x, ... (TwoSum), then the block
-// reduction of block_sum_pair; the result is valid in thread 0.  Loads go
-// through L2 so that pairs other CTAs of the same grid stored are seen.
-__device__ inline double cta_sum_pairs(const double* bs, int n) {
-    constexpr int U = 8;  // a thread's loads of one round, all in flight before the sums
-    double s = 0.0, c = 0.0;
-    for (int base = 0; base < n; base += U * (int)blockDim.x) {
-        double2 v[U];
-#pragma unroll
-        for (int q = 0; q < U; ++q) {
-            const int i = base + q * (int)blockDim.x + (int)threadIdx.x;
-            v[q] = i < n ? __ldcg(reinterpret_cast<const double2*>(bs) + i) : make_double2(0.0, 0.0);
-        }
-#pragma unroll
-        for (int q = 0; q < U; ++q) {
-            if (base + q * (int)blockDim.x + (int)threadIdx.x >= n) break;  // past the end: nothing to fold
-            double ns, e;
-            two_sum(s, v[q].x, ns, e);
-            s = ns;
-            c = c + v[q].y + e;
-        }
-    }
-    block_sum_pair(s, c);
-    return s + c;
-}
-
-// Epilogue of a 1-D grid whose CTAs each stored one pair at bs[2 blockIdx.x]
-// from thread 0: every CTA counts itself in with one atomicAdd after a fence,
-// and the CTA that arrives last sums all pairs in index order into *out and
-// re-arms the counter (zero between launches).  Nothing waits on another CTA.
-// Every thread of the CTA must call it, after thread 0's store.
-__device__ inline void finish_grid_sum(const double* bs, unsigned* counter, double* out) {
-    __shared__ int s_last;
-    if (threadIdx.x == 0) {
-        __threadfence();
-        s_last = atomicAdd(counter, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    const double t = cta_sum_pairs(bs, (int)gridDim.x);
-    if (threadIdx.x == 0) {
-        *out = t;
-        *counter = 0u;
-    }
-}
-
-// The same epilogue for grids whose CTAs each stored a SiteSum32 record
-// (store_site_record): the last CTA folds the records in index order with
-// FP32 TwoSum and integer sums and writes ee ln 2 + hi + lo as one FP64 value.
+// Epilogue of a 1-D grid whose CTAs each stored a SiteSum32 record
+// (store_site_record) from thread 0: every CTA counts itself in with one
+// atomicAdd after a fence, and the CTA that arrives last folds the records in
+// index order with FP32 TwoSum and integer sums, writes ee ln 2 + hi + lo as
+// one FP64 value into *out and re-arms the counter (zero between launches).
+// Nothing waits on another CTA.  Every thread of the CTA must call it, after
+// thread 0's store.
 __device__ inline void finish_grid_sum32(const double* bs, unsigned* counter, double* out) {
     __shared__ int s_last;
     if (threadIdx.x == 0) {
@@ -264,6 +220,108 @@ __device__ inline void finish_grid_sum32(const double* bs, unsigned* counter, do
     const SiteSum32 t = block_sum_site32f(a);
     if (threadIdx.x == 0) {
         *out = fma((double)t.ee, 0.69314718055994530942, (double)t.hi + (double)t.lo);
+        *counter = 0u;
+    }
+}
+
+// Sum of FP64 site log-likelihoods in integers.  A warp-wide FP64 instruction
+// occupies GB300's FP64 pipe for 16 cycles of its SM and a chain of TwoSum
+// shuffle steps waits on each, which put about 13 us at the end of a short
+// pass; integer adds do not.  A value x is split exactly into hi 2^-20 + lo
+// 2^-60 (hi, lo 64-bit; nothing of x is lost while |x| >= 2^-8, and 2^-61 at
+// most below), the parts are summed as integers, so the total is exact until
+// its one rounding at the end and does not depend on the order.  A value that
+// is not finite, or 2^40 and more, makes the sum NaN.
+struct SiteSum64 {
+    long long hi = 0, lo = 0;
+    int bad = 0;
+};
+
+__device__ __forceinline__ void site_sum64_add(SiteSum64& a, double x) {
+    if (!(fabs(x) < 1099511627776.0)) {
+        a.bad = 1;
+        return;
+    }
+    const long long h = __double2ll_rn(x * 1048576.0);
+    a.hi += h;
+    a.lo += __double2ll_rn(fma((double)h, -9.5367431640625e-07, x) * 1152921504606846976.0);
+}
+
+// carries lo beyond 40 bits into hi, leaving 0 <= lo < 2^40
+__device__ __forceinline__ void site_sum64_carry(SiteSum64& a) {
+    a.hi += a.lo >> 40;
+    a.lo &= (1ll << 40) - 1;
+}
+
+__device__ __forceinline__ void warp_sum_site64(SiteSum64& a) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        a.hi += __shfl_down_sync(0xffffffffu, a.hi, off);
+        a.lo += __shfl_down_sync(0xffffffffu, a.lo, off);
+    }
+    a.bad = __any_sync(0xffffffffu, a.bad);
+}
+
+// Block total, valid in thread 0.  All threads of the block must call it.
+__device__ inline SiteSum64 block_sum_site64(SiteSum64 a) {
+    __shared__ long long r_hi[32], r_lo[32];
+    __shared__ int r_bad[32];
+    warp_sum_site64(a);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __syncthreads();  // an earlier call may still be reading
+    if (lane == 0) {
+        r_hi[warp] = a.hi;
+        r_lo[warp] = a.lo;
+        r_bad[warp] = a.bad;
+    }
+    __syncthreads();
+    SiteSum64 t;
+    if (warp == 0) {
+        if (lane < (int)(blockDim.x >> 5)) {
+            t.hi = r_hi[lane];
+            t.lo = r_lo[lane];
+            t.bad = r_bad[lane];
+        }
+        warp_sum_site64(t);
+    }
+    return t;
+}
+
+// A block's record in the 16 bytes of its block-sum pair (hi = the smallest
+// 64-bit integer where the sum is not a number)
+__device__ __forceinline__ void store_site_record64(double* bs, size_t slot, SiteSum64 t) {
+    site_sum64_carry(t);
+    if (t.bad) t.hi = -0x7fffffffffffffffll - 1;
+    reinterpret_cast<longlong2*>(bs)[slot] = make_longlong2(t.hi, t.lo);
+}
+
+// finish_grid_sum32 for grids whose CTAs each stored such a record.
+__device__ inline void finish_grid_sum64(const double* bs, unsigned* counter, double* out) {
+    __shared__ int s_last64;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last64 = atomicAdd(counter, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last64) return;
+    __threadfence();
+    const longlong2* rec = reinterpret_cast<const longlong2*>(bs);
+    SiteSum64 a;
+    for (int i = (int)threadIdx.x; i < (int)gridDim.x; i += (int)blockDim.x) {
+        const longlong2 v = __ldcg(rec + i);
+        if (v.x == -0x7fffffffffffffffll - 1) a.bad = 1;
+        else a.hi += v.x;
+        a.lo += v.y;
+        site_sum64_carry(a);
+    }
+    SiteSum64 t = block_sum_site64(a);
+    if (threadIdx.x == 0) {
+        site_sum64_carry(t);
+        // hi may need more than 53 bits: its rounding error goes with lo
+        const double h = (double)t.hi;
+        const double rest = (double)(t.hi - (long long)h) * 9.5367431640625e-07 +
+                            (double)t.lo * 8.6736173798840355e-19;
+        *out = t.bad ? __longlong_as_double(0x7ff8000000000000ll) : h * 9.5367431640625e-07 + rest;
         *counter = 0u;
     }
 }

@@ -208,7 +208,7 @@ struct PruneArgs {
     const double* root_w;      // [S]
     const double* cat_w;       // [C]
     double* site_lnl;          // [n_sites]
-    double* block_sum;         // [2 * n_blocks] (sum, compensation)
+    double* block_sum;         // [2 * n_blocks] 16-byte records (store_site_record, store_site_record64)
     void* cond;                // T [n_int][C][n_sites][S] or null
     void* work;                // T scratch of the generic kernel [n_int][C][n_sites][S]
     // topology for the generic kernel (device arrays)
@@ -236,10 +236,11 @@ struct PruneArgs {
     // prune20v_kernel (three CTAs per SM), 7 = prune20v_kernel with split
     // BF16 products (kind::f16, FP32 accumulate).
     int variant;
+    int use_any;               // run prune_any_kernel (prune_any_blocks > 0)
     int n_nodes;
     void* scratch;             // kernel-specific scratch (prune20_scratch_bytes)
     // The last CTA of the kernel that stores the block sums adds them up into
-    // *lnl_out (finish_grid_sum), counting arrivals in *grid_done, which is
+    // *lnl_out (finish_grid_sum32 / 64), counting arrivals in *grid_done, which is
     // zero between launches; with grid_done null only the block sums and
     // per-site values are written.
     unsigned* grid_done;
@@ -313,6 +314,12 @@ cudaError_t launch_prune4w(const PruneArgs& a, int spt, int ts, int tps, int* n_
 // Staged 4-state FP32 kernel (plk_prune4s.cu): spt sites per thread.
 bool prune4s_fits(const PruneArgs& a, int spt);
 cudaError_t launch_prune4s(const PruneArgs& a, int spt, int* n_blocks, cudaStream_t st);
+// Any state count (plk_prune_any.cuh): a site over neighbouring lanes, P(t)
+// staged.  The number of blocks with which it takes this evaluation, 0 where
+// another kernel does (the tuned FP32 forms; 4 states once a thread per site
+// fills the chip; shapes whose matrices do not fit in shared memory).
+int prune_any_blocks(const PruneArgs& a, int S, int precision, bool store);
+cudaError_t launch_prune_any(const PruneArgs& a, int S, int precision, int* n_blocks, cudaStream_t st);
 // Chooses the kernel for (S, C, precision); returns the number of blocks used
 // for the partial sums in *n_blocks.
 cudaError_t launch_prune(const PruneArgs& a, int S, int precision, bool store, int* n_blocks,

@@ -11,9 +11,9 @@
 //                   per-thread shared-memory stack; per-site power-of-two
 //                   scaling; root reduction (src/simpleML.h:123-141) fused;
 //                   compensated block sums of the per-site lnL, added up by
-//                   the grid's last CTA (finish_grid_sum).
+//                   the grid's last CTA (finish_grid_sum32 / 64).
 //  prune_generic    the same pass for any state count (<= 24), vectors in a
-//                   global work buffer.
+//                   global work buffer (shapes prune_any_kernel does not fit).
 //  preorder_kernel  outside vectors from the root down and normalised
 //                   marginal posteriors (absent in the reference).
 #include <cstdio>
@@ -500,44 +500,17 @@ __global__ void __launch_bounds__(kPruneThreads) prune4_kernel(PruneArgs a) {
                 }
             }
         const double lnl = valid ? log(lsum) + (double)scale_e * 0.69314718055994530942 : 0.0;
-        if (valid) a.site_lnl[site] = lnl;
-        // ---- compensated block reduction
-        double s = valid ? lnl : 0.0, c = 0.0;
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const double os = __shfl_down_sync(0xffffffffu, s, off);
-            const double oc = __shfl_down_sync(0xffffffffu, c, off);
-            double ns, e;
-            two_sum(s, os, ns, e);
-            s = ns;
-            c = c + oc + e;
+        SiteSum64 sum;
+        if (valid) {
+            a.site_lnl[site] = lnl;
+            site_sum64_add(sum, lnl);
         }
-        __shared__ double red_s[32], red_c[32];
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        if (lane == 0) { red_s[warp] = s; red_c[warp] = c; }
-        __syncthreads();
-        if (warp == 0) {
-            const int nw = blockDim.x >> 5;
-            s = lane < nw ? red_s[lane] : 0.0;
-            c = lane < nw ? red_c[lane] : 0.0;
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                const double os = __shfl_down_sync(0xffffffffu, s, off);
-                const double oc = __shfl_down_sync(0xffffffffu, c, off);
-                double ns, e;
-                two_sum(s, os, ns, e);
-                s = ns;
-                c = c + oc + e;
-            }
-            if (lane == 0) {
-                a.block_sum[2 * blockIdx.x] = s;
-                a.block_sum[2 * blockIdx.x + 1] = c;
-            }
-        }
+        const SiteSum64 bsum = block_sum_site64(sum);
+        if (threadIdx.x == 0) store_site_record64(a.block_sum, blockIdx.x, bsum);
     }
-    if (a.grid_done) {  // FP32: SiteSum32 records; FP64: compensated pairs
+    if (a.grid_done) {  // SiteSum32 records in FP32, SiteSum64 records in FP64
         if constexpr (std::is_same<T, float>::value) finish_grid_sum32(a.block_sum, a.grid_done, a.lnl_out);
-        else finish_grid_sum(a.block_sum, a.grid_done, a.lnl_out);
+        else finish_grid_sum64(a.block_sum, a.grid_done, a.lnl_out);
     }
 }
 
@@ -623,7 +596,7 @@ __global__ void __launch_bounds__(kPruneThreads) prune_generic_kernel(GenericArg
             scale_e += e;
         }
     }
-    double lnl = 0.0;
+    SiteSum64 sum;
     if (valid) {
         const int r = g.n_int - 1;
         double lsum = 0.0;
@@ -640,40 +613,13 @@ __global__ void __launch_bounds__(kPruneThreads) prune_generic_kernel(GenericArg
                 lsum = fma(a.cat_w[k], lk, lsum);
             }
         }
-        lnl = log(lsum) + (double)scale_e * 0.69314718055994530942;
+        const double lnl = log(lsum) + (double)scale_e * 0.69314718055994530942;
         a.site_lnl[site] = lnl;
+        site_sum64_add(sum, lnl);
     }
-    double s = lnl, c = 0.0;
-    for (int off = 16; off > 0; off >>= 1) {
-        const double os = __shfl_down_sync(0xffffffffu, s, off);
-        const double oc = __shfl_down_sync(0xffffffffu, c, off);
-        double ns, e;
-        two_sum(s, os, ns, e);
-        s = ns;
-        c = c + oc + e;
-    }
-    __shared__ double red_s[32], red_c[32];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) { red_s[warp] = s; red_c[warp] = c; }
-    __syncthreads();
-    if (warp == 0) {
-        const int nw = blockDim.x >> 5;
-        s = lane < nw ? red_s[lane] : 0.0;
-        c = lane < nw ? red_c[lane] : 0.0;
-        for (int off = 16; off > 0; off >>= 1) {
-            const double os = __shfl_down_sync(0xffffffffu, s, off);
-            const double oc = __shfl_down_sync(0xffffffffu, c, off);
-            double ns, e;
-            two_sum(s, os, ns, e);
-            s = ns;
-            c = c + oc + e;
-        }
-        if (lane == 0) {
-            a.block_sum[2 * blockIdx.x] = s;
-            a.block_sum[2 * blockIdx.x + 1] = c;
-        }
-    }
-    if (a.grid_done) finish_grid_sum(a.block_sum, a.grid_done, a.lnl_out);
+    const SiteSum64 bsum = block_sum_site64(sum);
+    if (threadIdx.x == 0) store_site_record64(a.block_sum, blockIdx.x, bsum);
+    if (a.grid_done) finish_grid_sum64(a.block_sum, a.grid_done, a.lnl_out);
 }
 
 }  // namespace
@@ -704,6 +650,7 @@ cudaError_t launch_prune(const PruneArgs& a, int S, int precision, bool store, i
     const int blocks = (a.n_sites + kPruneThreads - 1) / kPruneThreads;
     *n_blocks = blocks;
     const bool fp64 = precision == PLK_FP64;
+    if (a.use_any) return launch_prune_any(a, S, precision, n_blocks, st);
     if (!fp64 && !store && S == 4 && a.C <= 8 && (a.variant == 1 || a.variant == 2) && prune4s_fits(a, a.variant))
         return launch_prune4s(a, a.variant, n_blocks, st);
     if (!fp64 && !store && S == 4 && a.variant >= 3 && a.variant <= 6 && prune4p_fits(a, (a.variant + 1) % 2 + 1))

@@ -1,0 +1,112 @@
+// Plan and dispatch of prune_any_kernel (plk_prune_any.cuh).
+#include "plk_prune_any.cuh"
+
+#include <algorithm>
+#include <atomic>
+
+namespace plk {
+
+namespace {
+
+constexpr size_t kAnySmem = 227 * 1024;
+constexpr int kAnyWarps = 8;  // per CTA at most
+
+int any_sm_count() {
+    static std::atomic<int> n{0};
+    int v = n.load();
+    if (v > 0) return v;
+    int dev = 0, c = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || c <= 0)
+        c = 152;
+    n.store(c);
+    return c;
+}
+
+struct AnyPlan {
+    dev::AnyLaunch launch{};
+    int H = 0, blocks = 0;
+    double cost = 0.0;  // estimated cycles of one op on the fullest SM
+};
+
+// H, warps per CTA and the tables' place for these counts; H = 0 where
+// nothing fits.
+AnyPlan any_plan(const PruneArgs& a, int S, bool fp64, int sms) {
+    AnyPlan best;
+    const int tsz = fp64 ? 8 : 4, C = a.C;
+    for (int H = 1; H <= 4; H *= 2) {
+        if (C * H > 32 || H > S || (H == 1 && S > 8)) continue;
+        const int R = (S + H - 1) / H, W = 32 / (C * H);
+        const long long warps = ((long long)a.n_sites + W - 1) / W;
+        const int per_sm = (int)((warps + sms - 1) / sms);
+        AnyPlan p;
+        p.H = H;
+        p.launch.depth = std::max(a.max_depth, 1);
+        // tip tables through the ring while they are of the size of P(t)
+        p.launch.stage_tips = a.n_codes <= 2 * S + 8 ? 1 : 0;
+        const int child = std::max(C * S * S, p.launch.stage_tips ? C * a.n_codes * S : 0);
+        p.launch.child_elems = (child * tsz + 15) / 16 * 16 / tsz;
+        // one CTA per SM while eight warps hold its sites: a table brought in
+        // once then serves every warp of the SM
+        const int want = std::max(1, std::min(kAnyWarps, per_sm));
+        bool fits = false;
+        // all tables resident (up to 8 states) while one CTA an SM is all
+        // there is to run, or two fit; else the ring
+        p.launch.slots = 0;
+        p.launch.warps = want;
+        if (S <= 8) {
+            const size_t need = dev::any_smem(S, H, fp64, p.launch, a);
+            fits = need <= (per_sm <= kAnyWarps ? kAnySmem : kAnySmem / 2);
+        }
+        for (int slots = 3; slots >= 2 && !fits; --slots)
+            for (int w = want; w >= 1 && !fits; --w) {
+                if (slots == 3 && w < (want + 1) / 2) break;  // rather two slots than half the warps
+                p.launch.slots = slots;
+                p.launch.warps = w;
+                fits = dev::any_smem(S, H, fp64, p.launch, a) <= kAnySmem;
+            }
+        if (!fits) continue;
+        // FP64: the SM's FP64 pipe takes 16 cycles a warp instruction; FP32:
+        // four schedulers; either against the latency of one warp's op
+        p.cost = fp64 ? std::max(16.0 * per_sm * R * 2 * S, 300.0 + 16.0 * R * 2 * S)
+                      : std::max((per_sm + 3) / 4 * (1.5 * R * S + 100.0), 200.0 + 2.0 * R * S + 5.0 * S);
+        p.blocks = (int)((warps + p.launch.warps - 1) / p.launch.warps);
+        if (best.H == 0 || p.cost < best.cost) best = p;
+    }
+    return best;
+}
+
+}  // namespace
+
+int prune_any_blocks(const PruneArgs& a, int S, int precision, bool store) {
+    const bool fp64 = precision == PLK_FP64;
+    if (S < 2 || S > kMaxStates || a.C > kMaxCats || a.n_ops < 1) return 0;
+    if (!fp64 && !store && ((S == 4 && a.C <= 8) || S == 20)) return 0;  // the tuned FP32 forms
+    const int sms = any_sm_count();
+    const AnyPlan p = any_plan(a, S, fp64, sms);
+    if (p.H == 0) return 0;
+    if (S == 4 && a.C <= 8) {
+        // prune4_kernel, a thread per site in 128-thread CTAs, issues the same
+        // FP64 instructions (32 per category and op) with less around them: it
+        // stays once its CTAs fill the SMs as evenly
+        const long long blocks = (a.n_sites + 127) / 128;
+        const double per_op = fp64 ? 16.0 * 32 * a.C : 0.25 * 1.5 * 64 * a.C;
+        const double cost4 = (double)((blocks + sms - 1) / sms) * 4 * per_op;
+        if (p.cost > 0.9 * cost4) return 0;
+    }
+    return p.blocks;
+}
+
+cudaError_t launch_prune_any(const PruneArgs& a, int S, int precision, int* n_blocks, cudaStream_t st) {
+    const bool fp64 = precision == PLK_FP64;
+    const AnyPlan p = any_plan(a, S, fp64, any_sm_count());
+    if (p.H == 0) return cudaErrorInvalidConfiguration;
+    *n_blocks = p.blocks;
+    if (fp64)
+        return S <= 12 ? launch_any64_lo(a, S, p.H, p.launch, p.blocks, st)
+                       : launch_any64_hi(a, S, p.H, p.launch, p.blocks, st);
+    return S <= 12 ? launch_any32_lo(a, S, p.H, p.launch, p.blocks, st)
+                   : launch_any32_hi(a, S, p.H, p.launch, p.blocks, st);
+}
+
+}  // namespace plk
