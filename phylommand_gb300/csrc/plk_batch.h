@@ -18,22 +18,11 @@ struct BatchItemDev {
     int tip_off;          // into tip32 ([tip_off + t][C][16][4])
     int n_tips, n_sites, site_stride;
     int model_off;        // doubles into model: lam[4] L[16] R[16] root_w[4] cat_rate[C] cat_w[C]
-    int moves_off, n_moves;  // into moves (NNI rearrangements of this tree)
-    int move_out_off;     // into the NNI output
+    int n_moves, move_out_off;  // NNI rearrangements of this tree, into the NNI output
     int n_int;            // internal nodes (the root is n_tips + n_int - 1)
-    int pad[2];
+    int pad[3];
 };
 static_assert(sizeof(BatchItemDev) == 64, "BatchItemDev is 64 bytes");
-
-// One NNI rearrangement of an item's tree (local node ids).
-//   kind 0: parent u is not the root; the new v' joins children x and y of the
-//           old tree, and the new u' joins v' with z (u's outside vector stays).
-//   kind 1: v and c are the root's children; v' joins x and y, c' joins p and q.
-struct NniMoveDev {
-    int kind, v, u, c;
-    int x, y, z, p;
-    int q, pad0, pad1, pad2;
-};
 
 struct BatchDev {
     int n_items, n_units, n_nodes_total, C;
@@ -56,17 +45,17 @@ struct BatchDev {
     const int* item_units;    // units of each item in site order
     double* lnl;              // [n_items]
     int* counter;             // work-queue head, zeroed before each launch
-    // NNI
-    const NniMoveDev* moves;
-    const long long* unit_move_off;  // [n_units] offset of each unit's per-move partials
-    double* unit_move_sums;          // [sum over units of n_moves][2]: 16-byte SiteSum32 records (store_site_record)
-    double* nni_out;                 // [sum over items of n_moves]
-    const int* move_item;            // [total moves] item of each output move
-    int total_moves, scratch_int;    // scratch_int: max internal nodes of any item
-    float4* scr_D;                   // per CTA: [scratch_int][C][128]
-    int* scr_ED;                     // per CTA: [scratch_int][128]
-    float4* scr_O;
-    int* scr_EO;
+    // NNI scoring and branch-length derivatives (plk_nni.cu)
+    float* Pn;                // [n_nodes_total][KP][j][i][2], KP = ceil(C / 2)
+    float* tipn;              // [n_tips_total][KP][code][i][2]
+    const int4* kids;         // [internal nodes of all items] (left, right, first move or -1, 0), local ids
+    float4* records;          // per item [warp tile][move or edge slot]: (hi, lo, exponent, -) or (d1 hi, lo, d2 hi, lo)
+    const long long* rec_off; // [n_items] into records
+    const int2* reduce_blocks;// (item, first output) of every CTA of the fold
+    double* nni_out;          // [sum over items of n_moves]
+    int scratch_int, pad3;    // max internal nodes of any item
+    float4* scr;              // per warp: messages, then outside vectors, [2 scratch_int][32 lanes][2]
+    int* scr_e;               // per warp: their exponents [2 scratch_int][sites of a warp]
 };
 
 inline int batch_model_stride(int C) { return 40 + 2 * C; }
@@ -86,30 +75,28 @@ cudaError_t launch_batch_pmat(const BatchDev& b, cudaStream_t st);
 cudaError_t launch_batch_prune(const BatchDev& b, const BatchForm& f, int grid, size_t smem, cudaStream_t st);
 cudaError_t launch_batch_reduce(const BatchDev& b, cudaStream_t st);
 
-// NNI scoring (plk_nni.cu): one tile per work unit, grid CTAs with their own
-// scratch slices; then the per-(item, move) reduction.
-size_t nni_smem_bytes(int C, bool codes_smem, int max_ops, int max_tips, int max_depth);
-cudaError_t launch_batch_nni(const BatchDev& b, bool codes_smem, int grid, size_t smem, cudaStream_t st);
-// resident CTAs per SM of the NNI (blen = false) or branch-length kernel
-int nni_occupancy(int C, bool codes_smem, size_t smem, bool blen);
-cudaError_t launch_batch_nni_reduce(const BatchDev& b, cudaStream_t st);
-
-// Branch-length derivatives of every edge of every item (plk_nni.cu): per
-// work unit the sums over its sites of d lnL / dt and d2 lnL / dt2 for each
-// edge slot (slot i = child i % 2 of internal node n_tips + i / 2), then per
-// item over its units in site order.  Same units, scratch and shared memory
-// as the NNI kernel.
+// NNI scoring and branch-length derivatives (plk_nni.cu): work units of `warps`
+// warps of down_sites_per_warp sites; the tables of an item in shared memory
+// (in_smem) or read through L1.  The edge slots of an item: slot i = child
+// i % 2 of internal node n_tips + i / 2.
 struct BlenDev {
-    const long long* unit_edge_off;  // [n_units] first slot of each unit in unit_edge_sums
-    double* unit_edge_sums;          // [slots][2]
-    const int* item_edge_off;        // [n_items] first global slot of each item
-    const int* edge_item;            // [total_slots]
-    int total_slots;
-    double* edge_out;                // [total_slots][2] (d1, d2)
+    float* ex;                 // [n_nodes_total][KP][m][2] exp(rho_km t), or null (NNI)
+    const int* item_edge_off;  // [n_items] first slot of each item
+    double* edge_out;          // [total slots][2] (d1, d2)
 };
-cudaError_t launch_batch_blen(const BatchDev& b, const BlenDev& bd, bool codes_smem, int grid, size_t smem,
-                              cudaStream_t st);
-cudaError_t launch_batch_blen_reduce(const BatchDev& b, const BlenDev& bd, cudaStream_t st);
+struct DownSize {              // warps per CTA; the largest item whose tables sit in shared memory
+    int warps = 0, nodes = 0, tips = 0, ints = 0;
+};
+constexpr int kDownWarps = 12;  // per CTA at most
+int down_sites_per_warp(int C);
+int down_smem_bytes(int C, bool blen, bool in_smem, const DownSize& z);
+// resident CTAs per SM
+int down_occupancy(int C, bool blen, bool in_smem, const DownSize& z);
+cudaError_t launch_down_tables(const BatchDev& b, const BlenDev& bd, cudaStream_t st);
+// units [unit0, unit1) on `grid` CTAs (the work-queue head zeroed before)
+cudaError_t launch_down(const BatchDev& b, const BlenDev& bd, bool blen, bool in_smem, const DownSize& z, int unit0,
+                        int unit1, int grid, cudaStream_t st);
+cudaError_t launch_down_reduce(const BatchDev& b, const BlenDev& bd, bool blen, int blocks, cudaStream_t st);
 
 // Summary statistics of every item (plk_features.cu): out[n_items][43].
 constexpr int kNumFeatures = 43;

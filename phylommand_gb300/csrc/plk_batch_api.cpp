@@ -52,20 +52,33 @@ struct ItemHost {
     Program prog;
     std::vector<double> t_eff;     // by internal id
     std::vector<int2> child;       // by internal id
+    std::vector<int> first_move;   // by post-order rank: the first NNI move across the edge above, or -1
     std::vector<uint8_t> codes;    // [n_tips][stride]
     std::vector<double> model;     // lam L R root_w cat_rate cat_w
-    std::vector<NniMoveDev> moves; // internal ids
-    std::vector<int> move_report;  // (caller's node id, which) per move
+    std::vector<int> move_report;  // (caller's node id, which) per NNI move
     std::vector<int> caller_id;    // caller's node id of every internal id
     bool has_model = false;
+    int n_moves() const { return (int)move_report.size() / 2; }
 };
 
 // Work units of one tile size plus their per-item index.
 struct UnitSet {
-    BBuf units, ptr, idx, sums, move_off;
+    BBuf units, ptr, idx, sums;
     int n_units = 0;
     int spt = 0;
-    std::vector<int2> host_units;
+};
+
+// Plan of NNI scoring or of the branch-length derivatives (plk_nni.cu) for
+// the current layout: warps per CTA, the units whose item's tables do not fit
+// in shared memory first, the records and the CTAs that fold them.
+struct DownPlan {
+    bool ready = false;
+    int n_units = 0, n_far = 0;  // units [0, n_far) read their tables through L1
+    DownSize size;
+    int grid_far = 0, grid_near = 0, n_blocks = 0, total_out = 0;
+    size_t n_records = 0;
+    std::vector<int> out_off;                   // first output of every item
+    BBuf units, rec_off, blocks, d_out_off;
 };
 
 constexpr int kThreads = 128;
@@ -83,13 +96,15 @@ struct plk_batch {
     // device layout
     BBuf d_items, d_codes, d_ops, d_teff, d_node_item, d_child, d_model, d_P32, d_tip32, d_lnl, d_counter;
     BBuf d_P32p, d_tip32p;  // paired layouts (C = 2, 4, 8)
-    BBuf d_moves, d_move_item, d_nni_out, d_unit_move_sums, d_scr_D, d_scr_ED, d_scr_O, d_scr_EO;
-    BBuf d_blen_ueo, d_blen_ues, d_blen_ieo, d_blen_ei, d_blen_out;  // branch-length derivative slots
+    // NNI scoring and branch-length derivatives
+    BBuf d_kids, d_Pn, d_tipn, d_records, d_nni_out, d_scr, d_scr_e;
+    BBuf d_blen_out, d_blen_ex;
     double* h_model = nullptr;  // pinned staging of the models
     double* h_lnl = nullptr;    // pinned lnL download
     size_t h_model_n = 0, h_lnl_n = 0;
-    int n_nodes_total = 0, max_ops = 0, max_tips = 0, max_depth = 0, max_int = 0, total_moves = 0;
-    UnitSet lnl_units, nni_units;
+    int n_nodes_total = 0, max_ops = 0, max_tips = 0, max_depth = 0, max_int = 0, total_moves = 0, tips_total = 0;
+    UnitSet lnl_units;
+    DownPlan nni_plan, blen_plan;
     // tuning of the lnL kernel
     BatchForm form;
     int grid = 0;
@@ -156,17 +171,6 @@ BatchDev device_view(plk_batch* b, const UnitSet& us) {
     d.item_units = us.idx.as<int>();
     d.lnl = b->d_lnl.as<double>();
     d.counter = b->d_counter.as<int>();
-    d.moves = b->d_moves.as<NniMoveDev>();
-    d.unit_move_off = us.move_off.as<long long>();
-    d.unit_move_sums = b->d_unit_move_sums.as<double>();
-    d.nni_out = b->d_nni_out.as<double>();
-    d.move_item = b->d_move_item.as<int>();
-    d.total_moves = b->total_moves;
-    d.scratch_int = b->max_int;
-    d.scr_D = b->d_scr_D.as<float4>();
-    d.scr_ED = b->d_scr_ED.as<int>();
-    d.scr_O = b->d_scr_O.as<float4>();
-    d.scr_EO = b->d_scr_EO.as<int>();
     return d;
 }
 
@@ -185,7 +189,7 @@ BatchDev lnl_view(plk_batch* b, const BatchForm* form) {
 
 // Work units for tiles of 128 * spt sites: items with the longest op lists
 // first, so the persistent grid ends on the cheapest units.
-plk_status build_units(plk_batch* b, UnitSet& us, int spt, bool with_moves) {
+plk_status build_units(plk_batch* b, UnitSet& us, int spt) {
     const int tile = kThreads * spt;
     std::vector<int> order(b->items.size());
     std::iota(order.begin(), order.end(), 0);
@@ -215,21 +219,7 @@ plk_status build_units(plk_batch* b, UnitSet& us, int spt, bool with_moves) {
     PLK_BCUDA(b, cudaMemcpy(us.ptr.p, ptr.data(), ptr.size() * sizeof(int), cudaMemcpyHostToDevice), "upload units");
     if (!idx.empty())
         PLK_BCUDA(b, cudaMemcpy(us.idx.p, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice), "upload units");
-    if (with_moves) {
-        std::vector<long long> off(units.size());
-        long long tot = 0;
-        for (size_t u = 0; u < units.size(); ++u) {
-            off[u] = tot;
-            tot += (long long)b->items[units[u].x].moves.size();
-        }
-        PLK_BCUDA(b, us.move_off.ensure(std::max<size_t>(off.size(), 1) * sizeof(long long)), "allocate move offsets");
-        PLK_BCUDA(b, cudaMemcpy(us.move_off.p, off.data(), off.size() * sizeof(long long), cudaMemcpyHostToDevice),
-                  "upload move offsets");
-        PLK_BCUDA(b, b->d_unit_move_sums.ensure((size_t)std::max<long long>(tot, 1) * 2 * sizeof(double)),
-                  "allocate move partial sums");
-    }
     us.spt = spt;
-    us.host_units = units;
     return PLK_OK;
 }
 
@@ -239,10 +229,9 @@ plk_status build_layout(plk_batch* b) {
     std::vector<Op> ops;
     std::vector<double> teff;
     std::vector<int2> node_item, child;
-    std::vector<NniMoveDev> moves;
-    std::vector<int> move_item;
+    std::vector<int4> kids;
     size_t codes_bytes = 0;
-    int tips_total = 0;
+    int tips_total = 0, total_moves = 0;
     b->max_ops = b->max_tips = b->max_depth = b->max_int = 0;
     for (size_t i = 0; i < b->items.size(); ++i) {
         const ItemHost& h = b->items[i];
@@ -257,17 +246,19 @@ plk_status build_layout(plk_batch* b) {
         d.n_sites = h.n_sites;
         d.site_stride = code_stride(h.n_sites);
         d.model_off = (int)i * batch_model_stride(C);
-        d.moves_off = (int)moves.size();
-        d.n_moves = (int)h.moves.size();
-        d.move_out_off = (int)moves.size();
+        d.n_moves = h.n_moves();
+        d.move_out_off = total_moves;
         d.n_int = h.n_int;
         codes_bytes += h.codes.size();
         ops.insert(ops.end(), h.prog.ops.begin(), h.prog.ops.end());
         teff.insert(teff.end(), h.t_eff.begin(), h.t_eff.end());
         child.insert(child.end(), h.child.begin(), h.child.end());
         for (int v = 0; v < h.n_nodes; ++v) node_item.push_back(make_int2((int)i, v));
-        moves.insert(moves.end(), h.moves.begin(), h.moves.end());
-        for (size_t m = 0; m < h.moves.size(); ++m) move_item.push_back((int)i);
+        for (int r = 0; r < h.n_int; ++r) {
+            const int2 ch = h.child[h.n_tips + r];
+            kids.push_back(make_int4(ch.x, ch.y, h.first_move[r], 0));
+        }
+        total_moves += h.n_moves();
         tips_total += h.n_tips;
         b->max_ops = std::max(b->max_ops, d.n_ops);
         b->max_tips = std::max(b->max_tips, h.n_tips);
@@ -275,7 +266,8 @@ plk_status build_layout(plk_batch* b) {
         b->max_int = std::max(b->max_int, h.n_int);
     }
     b->n_nodes_total = (int)teff.size();
-    b->total_moves = (int)moves.size();
+    b->total_moves = total_moves;
+    b->tips_total = tips_total;
     PLK_BCUDA(b, b->d_items.ensure(it.size() * sizeof(BatchItemDev)), "allocate batch table");
     PLK_BCUDA(b, b->d_codes.ensure(codes_bytes), "allocate tip codes");
     PLK_BCUDA(b, b->d_ops.ensure(ops.size() * sizeof(Op)), "allocate programs");
@@ -291,9 +283,7 @@ plk_status build_layout(plk_batch* b) {
     }
     PLK_BCUDA(b, b->d_lnl.ensure(it.size() * sizeof(double)), "allocate lnL");
     PLK_BCUDA(b, b->d_counter.ensure(sizeof(int)), "allocate counter");
-    PLK_BCUDA(b, b->d_moves.ensure(std::max<size_t>(moves.size(), 1) * sizeof(NniMoveDev)), "allocate moves");
-    PLK_BCUDA(b, b->d_move_item.ensure(std::max<size_t>(move_item.size(), 1) * sizeof(int)), "allocate moves");
-    PLK_BCUDA(b, b->d_nni_out.ensure(std::max<size_t>(moves.size(), 1) * sizeof(double)), "allocate NNI output");
+    PLK_BCUDA(b, b->d_kids.ensure(kids.size() * sizeof(int4)), "allocate node table");
     PLK_BCUDA(b, cudaMemcpy(b->d_items.p, it.data(), it.size() * sizeof(BatchItemDev), cudaMemcpyHostToDevice), "upload table");
     size_t off = 0;
     for (const ItemHost& h : b->items) {
@@ -307,12 +297,8 @@ plk_status build_layout(plk_batch* b) {
               "upload node map");
     PLK_BCUDA(b, cudaMemcpy(b->d_child.p, child.data(), child.size() * sizeof(int2), cudaMemcpyHostToDevice),
               "upload child table");
-    if (!moves.empty()) {
-        PLK_BCUDA(b, cudaMemcpy(b->d_moves.p, moves.data(), moves.size() * sizeof(NniMoveDev), cudaMemcpyHostToDevice),
-                  "upload moves");
-        PLK_BCUDA(b, cudaMemcpy(b->d_move_item.p, move_item.data(), move_item.size() * sizeof(int), cudaMemcpyHostToDevice),
-                  "upload moves");
-    }
+    PLK_BCUDA(b, cudaMemcpy(b->d_kids.p, kids.data(), kids.size() * sizeof(int4), cudaMemcpyHostToDevice),
+              "upload node table");
     const size_t mn = it.size() * batch_model_stride(C);
     if (mn > b->h_model_n) {
         if (b->h_model) cudaFreeHost(b->h_model);
@@ -320,7 +306,7 @@ plk_status build_layout(plk_batch* b) {
         PLK_BCUDA(b, cudaMallocHost(&b->h_model, mn * sizeof(double)), "allocate pinned models");
         b->h_model_n = mn;
     }
-    const size_t ln = std::max(it.size(), moves.size());
+    const size_t ln = std::max(it.size(), (size_t)total_moves);
     if (ln > b->h_lnl_n) {
         if (b->h_lnl) cudaFreeHost(b->h_lnl);
         b->h_lnl = nullptr;
@@ -332,7 +318,7 @@ plk_status build_layout(plk_batch* b) {
         b->exec = nullptr;
     }
     b->lnl_units.spt = 0;
-    b->nni_units.spt = 0;
+    b->nni_plan.ready = b->blen_plan.ready = false;
     b->tuned = false;
     b->layout_dirty = false;
     return PLK_OK;
@@ -390,7 +376,7 @@ plk_status tune(plk_batch* b) {
         const int occ = batch_occupancy(b->C, f, smem);
         if (occ < 1) continue;
         if (b->lnl_units.spt != f.spt) {
-            plk_status s = build_units(b, b->lnl_units, f.spt, false);
+            plk_status s = build_units(b, b->lnl_units, f.spt);
             if (s != PLK_OK) return s;
         }
         const BatchDev d = lnl_view(b, nullptr);
@@ -423,7 +409,7 @@ plk_status tune(plk_batch* b) {
     b->smem = best_smem;
     b->tuned_ms = best / 2.0;
     if (b->lnl_units.spt != best_form.spt) {
-        plk_status s = build_units(b, b->lnl_units, best_form.spt, false);
+        plk_status s = build_units(b, b->lnl_units, best_form.spt);
         if (s != PLK_OK) return s;
     }
     b->tuned = true;
@@ -511,12 +497,10 @@ void relabel_and_enumerate(int n_tips, int n_nodes, const int* left, const int* 
     }
     h->caller_id = oid;
     auto binary = [&](int v) { return v >= n_tips && (*L2)[v] >= 0 && (*R2)[v] >= 0; };
-    h->moves.clear();
     h->move_report.clear();
-    auto add = [&](int kind, int which, int v, int u, int c, int x, int y, int z, int p, int q) {
-        NniMoveDev m{};
-        m.kind = kind; m.v = v; m.u = u; m.c = c; m.x = x; m.y = y; m.z = z; m.p = p; m.q = q;
-        h->moves.push_back(m);
+    h->first_move.assign(n_nodes - n_tips, -1);
+    auto add = [&](int which, int v) {
+        if (h->first_move[v - n_tips] < 0) h->first_move[v - n_tips] = (int)h->move_report.size() / 2;
         h->move_report.push_back(oid[v]);
         h->move_report.push_back(which);
     };
@@ -525,14 +509,13 @@ void relabel_and_enumerate(int n_tips, int n_nodes, const int* left, const int* 
         const int u = parent[v];
         if (!binary(u)) continue;
         const int c = (*L2)[u] == v ? (*R2)[u] : (*L2)[u];
-        const int a = (*L2)[v], bb = (*R2)[v];
+        // a, b = the children of v
         if (u != r2) {
-            add(0, 0, v, u, -1, a, c, bb, -1, -1);   // v' = (a, c), u' = (v', b)
-            add(0, 1, v, u, -1, c, bb, a, -1, -1);   // v' = (c, b), u' = (v', a)
-        } else if ((*L2)[u] == v && binary(c)) {
-            const int d = (*L2)[c], e = (*R2)[c];
-            add(1, 2, v, u, c, a, d, -1, bb, e);     // v' = (a, d), c' = (b, e)
-            add(1, 3, v, u, c, a, e, -1, d, bb);     // v' = (a, e), c' = (d, b)
+            add(0, v);  // v' = (a, c), u' = (v', b)
+            add(1, v);  // v' = (c, b), u' = (v', a)
+        } else if ((*L2)[u] == v && binary(c)) {  // d, e = the children of c
+            add(2, v);  // v' = (a, d), c' = (b, e)
+            add(3, v);  // v' = (a, e), c' = (d, b)
         }
     }
 }
@@ -868,14 +851,14 @@ plk_status plk_nni_moves_host(int n_nodes, const int* left, const int* right, in
     std::vector<int> L2, R2;
     ItemHost h;
     relabel_and_enumerate(n_leaves, n_nodes, left, right, bl.data(), rank, root, &h, &L2, &R2, &B2);
-    *n_moves_out = (int)h.moves.size();
+    *n_moves_out = h.n_moves();
     if (moves_out) std::copy(h.move_report.begin(), h.move_report.end(), moves_out);
     return PLK_OK;
 }
 
 int plk_batch_nni_count(const plk_batch* b, int item) {
     if (!b || item < 0 || item >= (int)b->items.size()) return 0;
-    return (int)b->items[item].moves.size();
+    return b->items[item].n_moves();
 }
 
 plk_status plk_batch_nni_moves(const plk_batch* b, int item, int* moves) {
@@ -885,42 +868,165 @@ plk_status plk_batch_nni_moves(const plk_batch* b, int item, int* moves) {
     return PLK_OK;
 }
 
+}  // extern "C"
+
+namespace {
+
+constexpr size_t kSmemLimit = 227 * 1024;
+
+// The trees NNI scoring and the derivatives take: those whose op list and
+// spill stack (of a staged tile of 128 sites) fit in a CTA's shared memory.
+bool down_takes(const plk_batch* b) {
+    const size_t cm = b->C == 1 ? 1 : (b->C <= 4 ? 4 : 8);
+    const size_t stage = 2 * cm * (4 + 16) * 16, depth = std::max(b->max_depth, 1);
+    return 3 * stage + (size_t)b->max_ops * sizeof(Op) + depth * (cm * 16 + 4) * kThreads <= kSmemLimit;
+}
+
+// Plan of the down kernel for the batch's layout.  Warps per CTA: the fewest
+// (a power of two, up to 16) with which every warp tile of the batch is
+// resident at once, since an item's tables are then brought in for as few
+// idle warps as possible; 16 where there are more tiles than that.
+plk_status plan_down(plk_batch* b, DownPlan& p, bool blen) {
+    if (p.ready) return PLK_OK;
+    if (!down_takes(b))
+        return bfail(b, PLK_ERR_UNSUPPORTED, blen ? "trees too large for branch-length derivatives"
+                                                  : "trees too large for NNI scoring");
+    const int n_items = (int)b->items.size(), W = down_sites_per_warp(b->C);
+    long long tiles = 0;
+    for (const ItemHost& h : b->items) tiles += (h.n_sites + W - 1) / W;
+    // items by the length of their op list, longest first
+    std::vector<int> order(n_items);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return b->items[x].n_nodes > b->items[y].n_nodes; });
+    // the largest items whose tables do not fit read them through L1
+    int far = 0, occ = 0;
+    DownSize& z = p.size;
+    auto split = [&]() {
+        for (far = 0; far < n_items; ++far) {
+            z.nodes = z.tips = z.ints = 0;
+            for (int i = far; i < n_items; ++i) {
+                const ItemHost& h = b->items[order[i]];
+                z.nodes = std::max(z.nodes, h.n_nodes);
+                z.tips = std::max(z.tips, h.n_tips);
+                z.ints = std::max(z.ints, h.n_int);
+            }
+            if ((size_t)down_smem_bytes(b->C, blen, true, z) <= kSmemLimit) return;
+        }
+        z.nodes = z.tips = z.ints = 0;
+    };
+    for (z.warps = 1;; z.warps = std::min(2 * z.warps, kDownWarps)) {
+        split();
+        occ = down_occupancy(b->C, blen, far < n_items, z);
+        if (occ < 1) return bfail(b, PLK_ERR_UNSUPPORTED, "the pre-order kernel cannot run");
+        if (z.warps >= kDownWarps || (long long)occ * z.warps * b->n_sms >= tiles) break;
+    }
+    std::vector<int2> units;
+    std::vector<long long> rec_off(n_items);
+    std::vector<int2> blocks;
+    p.out_off.assign(n_items, 0);
+    p.total_out = 0;
+    long long records = 0;
+    for (int i = 0; i < n_items; ++i) {
+        const ItemHost& h = b->items[i];
+        const int n_out = blen ? 2 * h.n_int : h.n_moves();
+        p.out_off[i] = p.total_out;
+        p.total_out += n_out;
+        rec_off[i] = records;
+        records += (long long)n_out * ((h.n_sites + W - 1) / W);
+        for (int m = 0; m < n_out; m += 32) blocks.push_back(make_int2(i, m));
+    }
+    p.n_far = 0;
+    const int tile = z.warps * W;
+    for (int k = 0; k < n_items; ++k) {
+        if (k == far) p.n_far = (int)units.size();
+        for (int t = 0; t < (b->items[order[k]].n_sites + tile - 1) / tile; ++t) units.push_back(make_int2(order[k], t));
+    }
+    if (far == n_items) p.n_far = (int)units.size();
+    p.n_units = (int)units.size();
+    p.n_blocks = (int)blocks.size();
+    p.n_records = (size_t)std::max<long long>(records, 1);
+    p.grid_near = std::min(p.n_units - p.n_far, occ * b->n_sms);
+    p.grid_far = p.n_far == 0 ? 0 : std::min(p.n_far, std::max(1, down_occupancy(b->C, blen, false, z)) * b->n_sms);
+    PLK_BCUDA(b, p.units.ensure(units.size() * sizeof(int2)), "allocate units");
+    PLK_BCUDA(b, p.rec_off.ensure(rec_off.size() * sizeof(long long)), "allocate record offsets");
+    PLK_BCUDA(b, p.blocks.ensure(std::max<size_t>(blocks.size(), 1) * sizeof(int2)), "allocate record blocks");
+    PLK_BCUDA(b, p.d_out_off.ensure(p.out_off.size() * sizeof(int)), "allocate output offsets");
+    PLK_BCUDA(b, cudaMemcpy(p.units.p, units.data(), units.size() * sizeof(int2), cudaMemcpyHostToDevice), "upload units");
+    PLK_BCUDA(b, cudaMemcpy(p.rec_off.p, rec_off.data(), rec_off.size() * sizeof(long long), cudaMemcpyHostToDevice),
+              "upload record offsets");
+    if (!blocks.empty())
+        PLK_BCUDA(b, cudaMemcpy(p.blocks.p, blocks.data(), blocks.size() * sizeof(int2), cudaMemcpyHostToDevice),
+                  "upload record blocks");
+    PLK_BCUDA(b, cudaMemcpy(p.d_out_off.p, p.out_off.data(), p.out_off.size() * sizeof(int), cudaMemcpyHostToDevice),
+              "upload output offsets");
+    p.ready = true;
+    return PLK_OK;
+}
+
+// Enqueues the model upload, the tables, the kernel and the fold of its
+// records; the outputs are left on the device.
+plk_status enqueue_down(plk_batch* b, bool blen) {
+    DownPlan& p = blen ? b->blen_plan : b->nni_plan;
+    plk_status s = plan_down(b, p, blen);
+    if (s != PLK_OK) return s;
+    const size_t KP = (b->C + 1) / 2, W = down_sites_per_warp(b->C), n_items = b->items.size();
+    const size_t gw = (size_t)std::max(p.grid_near, p.grid_far) * p.size.warps;
+    PLK_BCUDA(b, b->d_scr.ensure(gw * b->max_int * 128 * sizeof(float4)), "allocate scratch");
+    PLK_BCUDA(b, b->d_scr_e.ensure(gw * b->max_int * 2 * W * sizeof(int)), "allocate scratch");
+    PLK_BCUDA(b, b->d_Pn.ensure((size_t)b->n_nodes_total * KP * 32 * sizeof(float)), "allocate P");
+    PLK_BCUDA(b, b->d_tipn.ensure((size_t)b->tips_total * KP * 128 * sizeof(float)), "allocate tip tables");
+    PLK_BCUDA(b, b->d_records.ensure(p.n_records * sizeof(float4)), "allocate records");
+    BlenDev bd{};
+    if (blen) {
+        PLK_BCUDA(b, b->d_blen_ex.ensure((size_t)b->n_nodes_total * KP * 8 * sizeof(float)), "allocate exponentials");
+        PLK_BCUDA(b, b->d_blen_out.ensure((size_t)p.total_out * 2 * sizeof(double)), "allocate derivatives");
+        bd = BlenDev{b->d_blen_ex.as<float>(), p.d_out_off.as<int>(),
+                     b->d_blen_out.as<double>()};
+    } else {
+        PLK_BCUDA(b, b->d_nni_out.ensure((size_t)p.total_out * sizeof(double)), "allocate NNI output");
+    }
+    BatchDev d = device_view(b, b->lnl_units);
+    d.units = p.units.as<int2>();
+    d.n_units = p.n_units;
+    d.Pn = b->d_Pn.as<float>();
+    d.tipn = b->d_tipn.as<float>();
+    d.kids = b->d_kids.as<int4>();
+    d.records = b->d_records.as<float4>();
+    d.rec_off = p.rec_off.as<long long>();
+    d.reduce_blocks = p.blocks.as<int2>();
+    d.nni_out = b->d_nni_out.as<double>();
+    d.scratch_int = b->max_int;
+    d.scr = b->d_scr.as<float4>();
+    d.scr_e = b->d_scr_e.as<int>();
+    PLK_BCUDA(b, cudaMemcpyAsync(b->d_model.p, b->h_model, n_items * batch_model_stride(b->C) * sizeof(double),
+                                 cudaMemcpyHostToDevice, b->stream), "upload models");
+    PLK_BCUDA(b, launch_down_tables(d, bd, b->stream), "batch tables launch");
+    if (p.grid_far > 0) {
+        PLK_BCUDA(b, cudaMemsetAsync(b->d_counter.p, 0, sizeof(int), b->stream), "clear work queue");
+        PLK_BCUDA(b, launch_down(d, bd, blen, false, p.size, 0, p.n_far, p.grid_far, b->stream),
+                  "pre-order kernel launch");
+    }
+    if (p.grid_near > 0) {
+        PLK_BCUDA(b, cudaMemsetAsync(b->d_counter.p, 0, sizeof(int), b->stream), "clear work queue");
+        PLK_BCUDA(b, launch_down(d, bd, blen, true, p.size, p.n_far, p.n_units, p.grid_near, b->stream),
+                  "pre-order kernel launch");
+    }
+    PLK_BCUDA(b, launch_down_reduce(d, bd, blen, p.n_blocks, b->stream), "record fold launch");
+    return PLK_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
 plk_status plk_batch_nni_loglik(plk_batch* b, double* out) {
     if (!b || !out) return b ? bfail(b, PLK_ERR_ARG, "out is NULL") : PLK_ERR_ARG;
     plk_status s = prepare_layout(b);
     if (s != PLK_OK) return s;
     if (b->total_moves == 0) return PLK_OK;
-    if (b->nni_units.spt != 1) {
-        s = build_units(b, b->nni_units, 1, true);
-        if (s != PLK_OK) return s;
-    }
-    // tip codes staged in shared memory or read from global, whichever lets
-    // more CTAs share an SM; one persistent CTA per resident slot
-    const size_t smem_staged = nni_smem_bytes(b->C, true, b->max_ops, b->max_tips, b->max_depth);
-    const size_t smem_global = nni_smem_bytes(b->C, false, b->max_ops, b->max_tips, b->max_depth);
-    if (smem_global > 227 * 1024) return bfail(b, PLK_ERR_UNSUPPORTED, "trees too large for NNI scoring");
-    const int occ_staged = smem_staged <= 227 * 1024 ? nni_occupancy(b->C, true, smem_staged, false) : 0;
-    const int occ_global = nni_occupancy(b->C, false, smem_global, false);
-    const bool codes_smem = occ_staged >= occ_global && occ_staged > 0;
-    const size_t smem = codes_smem ? smem_staged : smem_global;
-    const int per_sm = std::max(1, codes_smem ? occ_staged : occ_global);
-    const int grid = std::max(1, std::min(b->nni_units.n_units, per_sm * b->n_sms));
-    const size_t slice = (size_t)b->max_int * kThreads;
-    PLK_BCUDA(b, b->d_scr_D.ensure((size_t)grid * slice * b->C * sizeof(float4)), "allocate NNI scratch");
-    PLK_BCUDA(b, b->d_scr_O.ensure((size_t)grid * slice * b->C * sizeof(float4)), "allocate NNI scratch");
-    PLK_BCUDA(b, b->d_scr_ED.ensure((size_t)grid * slice * sizeof(int)), "allocate NNI scratch");
-    PLK_BCUDA(b, b->d_scr_EO.ensure((size_t)grid * slice * sizeof(int)), "allocate NNI scratch");
-    const BatchDev d = device_view(b, b->nni_units);
-    const size_t mn = b->items.size() * batch_model_stride(b->C);
-    plk_status se = batch_events(b, 1);
-    if (se != PLK_OK) return se;
+    if ((s = batch_events(b, 1)) != PLK_OK) return s;
     PLK_BCUDA(b, cudaEventRecord(b->ev[2], b->stream), "cudaEventRecord");
-    PLK_BCUDA(b, cudaMemsetAsync(b->d_counter.p, 0, sizeof(int), b->stream), "clear work queue");
-    PLK_BCUDA(b, cudaMemcpyAsync(b->d_model.p, b->h_model, mn * sizeof(double), cudaMemcpyHostToDevice, b->stream),
-              "upload models");
-    PLK_BCUDA(b, launch_batch_pmat(d, b->stream), "batch P(t) launch");
-    PLK_BCUDA(b, launch_batch_nni(d, codes_smem, grid, smem, b->stream), "NNI kernel launch");
-    PLK_BCUDA(b, launch_batch_nni_reduce(d, b->stream), "NNI reduce launch");
+    if ((s = enqueue_down(b, false)) != PLK_OK) return s;
     PLK_BCUDA(b, cudaMemcpyAsync(b->h_lnl, b->d_nni_out.p, (size_t)b->total_moves * sizeof(double),
                                  cudaMemcpyDeviceToHost, b->stream),
               "download NNI lnL");
@@ -947,69 +1053,14 @@ namespace {
 // d lnL / dt and d2 lnL / dt2 of every edge slot of every item into deriv
 // ([slot][2], item after item; item i's slots start at item_edge_off[i]).
 plk_status blen_pass(plk_batch* b, std::vector<double>& deriv, std::vector<int>& item_edge_off) {
-    const int n_items = (int)b->items.size();
-    if (n_items == 0) return bfail(b, PLK_ERR_STATE, "batch is empty");
+    if (b->items.empty()) return bfail(b, PLK_ERR_STATE, "batch is empty");
     for (const auto& it : b->items)
         if (!it.has_model) return bfail(b, PLK_ERR_STATE, "every item needs a model (plk_batch_set_model)");
     plk_status s = prepare_layout(b);
     if (s != PLK_OK) return s;
-    if (b->nni_units.spt != 1) {
-        s = build_units(b, b->nni_units, 1, true);
-        if (s != PLK_OK) return s;
-    }
-    // as for NNI scoring: staged or global tip codes by resident CTAs per SM
-    const size_t smem_staged = nni_smem_bytes(b->C, true, b->max_ops, b->max_tips, b->max_depth);
-    const size_t smem_global = nni_smem_bytes(b->C, false, b->max_ops, b->max_tips, b->max_depth);
-    if (smem_global > 227 * 1024) return bfail(b, PLK_ERR_UNSUPPORTED, "trees too large for branch-length derivatives");
-    const int occ_staged = smem_staged <= 227 * 1024 ? nni_occupancy(b->C, true, smem_staged, true) : 0;
-    const int occ_global = nni_occupancy(b->C, false, smem_global, true);
-    const bool codes_smem = occ_staged >= occ_global && occ_staged > 0;
-    const size_t smem = codes_smem ? smem_staged : smem_global;
-    const int per_sm = std::max(1, codes_smem ? occ_staged : occ_global);
-    const int grid = std::max(1, std::min(b->nni_units.n_units, per_sm * b->n_sms));
-    const size_t slice = (size_t)b->max_int * kThreads;
-    PLK_BCUDA(b, b->d_scr_D.ensure((size_t)grid * slice * b->C * sizeof(float4)), "allocate scratch");
-    PLK_BCUDA(b, b->d_scr_O.ensure((size_t)grid * slice * b->C * sizeof(float4)), "allocate scratch");
-    PLK_BCUDA(b, b->d_scr_ED.ensure((size_t)grid * slice * sizeof(int)), "allocate scratch");
-    PLK_BCUDA(b, b->d_scr_EO.ensure((size_t)grid * slice * sizeof(int)), "allocate scratch");
-    // edge slots: 2 per internal node of every item, per unit and per item
-    item_edge_off.assign(n_items, 0);
-    std::vector<int> edge_item;
-    int total_slots = 0;
-    for (int i = 0; i < n_items; ++i) {
-        item_edge_off[i] = total_slots;
-        total_slots += 2 * b->items[i].n_int;
-        edge_item.insert(edge_item.end(), 2 * b->items[i].n_int, i);
-    }
-    const std::vector<int2>& units = b->nni_units.host_units;
-    std::vector<long long> unit_edge_off(units.size());
-    long long unit_slots = 0;
-    for (size_t u = 0; u < units.size(); ++u) {
-        unit_edge_off[u] = unit_slots;
-        unit_slots += 2 * b->items[units[u].x].n_int;
-    }
-    PLK_BCUDA(b, b->d_blen_ueo.ensure(unit_edge_off.size() * sizeof(long long)), "allocate edge slots");
-    PLK_BCUDA(b, b->d_blen_ues.ensure((size_t)unit_slots * 2 * sizeof(double)), "allocate edge slots");
-    PLK_BCUDA(b, b->d_blen_ieo.ensure(item_edge_off.size() * sizeof(int)), "allocate edge slots");
-    PLK_BCUDA(b, b->d_blen_ei.ensure(edge_item.size() * sizeof(int)), "allocate edge slots");
-    PLK_BCUDA(b, b->d_blen_out.ensure((size_t)total_slots * 2 * sizeof(double)), "allocate edge slots");
-    PLK_BCUDA(b, cudaMemcpyAsync(b->d_blen_ueo.p, unit_edge_off.data(), unit_edge_off.size() * sizeof(long long),
-                                 cudaMemcpyHostToDevice, b->stream), "upload edge slots");
-    PLK_BCUDA(b, cudaMemcpyAsync(b->d_blen_ieo.p, item_edge_off.data(), item_edge_off.size() * sizeof(int),
-                                 cudaMemcpyHostToDevice, b->stream), "upload edge slots");
-    PLK_BCUDA(b, cudaMemcpyAsync(b->d_blen_ei.p, edge_item.data(), edge_item.size() * sizeof(int),
-                                 cudaMemcpyHostToDevice, b->stream), "upload edge slots");
-    BlenDev bd{b->d_blen_ueo.as<long long>(), b->d_blen_ues.as<double>(), b->d_blen_ieo.as<int>(),
-               b->d_blen_ei.as<int>(), total_slots, b->d_blen_out.as<double>()};
-    deriv.assign((size_t)total_slots * 2, 0.0);
-    const BatchDev d = device_view(b, b->nni_units);
-    const size_t mn = (size_t)n_items * batch_model_stride(b->C);
-    PLK_BCUDA(b, cudaMemsetAsync(b->d_counter.p, 0, sizeof(int), b->stream), "clear work queue");
-    PLK_BCUDA(b, cudaMemcpyAsync(b->d_model.p, b->h_model, mn * sizeof(double), cudaMemcpyHostToDevice, b->stream),
-              "upload models");
-    PLK_BCUDA(b, launch_batch_pmat(d, b->stream), "batch P(t) launch");
-    PLK_BCUDA(b, launch_batch_blen(d, bd, codes_smem, grid, smem, b->stream), "branch-length kernel launch");
-    PLK_BCUDA(b, launch_batch_blen_reduce(d, bd, b->stream), "branch-length reduce launch");
+    if ((s = enqueue_down(b, true)) != PLK_OK) return s;
+    item_edge_off = b->blen_plan.out_off;
+    deriv.resize((size_t)b->blen_plan.total_out * 2);
     PLK_BCUDA(b, cudaMemcpyAsync(deriv.data(), b->d_blen_out.p, deriv.size() * sizeof(double), cudaMemcpyDeviceToHost,
                                  b->stream), "download derivatives");
     PLK_BCUDA(b, cudaStreamSynchronize(b->stream), "branch-length derivatives");
