@@ -2,6 +2,12 @@
 // hand-written kernels (absent in the reference, whose optimiser always starts
 // from fixed values, src/treeator.cpp:612-615).
 //
+//  rows_kernel       (networks up to 256 wide) the whole forward pass, the loss
+//                    and the chain of activation gradients of 128 rows in one
+//                    CTA, activations staying in shared memory.
+//  update_kernel     weight and bias gradients of a tile over the whole batch,
+//                    and on them, still in registers, the Adam step.
+// Wider networks run layer by layer:
 //  gemm_tc_kernel    C[M x N] = sum_k A(m, k) B(n, k) with BF16 operands read
 //                    through arbitrary strides (so one kernel serves X W^T,
 //                    dZ W and dZ^T A), FP32 accumulation in tensor memory
@@ -15,6 +21,7 @@
 // Weights are BF16 in every GEMM (the network's storage precision), master
 // weights and optimiser moments FP32.  Feature dimensions are padded to 16
 // and the batch to 64 with zeros.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -254,6 +261,599 @@ __global__ void __launch_bounds__(128, 1) gemm_tc_kernel(GemmArgs g) {
     }
 }
 
+// ---------------------------------------------------------------------------
+// Networks whose layers are at most 256 wide: two kernels a training step.
+//
+// Layer by layer, a step of 43-256-256-256-7 on 256 rows was 40 launches, the
+// GEMMs 30 us each (operands gathered two bytes at a time, K in four waits, 16
+// CTAs): 525 us.  Rows do not depend on one another until the weight
+// gradients, so rows_kernel takes 128 rows through every layer, forward and
+// back, in one cluster of four CTAs.  It is a chain of products with nothing to
+// run beside it, so what counts is the latency of a link: each CTA computes a
+// quarter of a layer's columns (its weights a contiguous slice of an image
+// that update_kernel keeps in the operand's layout, brought in by one bulk
+// copy a layer ahead), one thread issues the MMAs, and the epilogue writes the
+// BF16 results as a slice of the next layer's A operand (K-major core matrices,
+// no swizzle), which one bulk copy each takes to the other CTAs' shared memory
+// and their barriers.  One CTA a row block did the same in 56 us a pass, four
+// with every thread storing to every CTA and a cluster barrier a layer in 34,
+// this in 29.  update_kernel then has a CTA per 128 x 32 tile of every
+// weight matrix, the batch as K; its operands are transposed on the way by
+// ldmatrix.trans / stmatrix.  A step, with the host's part, 525 -> 65 us.
+// Every wait on an mbarrier is bounded; one that runs out raises the network's
+// fail flag, so the loss is NaN and the weights stay as they were.
+// ---------------------------------------------------------------------------
+constexpr int kNetWide = 256;   // widest layer (padded to 16)
+constexpr int kNetLayers = 8;   // weight layers
+constexpr int kNetThreads = 256;
+constexpr int kNetCtas = 4;     // of a row block's cluster
+constexpr int kUpN = 32, kUpK = 256;  // update tile: inputs, batch rows per pass
+
+struct NetLayer {
+    int in, out, pin, pout;           // real and padded widths
+    const __nv_bfloat16* wf;          // image of W (N = out, K = in), see net_image_at
+    const __nv_bfloat16* wt;          // image of W^T (N = in, K = out)
+    const float* bias;
+    __nv_bfloat16 *act, *dz;          // layer input [rows][pin], output gradient [rows][pout]
+    size_t w_off, b_off;              // into the flat parameters
+    int tiles_n, tile0;               // update_kernel: input tiles, first CTA of the layer
+};
+
+struct NetArgs {
+    int L, batch, backward, adam;
+    NetLayer layer[kNetLayers];
+    const float *x, *t;               // [batch][n_in], [batch][n_out]
+    float* y;                         // [batch][n_out]
+    float* loss_part;                 // [CTAs]
+    float* loss;
+    int* fail;
+    float *p, *g, *m, *v;
+    float lr, b1, b2, eps, c1, c2;
+};
+
+// Columns a CTA of the cluster takes of N, and where element (n, k) of a
+// weight image sits: [CTA][K / 8][columns][8].
+__host__ __device__ constexpr int net_share(int N) { return (N / 16 + kNetCtas - 1) / kNetCtas * 16; }
+__host__ __device__ constexpr size_t net_image_elems(int N, int K) { return (size_t)kNetCtas * net_share(N) * K; }
+__device__ __forceinline__ size_t net_image_at(int n, int k, int N, int K) {
+    const int w = net_share(N);
+    return ((size_t)(n / w * (K / 8) + (k >> 3)) * w + n % w) * 8 + (k & 7);
+}
+
+__device__ __forceinline__ bool net_wait(uint32_t mbar, uint32_t parity) {
+    for (int it = 0; it < kGWaitLimit; ++it) {
+        uint32_t ok;
+        asm volatile(
+            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+            "selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(ok)
+            : "r"(mbar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
+// the MMAs of a K-deep product, A [K / 8][128][8] and B [K / 8][N][8], committed to mbar
+__device__ __forceinline__ void net_mma(uint32_t tmem, uint32_t a, uint32_t b, int N, int K, bool first, uint32_t mbar) {
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((kGM >> 4) << 24);
+    // one thread issues them: a step of K is an addition to each descriptor's
+    // address (16-byte units; the operands lie below 256 KB, so nothing carries)
+    uint64_t ad = g_smem_desc(a, kGM * 16, 128), bd = g_smem_desc(b, N * 16, 128);
+    uint32_t accum = first ? 0u : 1u;
+#pragma unroll 4
+    for (int ks = 0; ks < K / 16; ++ks) {
+        asm volatile(
+            "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+            "l"(ad), "l"(bd), "r"(idesc), "r"(accum));
+        ad += 2 * kGM;
+        bd += 2 * N;
+        accum = 1u;
+    }
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar) : "memory");
+}
+
+__device__ __forceinline__ void net_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void net_ld16(uint32_t taddr, float (&v)[16]) {
+    uint32_t r[16];
+    net_ld16_issue(taddr, r);
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        asm volatile("" : "+r"(r[i]));  // no use ahead of the wait
+        v[i] = __uint_as_float(r[i]);
+    }
+}
+
+__device__ __forceinline__ uint4 net_pack8(const float* v) {
+    uint4 o;
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+        w[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    o.x = w[0]; o.y = w[1]; o.z = w[2]; o.w = w[3];
+    return o;
+}
+
+// TMEM and the mbarriers of a CTA (all threads call it)
+constexpr int kNetBars = 5;
+__device__ __forceinline__ uint32_t net_begin(uint32_t* s_tmem, uint64_t* s_bar, int* s_fail, int cols) {
+    const uint32_t bar = static_cast<uint32_t>(__cvta_generic_to_shared(s_bar));
+    if (threadIdx.x < 32) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
+                         static_cast<uint32_t>(__cvta_generic_to_shared(s_tmem))),
+                     "r"(cols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kNetBars; ++i)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar + 8 * i) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        *s_fail = 0;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    return *s_tmem;
+}
+__device__ __forceinline__ void net_end(uint32_t tmem, int cols) {
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(cols) : "memory");
+    }
+}
+
+constexpr int kRowsA = kGM * kNetWide * 2;                          // one A operand
+constexpr int kRowsW = net_share(kNetWide) * kNetWide * 2;          // one weight slice
+constexpr int kRowsSmem = 2 * kRowsA + 2 * kRowsW;
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+__global__ void __cluster_dims__(kNetCtas, 1, 1) __launch_bounds__(kNetThreads, 1)
+    rows_kernel(const __grid_constant__ NetArgs n) {
+    extern __shared__ __align__(128) unsigned char net_sm[];
+    // MMAs done, weights landed (two buffers), the other CTAs' slices of A landed (two)
+    __shared__ __align__(8) uint64_t s_bar[kNetBars];
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_fail;
+    __shared__ float s_red[kNetThreads];
+    __shared__ __align__(16) float s_bias[kNetLayers][net_share(kNetWide)];
+    __shared__ uint32_t s_pos[kNetLayers][kNetThreads];  // ReLU: the positive ones of a thread's 32 columns
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = blockIdx.x % kNetCtas, row0 = blockIdx.x / kNetCtas * kGM;
+    const uint32_t a_sm = static_cast<uint32_t>(__cvta_generic_to_shared(net_sm)), w_sm = a_sm + 2 * kRowsA;
+    const uint32_t bar = static_cast<uint32_t>(__cvta_generic_to_shared(s_bar));
+    const uint32_t tmem = net_begin(&s_tmem, s_bar, &s_fail, net_share(kNetWide));
+    const int L = n.L, steps = n.backward ? 2 * L - 1 : L;
+    // step st: layer l forward (st < L) or back (layers L - 1 .. 1)
+    auto layer_of = [&](int st) { return st < L ? st : 2 * L - 1 - st; };
+    // thread 0: this CTA's slice of step st's weights, in 32 KB copies
+    auto load_w = [&](int st) {
+        const NetLayer& ly = n.layer[layer_of(st)];
+        const int N = st < L ? ly.pout : ly.pin, K = st < L ? ly.pin : ly.pout;
+        const uint32_t bytes = (uint32_t)(net_share(N) * K * 2), to = w_sm + (st & 1) * kRowsW, b = bar + 8 + 8 * (st & 1);
+        const char* src = reinterpret_cast<const char*>(st < L ? ly.wf : ly.wt) + (size_t)rank * bytes;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(b), "r"(bytes) : "memory");
+        for (uint32_t off = 0; off < bytes; off += 32768) {
+            const uint32_t c = min(32768u, bytes - off);
+            asm volatile(
+                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(to + off),
+                "l"(src + off), "r"(c), "r"(b)
+                : "memory");
+        }
+    };
+    if (tid == 0) load_w(0);
+    const int r = 32 * (warp & 3) + lane, row = row0 + r;
+    // the biases of this CTA's columns, and the targets of this thread's first
+    // sixteen outputs: their latency passes beside the inputs'
+    float bv[kNetLayers];
+#pragma unroll
+    for (int l = 0; l < kNetLayers; ++l) {
+        const int share = l < L ? net_share(n.layer[l].pout) : 0, c = rank * share + tid;
+        bv[l] = l < L && tid < share && c < n.layer[l].out ? n.layer[l].bias[c] : 0.0f;
+    }
+    float tv[16];
+    if (n.backward) {
+        const int out = n.layer[L - 1].out, c0 = rank * net_share(n.layer[L - 1].pout) + 16 * (warp >> 2);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) tv[j] = row < n.batch && c0 + j < out ? n.t[(size_t)row * out + c0 + j] : 0.0f;
+    }
+    // the rows' inputs as BF16: A operand and, for the weight gradients, the first layer's input
+    {
+        const NetLayer& l0 = n.layer[0];
+        const int chunks = l0.pin / 8, total = kGM * chunks;
+        for (int base = tid; base < total; base += 4 * kNetThreads) {
+            float v[4][8];  // four chunks' loads in flight: they come over the host link
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = base + u * kNetThreads, rr = i / chunks, c = i % chunks;
+                const bool in = i < total && row0 + rr < n.batch;
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    v[u][j] = in && 8 * c + j < l0.in ? n.x[(size_t)(row0 + rr) * l0.in + 8 * c + j] : 0.0f;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = base + u * kNetThreads, rr = i / chunks, c = i % chunks;
+                if (i >= total) break;
+                const uint4 o = net_pack8(v[u]);
+                *reinterpret_cast<uint4*>(net_sm + ((size_t)c * kGM + rr) * 16) = o;
+                if (n.backward && rank == 0 && row0 + rr < n.batch)
+                    *reinterpret_cast<uint4*>(l0.act + (size_t)(row0 + rr) * l0.pin + 8 * c) = o;
+            }
+        }
+    }
+#pragma unroll
+    for (int l = 0; l < kNetLayers; ++l)
+        if (tid < net_share(kNetWide)) s_bias[l][tid] = bv[l];
+    asm volatile("fence.proxy.async;\n" ::: "memory");  // the A rows -> the tensor cores
+    cluster_barrier();  // every CTA of the cluster runs before anything is written into it
+    const uint32_t trow = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+    float sq = 0.0f;
+    uint32_t mma_phase = 0;
+    for (int st = 0; st < steps; ++st) {
+        const bool fwd = st < L, last = st == L - 1;
+        const int l = layer_of(st);
+        const NetLayer& ly = n.layer[l];
+        const int N = fwd ? ly.pout : ly.pin, K = fwd ? ly.pin : ly.pout, share = net_share(N), n0 = rank * share;
+        if (!net_wait(bar + 8 + 8 * (st & 1), (st >> 1) & 1)) {
+            net_wait(bar + 8 + 8 * (st & 1), (st >> 1) & 1);  // a last bounded wait for the copy in flight
+            s_fail = 1;
+        }
+        if (st > 0 && !net_wait(bar + 24 + 8 * (st & 1), ((st - 1) >> 1) & 1)) {
+            net_wait(bar + 24 + 8 * (st & 1), ((st - 1) >> 1) & 1);
+            s_fail = 1;
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+        __syncthreads();
+        const bool go = s_fail == 0 && n0 < N;  // a CTA past the last columns only keeps step
+        if (go && tid == 0) {
+            asm volatile("fence.proxy.async;\n" ::: "memory");
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            net_mma(tmem, a_sm + (st & 1) * kRowsA, w_sm + (st & 1) * kRowsW, share, K, true, bar);
+        }
+        // the other buffer's products were waited for in the step before
+        if (tid == 32 && st + 1 < steps) load_w(st + 1);
+        bool done = false;
+        if (go) {
+            done = net_wait(bar, mma_phase) || net_wait(bar, mma_phase);
+            if (!done) s_fail = 1;
+            mma_phase ^= 1u;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        // this thread's row: its half of the CTA's columns
+        const bool all_done = __all_sync(0xffffffffu, done);
+        uint32_t acc[2][16];
+        if (all_done) {
+            net_ld16_issue(trow + 16 * (warp >> 2), acc[0]);
+            net_ld16_issue(trow + 16 * (warp >> 2) + 32, acc[1]);
+            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int cl = 16 * (warp >> 2) + 32 * q, c0 = n0 + cl;  // in the CTA's columns, in the layer's
+            if (cl >= share || c0 >= N || !all_done) continue;
+            float v[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                asm volatile("" : "+r"(acc[q][j]));  // no use ahead of the wait
+                v[j] = __uint_as_float(acc[q][j]);
+            }
+            if (fwd) {
+                uint32_t pos = 0;
+#pragma unroll
+                for (int j = 0; j < 16; j += 4) {  // past the width the products and the biases are zero
+                    const float4 b4 = *reinterpret_cast<const float4*>(&s_bias[l][cl + j]);
+                    v[j] += b4.x;
+                    v[j + 1] += b4.y;
+                    v[j + 2] += b4.z;
+                    v[j + 3] += b4.w;
+                }
+                if (!last)
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] = fmaxf(v[j], 0.0f);
+                if (!last && n.backward) {
+                    // what the gradient lets through: the output as it is stored
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (__bfloat162float(__float2bfloat16(v[j])) > 0.0f) pos |= 1u << j;
+                    s_pos[l][tid] = q == 0 ? pos : (s_pos[l][tid] | (pos << 16));
+                }
+            } else {
+                const uint32_t pos = s_pos[l - 1][tid] >> (16 * q);
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    if (!((pos >> j) & 1u)) v[j] = 0.0f;
+            }
+            if (last) {
+                const float scale = 2.f / ((float)n.batch * ly.out);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    float gr = 0.0f;
+                    if (row < n.batch && c0 + j < ly.out) {
+                        if (n.y) n.y[(size_t)row * ly.out + c0 + j] = v[j];
+                        if (n.backward) {
+                            const float d = v[j] - (q == 0 ? tv[j] : n.t[(size_t)row * ly.out + c0 + j]);
+                            sq += d * d;
+                            gr = scale * d;
+                        }
+                    }
+                    v[j] = gr;
+                }
+            }
+            const uint4 o0 = net_pack8(v), o1 = net_pack8(v + 8);
+            if (st + 1 < steps) {
+                // this CTA's slice of the next step's A operand
+                unsigned char* at = net_sm + ((st + 1) & 1) * kRowsA + ((c0 / 8) * kGM + r) * 16;
+                *reinterpret_cast<uint4*>(at) = o0;
+                *reinterpret_cast<uint4*>(at + kGM * 16) = o1;
+            }
+            if (n.backward && row < n.batch) {
+                // a layer's output is the next one's input; its gradient that of the layer below
+                __nv_bfloat16* dst = last ? ly.dz : (fwd ? n.layer[l + 1].act : n.layer[l - 1].dz);
+                uint4* g = reinterpret_cast<uint4*>(dst + (size_t)row * N + c0);
+                g[0] = o0;
+                g[1] = o1;
+            }
+        }
+        // the slice to the other CTAs; theirs arrive on this one's barrier.  A
+        // buffer is free by then: a CTA reaches this point only with the slices
+        // that every other CTA sent after its products of the step before.
+        asm volatile("fence.proxy.async;\n" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+        __syncthreads();
+        if (tid == 0 && st + 1 < steps) {
+            const int own = max(0, min(share, N - n0));
+            const uint32_t b = bar + 24 + 8 * ((st + 1) & 1), bytes = (uint32_t)own * kGM * 2;
+            const uint32_t at = a_sm + ((st + 1) & 1) * kRowsA + (uint32_t)(n0 / 8 * kGM) * 16;
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(b),
+                         "r"((uint32_t)(N - own) * kGM * 2)
+                         : "memory");
+            for (int d = 1; d < kNetCtas && own > 0; ++d) {
+                const int cta = (rank + d) % kNetCtas;
+                uint32_t to, tb;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(to) : "r"(at), "r"(cta));
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(tb) : "r"(b), "r"(cta));
+                asm volatile(
+                    "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(to),
+                    "r"(at), "r"(bytes), "r"(tb)
+                    : "memory");
+            }
+        }
+    }
+    cluster_barrier();  // every copy from and into this CTA's shared memory has landed
+    if (s_fail) {
+        if (tid == 0) *n.fail = 1;
+        if (n.y && warp < 4 && row < n.batch && rank == 0)
+            for (int c = 0; c < n.layer[L - 1].out; ++c)
+                n.y[(size_t)row * n.layer[L - 1].out + c] = __int_as_float(0x7fc00000);
+    }
+    if (n.backward) {
+        s_red[tid] = sq;
+        __syncthreads();
+        for (int off = kNetThreads / 2; off > 0; off >>= 1) {
+            if (tid < off) s_red[tid] += s_red[tid + off];
+            __syncthreads();
+        }
+        if (tid == 0) n.loss_part[blockIdx.x] = s_red[0];
+    }
+    net_end(tmem, net_share(kNetWide));
+}
+
+// Shared memory of update_kernel: the row-major tiles (rows padded by 16 bytes
+// against bank conflicts), then the operands [K / 8][rows][8].
+constexpr int kUpPitchA = kGM * 2 + 16, kUpPitchB = kUpN * 2 + 16;
+constexpr int kUpStageA = kUpK * kUpPitchA, kUpStageB = kUpK * kUpPitchB;
+constexpr int kUpOpA = kUpK * kGM * 2, kUpOpB = kUpK * kUpN * 2;
+constexpr int kUpSmem = kUpOpA + kUpOpB + kUpStageA + kUpStageB;
+
+// 8 x 8 blocks of src (row-major [k][columns], `pitch` bytes a row) into dst
+// ([k / 8][columns][8]): four blocks of neighbouring columns an instruction
+__device__ __forceinline__ void net_transpose(uint32_t src, int pitch, uint32_t dst, int cols, int k) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int quads = cols / 32, n = k / 8 * quads;
+    for (int i = warp; i < n; i += kNetThreads / 32) {
+        const int kg = i / quads, col = (i % quads) * 32 + (lane >> 3) * 8, r = lane & 7;
+        const uint32_t s = src + (uint32_t)((8 * kg + r) * pitch + col * 2);
+        const uint32_t d = dst + (uint32_t)((kg * cols + col + r) * 16);
+        uint32_t x[4];
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                     : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3])
+                     : "r"(s)
+                     : "memory");
+        asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};\n" ::"r"(d), "r"(x[0]), "r"(x[1]),
+                     "r"(x[2]), "r"(x[3])
+                     : "memory");
+    }
+}
+
+// rows [k0, k0 + kUpK) of src ([rows][width]), columns [c0, c0 + cols), zero past the batch and the width
+template <int COLS>
+__device__ __forceinline__ void net_stage(unsigned char* dst, int pitch, const __nv_bfloat16* src, int width, int c0,
+                                          int k0, int batch) {
+    constexpr int chunks = COLS / 8;
+    const uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+#pragma unroll
+    for (int i0 = 0; i0 < kUpK * chunks; i0 += kNetThreads) {
+        const int r = (i0 + threadIdx.x) / chunks, c = threadIdx.x % chunks;
+        const bool in = k0 + r < batch && c0 + 8 * c < width;
+        const __nv_bfloat16* from = in ? src + (size_t)(k0 + r) * width + c0 + 8 * c : src;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(to + r * pitch + 16 * c), "l"(from),
+                     "r"(in ? 16 : 0)
+                     : "memory");
+    }
+}
+
+// one Adam update of a parameter from its gradient, every rounding spelt out
+// (those adam_kernel's expressions compile to): training amplifies a last bit
+__device__ __forceinline__ void net_adam(const NetArgs& n, float gi, float& p, float& m, float& v) {
+    m = fmaf(__fsub_rn(1.f, n.b1), gi, __fmul_rn(n.b1, m));
+    v = fmaf(__fmul_rn(__fsub_rn(1.f, n.b2), gi), gi, __fmul_rn(n.b2, v));
+    p -= n.lr * (m / n.c1) / (sqrtf(v / n.c2) + n.eps);
+}
+
+__global__ void __launch_bounds__(kNetThreads, 1) update_kernel(const __grid_constant__ NetArgs n, int row_ctas) {
+    extern __shared__ __align__(128) unsigned char net_sm[];
+    __shared__ __align__(8) uint64_t s_bar[kNetBars];
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_fail;
+    if (*n.fail) {  // a row block gave up: no update, and the loss says so
+        if (blockIdx.x == 0 && threadIdx.x == 0) *n.loss = __int_as_float(0x7fc00000);
+        return;
+    }
+    int l = 0;
+    while (l + 1 < n.L && (int)blockIdx.x >= n.layer[l + 1].tile0) ++l;
+    const NetLayer& ly = n.layer[l];
+    const int t = blockIdx.x - ly.tile0, m0 = t / ly.tiles_n * kGM, n0 = t % ly.tiles_n * kUpN;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    unsigned char *stA = net_sm + kUpOpA + kUpOpB, *stB = stA + kUpStageA;
+    const uint32_t a_sm = static_cast<uint32_t>(__cvta_generic_to_shared(net_sm));
+    const uint32_t bar = static_cast<uint32_t>(__cvta_generic_to_shared(s_bar));
+    const uint32_t tmem = net_begin(&s_tmem, s_bar, &s_fail, kUpN);
+    float bias = 0.0f;  // thread o < 128 of the tiles with n0 = 0: the bias gradient of output m0 + o
+    bool ok = true;
+    uint32_t phase = 0;
+    for (int k0 = 0; k0 < n.batch; k0 += kUpK, phase ^= 1u) {
+        net_stage<kGM>(stA, kUpPitchA, ly.dz, ly.pout, m0, k0, n.batch);
+        net_stage<kUpN>(stB, kUpPitchB, ly.act, ly.pin, n0, k0, n.batch);
+        asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();
+        const int K = (min(kUpK, n.batch - k0) + 15) / 16 * 16;
+        net_transpose(a_sm + kUpOpA + kUpOpB, kUpPitchA, a_sm, kGM, K);
+        net_transpose(a_sm + kUpOpA + kUpOpB + kUpStageA, kUpPitchB, a_sm + kUpOpA, kUpN, K);
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+        __syncthreads();
+        if (tid == 0) {
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            net_mma(tmem, a_sm, a_sm + kUpOpA, kUpN, K, k0 == 0, bar);
+        }
+        if (n0 == 0 && tid < kGM)
+#pragma unroll 16
+            for (int r = 0; r < K; ++r)
+                bias += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(stA + (size_t)r * kUpPitchA + 2 * tid));
+        if (!net_wait(bar, phase)) {
+            net_wait(bar, phase);
+            s_fail = 1;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        __syncthreads();
+        ok = s_fail == 0;
+        if (!ok) break;
+    }
+    // the tile's gradient through shared memory, so that the parameters and
+    // moments go by whole rows of 32 (a thread a row of sixteen touched 32 rows
+    // an instruction: 12 of the kernel's 21 us)
+    float* const s_g = reinterpret_cast<float*>(stA);                                   // [128][33]
+    __nv_bfloat16* const s_h = reinterpret_cast<__nv_bfloat16*>(stB);                   // [128][40]
+    {
+        float v[16];
+        net_ld16(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 16 * (warp >> 2), v);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) s_g[(32 * (warp & 3) + lane) * 33 + 16 * (warp >> 2) + j] = v[j];
+    }
+    __syncthreads();
+    if (ok) {
+        constexpr int kRows = kGM / (kNetThreads / 32);  // rows of a warp
+        const int c = n0 + lane;
+        const size_t at = ly.w_off + (size_t)(m0 + warp) * ly.in + c, step = (size_t)(kNetThreads / 32) * ly.in;
+        if (n.adam) {
+            float p[kRows], m[kRows], v[kRows];
+            bool in[kRows];
+#pragma unroll
+            for (int i = 0; i < kRows; ++i) {
+                in[i] = c < ly.in && m0 + warp + 8 * i < ly.out;
+                p[i] = m[i] = v[i] = 0.0f;
+                if (in[i]) {
+                    p[i] = n.p[at + i * step];
+                    m[i] = n.m[at + i * step];
+                    v[i] = n.v[at + i * step];
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < kRows; ++i) {
+                if (in[i]) {
+                    net_adam(n, s_g[(warp + 8 * i) * 33 + lane], p[i], m[i], v[i]);
+                    n.p[at + i * step] = p[i];
+                    n.m[at + i * step] = m[i];
+                    n.v[at + i * step] = v[i];
+                }
+                s_h[(warp + 8 * i) * 40 + lane] = __float2bfloat16(p[i]);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < kRows; ++i)
+                if (c < ly.in && m0 + warp + 8 * i < ly.out) n.g[at + i * step] = s_g[(warp + 8 * i) * 33 + lane];
+        }
+    }
+    __syncthreads();
+    if (ok && n.adam) {
+        // the images, eight weights at a time (shares and tiles are multiples of eight)
+        __nv_bfloat16* wf = const_cast<__nv_bfloat16*>(ly.wf);
+        __nv_bfloat16* wt = const_cast<__nv_bfloat16*>(ly.wt);
+        for (int i = tid; i < kGM * (kUpN / 8); i += kNetThreads) {
+            const int o = i % kGM, c8 = i / kGM * 8;
+            if (m0 + o < ly.pout && n0 + c8 < ly.pin)
+                *reinterpret_cast<uint4*>(wf + net_image_at(m0 + o, n0 + c8, ly.pout, ly.pin)) =
+                    *reinterpret_cast<const uint4*>(s_h + o * 40 + c8);
+            const int c = i % kUpN, o8 = i / kUpN * 8;
+            if (m0 + o8 < ly.pout && n0 + c < ly.pin) {
+                __align__(16) __nv_bfloat16 h[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) h[j] = s_h[(o8 + j) * 40 + c];
+                *reinterpret_cast<uint4*>(wt + net_image_at(n0 + c, m0 + o8, ly.pin, ly.pout)) =
+                    *reinterpret_cast<const uint4*>(h);
+            }
+        }
+    }
+    if (ok && n0 == 0 && tid < kGM && m0 + tid < ly.out) {
+        const size_t i = ly.b_off + m0 + tid;
+        if (n.adam) {
+            float p = n.p[i], m = n.m[i], vv = n.v[i];
+            net_adam(n, bias, p, m, vv);
+            n.p[i] = p;
+            n.m[i] = m;
+            n.v[i] = vv;
+        } else {
+            n.g[i] = bias;
+        }
+    }
+    if (tid == 0 && !ok) *n.fail = 1;
+    if (blockIdx.x == 0 && tid == 0) {
+        float s = 0.0f;
+        for (int i = 0; i < row_ctas; ++i) s += n.loss_part[i];
+        const NetLayer& top = n.layer[n.L - 1];
+        *n.loss = ok ? s / ((float)n.batch * top.out) : __int_as_float(0x7fc00000);
+    }
+    net_end(tmem, kUpN);
+}
+
+// both images of one layer's weights from the FP32 parameters, zero in the padding
+__global__ void pack_images_kernel(const float* w, int in, int out, int pin, int pout, __nv_bfloat16* wf,
+                                   __nv_bfloat16* wt) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= pin * pout) return;
+    const int o = i / pin, c = i % pin;
+    const __nv_bfloat16 h = __float2bfloat16(o < out && c < in ? w[(size_t)o * in + c] : 0.0f);
+    wf[net_image_at(o, c, pout, pin)] = h;
+    wt[net_image_at(c, o, pin, pout)] = h;
+}
+
 cudaError_t gemm(const GemmArgs& g, cudaStream_t st) {
     dim3 grid((g.N + kGN - 1) / kGN, (g.M + kGM - 1) / kGM);
     gemm_tc_kernel<<<grid, 128, 0, st>>>(g);
@@ -281,7 +881,21 @@ struct plk_mlp {
     __nv_bfloat16 *dz = nullptr, *dz2 = nullptr;
     float *xin = nullptr, *tin = nullptr, *loss = nullptr;
     long long step = 0;
+    // networks up to kNetWide wide (rows_kernel, update_kernel): the weight
+    // images, the layers' inputs and gradients [cap rows], row blocks' losses,
+    // and a pinned block the kernels read the rows from and write the loss to
+    bool narrow = false;
+    std::vector<__nv_bfloat16*> wf, wt, n_act, n_dz;
+    int n_cap = 0;
+    float *loss_part = nullptr, *y_dev = nullptr;
+    int* fail = nullptr;
+    char *host = nullptr, *host_dev = nullptr;
+    size_t host_bytes = 0;
     ~plk_mlp() {
+        for (auto* v : {&wf, &wt, &n_act, &n_dz})
+            for (auto* q : *v) cudaFree(q);
+        cudaFree(loss_part); cudaFree(y_dev); cudaFree(fail);
+        if (host) cudaFreeHost(host);
         cudaFree(p); cudaFree(g); cudaFree(m); cudaFree(v);
         for (auto* q : wb) cudaFree(q);
         for (auto* q : act) cudaFree(q);
@@ -331,7 +945,134 @@ plk_status ensure_batch(plk_mlp* m, int batch) {
     return PLK_OK;
 }
 
+// ---- networks up to kNetWide wide --------------------------------------------
+constexpr size_t kHostRows = 4 << 20;  // rows larger than this are copied to the device instead
+
+plk_status net_images(plk_mlp* m) {
+    PLK_MCUDA(m, cudaStreamSynchronize(nullptr), "upload weights");  // copied on the default stream
+    for (int l = 0; l < n_layers(m); ++l) {
+        const int n = m->pdims[l] * m->pdims[l + 1];
+        pack_images_kernel<<<(n + 255) / 256, 256, 0, m->stream>>>(m->p + m->w_off[l], m->dims[l], m->dims[l + 1],
+                                                                  m->pdims[l], m->pdims[l + 1], m->wf[l], m->wt[l]);
+    }
+    PLK_MCUDA(m, cudaGetLastError(), "weight images");
+    PLK_MCUDA(m, cudaStreamSynchronize(m->stream), "weight images");
+    return PLK_OK;
+}
+
+// Room for `batch` rows, and the pinned block: [loss][x][t], read and written
+// by the kernels in place.
+plk_status net_ensure(plk_mlp* m, int batch, bool train) {
+    const int rows = (batch + kGM - 1) / kGM * kGM;
+    const size_t xb = (size_t)batch * m->dims.front() * sizeof(float), tb = (size_t)batch * m->dims.back() * sizeof(float);
+    const size_t want = 256 + (xb + tb <= kHostRows ? (xb + 255) / 256 * 256 + tb : 0);
+    if (want > m->host_bytes) {
+        if (m->host) cudaFreeHost(m->host);
+        m->host = nullptr;
+        m->host_bytes = 0;
+        PLK_MCUDA(m, cudaHostAlloc(&m->host, want, cudaHostAllocMapped), "allocate pinned rows");
+        void* d = nullptr;
+        PLK_MCUDA(m, cudaHostGetDevicePointer(&d, m->host, 0), "pinned rows");
+        m->host_dev = static_cast<char*>(d);
+        m->host_bytes = want;
+    }
+    if (!m->fail) {
+        PLK_MCUDA(m, cudaMalloc(&m->fail, sizeof(int)), "allocate flag");
+        PLK_MCUDA(m, cudaMemsetAsync(m->fail, 0, sizeof(int), m->stream), "clear flag");
+    }
+    if (rows > m->n_cap) {
+        for (auto* v : {&m->n_act, &m->n_dz}) {
+            for (auto* q : *v) cudaFree(q);
+            v->clear();
+        }
+        cudaFree(m->loss_part); cudaFree(m->y_dev); cudaFree(m->xin); cudaFree(m->tin);
+        m->loss_part = m->y_dev = m->xin = m->tin = nullptr;
+        m->n_cap = 0;
+        PLK_MCUDA(m, cudaMalloc(&m->loss_part, rows / kGM * kNetCtas * sizeof(float)), "allocate losses");
+        PLK_MCUDA(m, cudaMalloc(&m->y_dev, (size_t)rows * m->dims.back() * sizeof(float)), "allocate outputs");
+        PLK_MCUDA(m, cudaMalloc(&m->xin, (size_t)rows * m->dims.front() * sizeof(float)), "allocate inputs");
+        PLK_MCUDA(m, cudaMalloc(&m->tin, (size_t)rows * m->dims.back() * sizeof(float)), "allocate targets");
+        m->n_cap = rows;
+    }
+    if (train && m->n_act.empty())
+        for (int l = 0; l < n_layers(m); ++l) {
+            __nv_bfloat16* q = nullptr;
+            PLK_MCUDA(m, cudaMalloc(&q, (size_t)m->n_cap * m->pdims[l] * sizeof(__nv_bfloat16)), "allocate activations");
+            m->n_act.push_back(q);
+            PLK_MCUDA(m, cudaMalloc(&q, (size_t)m->n_cap * m->pdims[l + 1] * sizeof(__nv_bfloat16)), "allocate gradients");
+            m->n_dz.push_back(q);
+        }
+    return PLK_OK;
+}
+
+// One pass over `batch` rows: forward (t null), gradients, or an Adam step.
+// The loss is in the pinned block once the stream has drained (net_loss).
+plk_status net_pass(plk_mlp* m, int batch, const float* x, const float* t, bool adam, float lr, float* y_dev) {
+    plk_status s = net_ensure(m, batch, t != nullptr);
+    if (s != PLK_OK) return s;
+    const int L = n_layers(m);
+    const size_t xb = (size_t)batch * m->dims.front() * sizeof(float), tb = (size_t)batch * m->dims.back() * sizeof(float);
+    NetArgs n{};
+    n.L = L;
+    n.batch = batch;
+    n.backward = t != nullptr;
+    n.adam = adam;
+    if (xb + tb <= kHostRows) {
+        char* xs = m->host + 256;
+        char* ts = xs + (xb + 255) / 256 * 256;
+        std::memcpy(xs, x, xb);
+        if (t) std::memcpy(ts, t, tb);
+        n.x = reinterpret_cast<const float*>(m->host_dev + (xs - m->host));
+        n.t = reinterpret_cast<const float*>(m->host_dev + (ts - m->host));
+    } else {
+        PLK_MCUDA(m, cudaMemcpyAsync(m->xin, x, xb, cudaMemcpyHostToDevice, m->stream), "upload inputs");
+        if (t) PLK_MCUDA(m, cudaMemcpyAsync(m->tin, t, tb, cudaMemcpyHostToDevice, m->stream), "upload targets");
+        n.x = m->xin;
+        n.t = m->tin;
+    }
+    n.y = y_dev;
+    n.loss_part = m->loss_part;
+    n.loss = reinterpret_cast<float*>(m->host_dev);
+    n.fail = m->fail;
+    n.p = m->p; n.g = m->g; n.m = m->m; n.v = m->v;
+    int tiles = 0;
+    for (int l = 0; l < L; ++l) {
+        NetLayer& ly = n.layer[l];
+        ly.in = m->dims[l]; ly.out = m->dims[l + 1]; ly.pin = m->pdims[l]; ly.pout = m->pdims[l + 1];
+        ly.wf = m->wf[l]; ly.wt = m->wt[l];
+        ly.bias = m->p + m->b_off[l];
+        ly.w_off = m->w_off[l]; ly.b_off = m->b_off[l];
+        if (t) { ly.act = m->n_act[l]; ly.dz = m->n_dz[l]; }
+        ly.tiles_n = (ly.in + kUpN - 1) / kUpN;
+        ly.tile0 = tiles;
+        tiles += ly.tiles_n * ((ly.out + kGM - 1) / kGM);
+    }
+    const int row_ctas = (batch + kGM - 1) / kGM * kNetCtas;
+    rows_kernel<<<row_ctas, kNetThreads, kRowsSmem, m->stream>>>(n);
+    PLK_MCUDA(m, cudaGetLastError(), "row kernel");
+    if (!t) return PLK_OK;
+    if (n.adam) {
+        ++m->step;
+        n.lr = lr;
+        n.b1 = 0.9f; n.b2 = 0.999f; n.eps = 1e-8f;
+        n.c1 = 1.f - std::pow(n.b1, (float)m->step);
+        n.c2 = 1.f - std::pow(n.b2, (float)m->step);
+    }
+    update_kernel<<<tiles, kNetThreads, kUpSmem, m->stream>>>(n, row_ctas);
+    PLK_MCUDA(m, cudaGetLastError(), "update kernel");
+    return PLK_OK;
+}
+
+// The last pass's loss; a pass that gave up (NaN) leaves its flag cleared for
+// the next one.
+float net_loss(plk_mlp* m) {
+    const float v = *reinterpret_cast<const float*>(m->host);
+    if (std::isnan(v)) cudaMemsetAsync(m->fail, 0, sizeof(int), m->stream);
+    return v;
+}
+
 plk_status refresh_bf16(plk_mlp* m) {
+    if (m->narrow) return net_images(m);
     // BF16 copies of every layer's weights from the FP32 master
     std::vector<float> host(m->n_params);
     PLK_MCUDA(m, cudaMemcpy(host.data(), m->p, m->n_params * sizeof(float), cudaMemcpyDeviceToHost), "read weights");
@@ -456,11 +1197,28 @@ plk_status plk_mlp_create(plk_mlp** out, int device, int n_in, int n_hidden, int
     if (e == cudaSuccess) e = cudaMalloc(&m->m, off * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&m->v, off * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&m->loss, sizeof(float));
-    for (int l = 0; e == cudaSuccess && l + 1 < (int)m->dims.size(); ++l) {
+    m->narrow = (int)m->dims.size() - 1 <= kNetLayers && *std::max_element(m->pdims.begin(), m->pdims.end()) <= kNetWide;
+    for (int l = 0; !m->narrow && e == cudaSuccess && l + 1 < (int)m->dims.size(); ++l) {
         __nv_bfloat16* w = nullptr;
         e = cudaMalloc(&w, (size_t)m->pdims[l + 1] * m->pdims[l] * sizeof(__nv_bfloat16));
         m->wb.push_back(w);
     }
+    for (int l = 0; m->narrow && e == cudaSuccess && l + 1 < (int)m->dims.size(); ++l) {
+        // zero past the last CTA's columns
+        const size_t fb = net_image_elems(m->pdims[l + 1], m->pdims[l]) * sizeof(__nv_bfloat16);
+        const size_t tb = net_image_elems(m->pdims[l], m->pdims[l + 1]) * sizeof(__nv_bfloat16);
+        __nv_bfloat16 *f = nullptr, *w = nullptr;
+        e = cudaMalloc(&f, fb);
+        m->wf.push_back(f);
+        if (e == cudaSuccess) e = cudaMalloc(&w, tb);
+        m->wt.push_back(w);
+        if (e == cudaSuccess) e = cudaMemset(f, 0, fb);
+        if (e == cudaSuccess) e = cudaMemset(w, 0, tb);
+    }
+    if (m->narrow && e == cudaSuccess)
+        e = cudaFuncSetAttribute(rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsSmem);
+    if (m->narrow && e == cudaSuccess)
+        e = cudaFuncSetAttribute(update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpSmem);
     if (e != cudaSuccess) {
         delete m;
         return report_error(PLK_ERR_ALLOC, cudaGetErrorString(e));
@@ -515,8 +1273,16 @@ plk_status plk_mlp_set_params(plk_mlp* m, const float* in) {
 plk_status plk_mlp_forward(plk_mlp* m, int batch, const float* x, float* y) {
     if (!m || batch < 1 || !x || !y) return m ? mfail(m, PLK_ERR_ARG, "bad arguments to plk_mlp_forward") : PLK_ERR_ARG;
     PLK_MCUDA(m, cudaSetDevice(m->device), "cudaSetDevice");
-    plk_status s = ensure_batch(m, batch);
-    if (s != PLK_OK) return s;
+    plk_status s;
+    if (m->narrow) {
+        if ((s = net_ensure(m, batch, false)) != PLK_OK) return s;
+        if ((s = net_pass(m, batch, x, nullptr, false, 0.0f, m->y_dev)) != PLK_OK) return s;
+        PLK_MCUDA(m, cudaMemcpyAsync(y, m->y_dev, (size_t)batch * m->dims.back() * sizeof(float), cudaMemcpyDeviceToHost,
+                                     m->stream), "download outputs");
+        PLK_MCUDA(m, cudaStreamSynchronize(m->stream), "forward");
+        return PLK_OK;
+    }
+    if ((s = ensure_batch(m, batch)) != PLK_OK) return s;
     PLK_MCUDA(m, cudaMemcpyAsync(m->xin, x, (size_t)batch * m->dims.front() * sizeof(float), cudaMemcpyHostToDevice,
                                  m->stream), "upload inputs");
     if ((s = forward(m, batch)) != PLK_OK) return s;
@@ -530,8 +1296,18 @@ plk_status plk_mlp_forward(plk_mlp* m, int batch, const float* x, float* y) {
 plk_status plk_mlp_gradients(plk_mlp* m, int batch, const float* x, const float* t, float* grad, float* loss) {
     if (!m || batch < 1 || !x || !t) return m ? mfail(m, PLK_ERR_ARG, "bad arguments to plk_mlp_gradients") : PLK_ERR_ARG;
     PLK_MCUDA(m, cudaSetDevice(m->device), "cudaSetDevice");
-    plk_status s = ensure_batch(m, batch);
-    if (s != PLK_OK) return s;
+    plk_status s;
+    if (m->narrow) {
+        if ((s = net_pass(m, batch, x, t, false, 0.0f, nullptr)) != PLK_OK) return s;
+        if (grad)
+            PLK_MCUDA(m, cudaMemcpyAsync(grad, m->g, m->n_params * sizeof(float), cudaMemcpyDeviceToHost, m->stream),
+                      "download gradients");
+        PLK_MCUDA(m, cudaStreamSynchronize(m->stream), "gradients");
+        const float v = net_loss(m);
+        if (loss) *loss = v;
+        return PLK_OK;
+    }
+    if ((s = ensure_batch(m, batch)) != PLK_OK) return s;
     PLK_MCUDA(m, cudaMemcpyAsync(m->xin, x, (size_t)batch * m->dims.front() * sizeof(float), cudaMemcpyHostToDevice,
                                  m->stream), "upload inputs");
     PLK_MCUDA(m, cudaMemcpyAsync(m->tin, t, (size_t)batch * m->dims.back() * sizeof(float), cudaMemcpyHostToDevice,
@@ -547,8 +1323,16 @@ plk_status plk_mlp_gradients(plk_mlp* m, int batch, const float* x, const float*
 }
 
 plk_status plk_mlp_train_step(plk_mlp* m, int batch, const float* x, const float* t, float lr, float* loss) {
-    plk_status s = plk_mlp_gradients(m, batch, x, t, nullptr, nullptr);
-    if (s != PLK_OK) return s;
+    plk_status s;
+    if (m && m->narrow && batch >= 1 && x && t) {
+        PLK_MCUDA(m, cudaSetDevice(m->device), "cudaSetDevice");
+        if ((s = net_pass(m, batch, x, t, true, lr, nullptr)) != PLK_OK) return s;
+        PLK_MCUDA(m, cudaStreamSynchronize(m->stream), "train step");
+        const float v = net_loss(m);
+        if (loss) *loss = v;
+        return PLK_OK;
+    }
+    if ((s = plk_mlp_gradients(m, batch, x, t, nullptr, nullptr)) != PLK_OK) return s;
     ++m->step;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - std::pow(b1, (float)m->step), c2 = 1.f - std::pow(b2, (float)m->step);
