@@ -509,9 +509,16 @@ void clear_counters(plk_handle* h) {
     if (h->d_done.p && h->d_done.bytes) cudaMemsetAsync(h->d_done.p, 0, h->d_done.bytes, h->stream);
 }
 
+// What a node-state pass asks of run_prune, and what it finds afterwards.
+struct NodePass {
+    bool marginal;  // the pre-order pass follows
+    void* cond;     // the conditional vectors of every internal node, or null where any is set
+    bool any;       // prune_any_kernel ran: its output (marginal: the messages, in d_cond) is there
+};
+
 // Runs the post-order pass (P(t) already built); store != null asks for the
-// conditional vectors of every internal node in *store.
-plk_status run_prune(plk_handle* h, int precision, void** store, cudaEvent_t* after_prune = nullptr) {
+// node states or what the pre-order pass needs.
+plk_status run_prune(plk_handle* h, int precision, NodePass* store, cudaEvent_t* after_prune = nullptr) {
     // a streamed alignment's codes: a tuned warp-independent FP32 pass starts
     // while they land and waits per tile; every other pass after all of them
     bool streamed = false;
@@ -525,7 +532,8 @@ plk_status run_prune(plk_handle* h, int precision, void** store, cudaEvent_t* af
     }
     const size_t tsz = precision == PLK_FP64 ? sizeof(double) : sizeof(float);
     const size_t vec_bytes = (size_t)h->post.size() * h->C * h->n_sites * h->S * tsz;
-    const int any_blocks = prune_any_blocks(prune_args(h, precision), h->S, precision, store != nullptr);
+    const int any_blocks =
+        prune_any_blocks(prune_args(h, precision), h->S, precision, store != nullptr, store && store->marginal);
     // the smallest tile elsewhere: 64 sites (prune4p, two threads per site)
     const int blocks = std::max((h->n_sites + 63) / 64, any_blocks);
     PLK_CUDA(h, h->d_site_lnl.ensure(sizeof(double) * h->n_sites), "allocate site lnL");
@@ -566,9 +574,11 @@ plk_status run_prune(plk_handle* h, int precision, void** store, cudaEvent_t* af
         }
         a.variant = h->variant;
     } else if (a.use_any) {
-        if (store) {
-            PLK_CUDA(h, h->d_cond.ensure(vec_bytes), "allocate node vectors");
-            a.cond = h->d_cond.p;
+        if (store && store->marginal) {
+            PLK_CUDA(h, h->d_cond.ensure(vec_bytes), "allocate node messages");
+            a.msg = h->d_cond.p;
+        } else if (store) {
+            a.nodes = h->d_nodes_out.as<double>();
         }
     } else if (!fused) {
         PLK_CUDA(h, h->d_work.ensure(vec_bytes), "allocate work vectors");
@@ -623,7 +633,10 @@ plk_status run_prune(plk_handle* h, int precision, void** store, cudaEvent_t* af
         return cuda_fail(h, le, "post-order kernel launch");
     }
     if (after_prune) PLK_CUDA(h, cudaEventRecord(*after_prune, h->stream), "cudaEventRecord");
-    if (store) *store = a.cond;
+    if (store) {
+        store->cond = a.cond;
+        store->any = a.use_any != 0;
+    }
     return PLK_OK;
 }
 
@@ -1159,18 +1172,20 @@ plk_status plk_node_states(plk_handle* h, int mode, int precision, double* out) 
     }
     if (h->bad_tip) return fail(h, PLK_ERR_TIP, "a tip cell allows no state of the model");
     if ((s = build_pmats(h)) != PLK_OK) return s;
-    void* cond = nullptr;
-    if ((s = run_prune(h, precision, &cond)) != PLK_OK) return s;
     const int n_int = (int)h->post.size();
     const size_t out_n = (size_t)n_int * h->n_sites * h->S;
     PLK_CUDA(h, h->d_nodes_out.ensure(out_n * sizeof(double)), "allocate node output");
+    NodePass pass{mode == PLK_NODES_MARGINAL, nullptr, false};
+    if ((s = run_prune(h, precision, &pass)) != PLK_OK) return s;
     if (mode == PLK_NODES_COND) {
-        PLK_CUDA(h, launch_cond_normalise(cond, h->d_catw.as<double>(), n_int, h->C, h->n_sites, h->S, precision,
+        if (!pass.any)
+            PLK_CUDA(h, launch_cond_normalise(pass.cond, h->d_catw.as<double>(), n_int, h->C, h->n_sites, h->S, precision,
                                           h->d_nodes_out.as<double>(), h->stream),
                  "normalise kernel launch");
     } else {
         const size_t tsz = precision == PLK_FP64 ? sizeof(double) : sizeof(float);
-        PLK_CUDA(h, h->d_outside.ensure((size_t)n_int * h->C * h->n_sites * h->S * tsz), "allocate outside vectors");
+        if (!pass.any)
+            PLK_CUDA(h, h->d_outside.ensure((size_t)n_int * h->C * h->n_sites * h->S * tsz), "allocate outside vectors");
         PreorderArgs p{};
         const bool fp64 = precision == PLK_FP64;
         p.order = h->d_order.as<int>(); p.left = h->d_left.as<int>(); p.right = h->d_right.as<int>();
@@ -1180,8 +1195,10 @@ plk_status plk_node_states(plk_handle* h, int mode, int precision, double* out) 
         p.P = fp64 ? (const void*)h->d_P64.p : (const void*)h->d_P32.p;
         p.tipT = fp64 ? (const void*)h->d_tip64.p : (const void*)h->d_tip32.p;
         p.root_w = h->d_rootw.as<double>(); p.cat_w = h->d_catw.as<double>();
-        p.cond = cond; p.outside = h->d_outside.p; p.out = h->d_nodes_out.as<double>();
-        PLK_CUDA(h, launch_preorder(p, precision, h->stream), "pre-order kernel launch");
+        p.cond = pass.cond; p.outside = h->d_outside.p; p.out = h->d_nodes_out.as<double>();
+        p.n_nodes = h->n_nodes;
+        PLK_CUDA(h, pass.any ? launch_down_any(p, h->d_cond.p, precision, h->stream) : launch_preorder(p, precision, h->stream),
+                 "pre-order kernel launch");
     }
     if (!h->patterns) {
         PLK_CUDA(h, cudaMemcpyAsync(out, h->d_nodes_out.p, out_n * sizeof(double), cudaMemcpyDeviceToHost, h->stream),

@@ -237,6 +237,11 @@ struct PruneArgs {
     // BF16 products (kind::f16, FP32 accumulate).
     int variant;
     int use_any;               // run prune_any_kernel (prune_any_blocks > 0)
+    // with use_any, for the node states: the messages of the internal nodes
+    // ([node][site][C][S], for launch_down_any) or the normalised conditional
+    // vectors ([rank][site][S]); null otherwise
+    void* msg;
+    double* nodes;
     int n_nodes;
     void* scratch;             // kernel-specific scratch (prune20_scratch_bytes)
     // The last CTA of the kernel that stores the block sums adds them up into
@@ -318,7 +323,9 @@ cudaError_t launch_prune4s(const PruneArgs& a, int spt, int* n_blocks, cudaStrea
 // staged.  The number of blocks with which it takes this evaluation, 0 where
 // another kernel does (the tuned FP32 forms; 4 states once a thread per site
 // fills the chip; shapes whose matrices do not fit in shared memory).
-int prune_any_blocks(const PruneArgs& a, int S, int precision, bool store);
+// nodes: a node-state pass, which it takes wherever its tables fit (with the
+// pre-order pass after it, where `marginal`).
+int prune_any_blocks(const PruneArgs& a, int S, int precision, bool nodes, bool marginal = false);
 cudaError_t launch_prune_any(const PruneArgs& a, int S, int precision, int* n_blocks, cudaStream_t st);
 // Chooses the kernel for (S, C, precision); returns the number of blocks used
 // for the partial sums in *n_blocks.
@@ -349,7 +356,11 @@ struct PreorderArgs {
     const void* cond;   // T [n_int][C][n_sites][S]
     void* outside;      // T [n_int][C][n_sites][S]
     double* out;        // [n_int][n_sites][S] normalised
+    int n_nodes;
 };
+// The pre-order pass after a prune_any pass that left its messages in msg
+// (plk_prune_any.cuh).
+cudaError_t launch_down_any(const PreorderArgs& a, void* msg, int precision, cudaStream_t st);
 cudaError_t launch_preorder(const PreorderArgs& a, int precision, cudaStream_t st);
 cudaError_t launch_cond_normalise(const void* cond, const double* cat_w, int n_int, int C,
                                   int n_sites, int S, int precision, double* out,

@@ -30,21 +30,22 @@ struct AnyPlan {
 };
 
 // H, warps per CTA and the tables' place for these counts; H = 0 where
-// nothing fits.
-AnyPlan any_plan(const PruneArgs& a, int S, bool fp64, int sms) {
+// nothing fits.  smem(H, launch): the bytes of a CTA.
+template <class Smem>
+AnyPlan any_plan(int S, int C, bool fp64, int n_sites, int n_codes, int max_depth, int sms, Smem smem) {
     AnyPlan best;
-    const int tsz = fp64 ? 8 : 4, C = a.C;
+    const int tsz = fp64 ? 8 : 4;
     for (int H = 1; H <= 4; H *= 2) {
         if (C * H > 32 || H > S || (H == 1 && S > 8)) continue;
         const int R = (S + H - 1) / H, W = 32 / (C * H);
-        const long long warps = ((long long)a.n_sites + W - 1) / W;
+        const long long warps = ((long long)n_sites + W - 1) / W;
         const int per_sm = (int)((warps + sms - 1) / sms);
         AnyPlan p;
         p.H = H;
-        p.launch.depth = std::max(a.max_depth, 1);
+        p.launch.depth = std::max(max_depth, 1);
         // tip tables through the ring while they are of the size of P(t)
-        p.launch.stage_tips = a.n_codes <= 2 * S + 8 ? 1 : 0;
-        const int child = std::max(C * S * S, p.launch.stage_tips ? C * a.n_codes * S : 0);
+        p.launch.stage_tips = n_codes <= 2 * S + 8 ? 1 : 0;
+        const int child = std::max(C * S * S, p.launch.stage_tips ? C * n_codes * S : 0);
         p.launch.child_elems = (child * tsz + 15) / 16 * 16 / tsz;
         // one CTA per SM while eight warps hold its sites: a table brought in
         // once then serves every warp of the SM
@@ -55,7 +56,7 @@ AnyPlan any_plan(const PruneArgs& a, int S, bool fp64, int sms) {
         p.launch.slots = 0;
         p.launch.warps = want;
         if (S <= 8) {
-            const size_t need = dev::any_smem(S, H, fp64, p.launch, a);
+            const size_t need = smem(H, p.launch);
             fits = need <= (per_sm <= kAnyWarps ? kAnySmem : kAnySmem / 2);
         }
         for (int slots = 3; slots >= 2 && !fits; --slots)
@@ -63,7 +64,7 @@ AnyPlan any_plan(const PruneArgs& a, int S, bool fp64, int sms) {
                 if (slots == 3 && w < (want + 1) / 2) break;  // rather two slots than half the warps
                 p.launch.slots = slots;
                 p.launch.warps = w;
-                fits = dev::any_smem(S, H, fp64, p.launch, a) <= kAnySmem;
+                fits = smem(H, p.launch) <= kAnySmem;
             }
         if (!fits) continue;
         // FP64: the SM's FP64 pipe takes 16 cycles a warp instruction; FP32:
@@ -76,22 +77,39 @@ AnyPlan any_plan(const PruneArgs& a, int S, bool fp64, int sms) {
     return best;
 }
 
+AnyPlan up_plan(const PruneArgs& a, int S, bool fp64, bool cond_nodes, int sms) {
+    return any_plan(S, a.C, fp64, a.n_sites, a.n_codes, a.max_depth, sms, [&](int H, dev::AnyLaunch p) {
+        static double some;
+        p.nodes = cond_nodes ? &some : nullptr;  // only its presence counts
+        return dev::any_smem(S, H, fp64, p, a);
+    });
+}
+AnyPlan down_plan(const PreorderArgs& a, int S, bool fp64, int sms) {
+    return any_plan(S, a.C, fp64, a.n_sites, a.n_codes, 0, sms,
+                    [&](int H, const dev::AnyLaunch& p) { return dev::any_down_smem(S, H, fp64, p, a); });
+}
+
 }  // namespace
 
-int prune_any_blocks(const PruneArgs& a, int S, int precision, bool store) {
+int prune_any_blocks(const PruneArgs& a, int S, int precision, bool nodes, bool marginal) {
     const bool fp64 = precision == PLK_FP64;
     if (S < 2 || S > kMaxStates || a.C > kMaxCats || a.n_ops < 1) return 0;
-    if (!fp64 && !store && ((S == 4 && a.C <= 8) || S == 20)) return 0;  // the tuned FP32 forms
+    if (!fp64 && !nodes && ((S == 4 && a.C <= 8) || S == 20)) return 0;  // the tuned FP32 forms
     const int sms = any_sm_count();
-    const AnyPlan p = any_plan(a, S, fp64, sms);
+    const AnyPlan p = up_plan(a, S, fp64, nodes && !marginal, sms);
     if (p.H == 0) return 0;
-    if (S == 4 && a.C <= 8) {
+    if (marginal) {
+        PreorderArgs d{};
+        d.n_int = a.n_int; d.n_tips = a.n_tips; d.n_nodes = a.n_nodes; d.n_sites = a.n_sites; d.n_codes = a.n_codes;
+        d.C = a.C;
+        if (down_plan(d, S, fp64, sms).H == 0) return 0;
+    }
+    if (S == 4 && a.C <= 8 && !nodes) {
         // prune4_kernel, a thread per site in 128-thread CTAs, issues the same
         // FP64 instructions (32 per category and op) with less around them: it
         // stays once its CTAs fill the SMs as evenly
         const long long blocks = (a.n_sites + 127) / 128;
-        const double per_op = fp64 ? 16.0 * 32 * a.C : 0.25 * 1.5 * 64 * a.C;
-        const double cost4 = (double)((blocks + sms - 1) / sms) * 4 * per_op;
+        const double cost4 = (double)((blocks + sms - 1) / sms) * 4 * 16.0 * 32 * a.C;
         if (p.cost > 0.9 * cost4) return 0;
     }
     return p.blocks;
@@ -99,14 +117,28 @@ int prune_any_blocks(const PruneArgs& a, int S, int precision, bool store) {
 
 cudaError_t launch_prune_any(const PruneArgs& a, int S, int precision, int* n_blocks, cudaStream_t st) {
     const bool fp64 = precision == PLK_FP64;
-    const AnyPlan p = any_plan(a, S, fp64, any_sm_count());
+    AnyPlan p = up_plan(a, S, fp64, a.nodes != nullptr, any_sm_count());
     if (p.H == 0) return cudaErrorInvalidConfiguration;
+    p.launch.msg = a.msg;
+    p.launch.nodes = a.nodes;
     *n_blocks = p.blocks;
     if (fp64)
         return S <= 12 ? launch_any64_lo(a, S, p.H, p.launch, p.blocks, st)
                        : launch_any64_hi(a, S, p.H, p.launch, p.blocks, st);
     return S <= 12 ? launch_any32_lo(a, S, p.H, p.launch, p.blocks, st)
                    : launch_any32_hi(a, S, p.H, p.launch, p.blocks, st);
+}
+
+cudaError_t launch_down_any(const PreorderArgs& a, void* msg, int precision, cudaStream_t st) {
+    const bool fp64 = precision == PLK_FP64;
+    AnyPlan p = down_plan(a, a.S, fp64, any_sm_count());
+    if (p.H == 0) return cudaErrorInvalidConfiguration;
+    p.launch.msg = msg;
+    if (fp64)
+        return a.S <= 12 ? launch_down64_lo(a, a.S, p.H, p.launch, p.blocks, st)
+                         : launch_down64_hi(a, a.S, p.H, p.launch, p.blocks, st);
+    return a.S <= 12 ? launch_down32_lo(a, a.S, p.H, p.launch, p.blocks, st)
+                     : launch_down32_hi(a, a.S, p.H, p.launch, p.blocks, st);
 }
 
 }  // namespace plk

@@ -45,6 +45,9 @@ struct AnyLaunch {
     int child_elems; // T elements between the two children of a slot
     int depth;       // spill-stack slots
     int stage_tips;  // tip tables go through the ring (else tip rows come from global memory)
+    // node states (plk_node_states)
+    void* msg;       // T [internal node][site][C][S]: messages to the parents, or null
+    double* nodes;   // [rank][site][S]: normalised conditional vectors, or null
 };
 
 template <typename T, int S, int H>
@@ -61,16 +64,31 @@ struct AnyShape {
 };
 
 // Shared memory of a launch: tables (the ring [slots][2][child], or all P(t)
-// then all tip tables) | [warps] exchange rows | [depth][warps][R][32] spilled
-// rows | ops | tip codes [tip][sites of the CTA].
-inline size_t any_smem(int S, int H, bool fp64, const AnyLaunch& p, const PruneArgs& a) {
-    const int R = (S + H - 1) / H, V = fp64 ? (S % 2 == 0 ? 2 : 1) : (S % 4 == 0 ? 4 : (S % 2 == 0 ? 2 : 1));
+// then all tip tables) | [warps] exchange rows | what the pass itself needs |
+// [warps] pairs of vectors and sums of the node output (node_out) | ops or node
+// table | tip codes [tip][sites of the CTA].
+inline size_t any_node_bytes(int S, int C, int H, bool fp64) {  // of a warp
+    return (size_t)(32 / H) * S * (fp64 ? 16 : 8) + (size_t)(32 / (C * H)) * (S + 1) * 8;
+}
+inline size_t any_base_smem(int S, int H, bool fp64, const AnyLaunch& p, int C, int n_nodes, int n_tips, int n_codes) {
+    const int V = fp64 ? (S % 2 == 0 ? 2 : 1) : (S % 4 == 0 ? 4 : (S % 2 == 0 ? 2 : 1));
     const int SX = (S / V) % 2 == 1 ? S : S + V;
     const size_t exch = H == 1 && S <= 8 ? 0 : 2 * (size_t)(32 / H) * SX, tsz = fp64 ? 8 : 4;
     const size_t tables = p.slots ? (size_t)p.slots * 2 * p.child_elems
-                                  : ((size_t)a.n_nodes * a.C * S * S + 3) / 4 * 4 + (size_t)a.n_tips * a.C * a.n_codes * S;
-    return (tsz * tables + 15) / 16 * 16 + tsz * (p.warps * exch + (size_t)p.depth * p.warps * R * 32) +
-           (size_t)a.n_ops * sizeof(Op) + (size_t)a.n_tips * p.warps * (32 / (a.C * H));
+                                  : ((size_t)n_nodes * C * S * S + 3) / 4 * 4 + (size_t)n_tips * C * n_codes * S;
+    return (tsz * tables + 15) / 16 * 16 + tsz * p.warps * exch + (size_t)n_tips * p.warps * (32 / (C * H));
+}
+// the post-order pass: its spill stack [depth][warps][R][32] and op list
+inline size_t any_smem(int S, int H, bool fp64, const AnyLaunch& p, const PruneArgs& a) {
+    const int R = (S + H - 1) / H;
+    return any_base_smem(S, H, fp64, p, a.C, a.n_nodes, a.n_tips, a.n_codes) +
+           (size_t)(fp64 ? 8 : 4) * p.depth * p.warps * R * 32 + (size_t)a.n_ops * sizeof(Op) +
+           (p.nodes ? (p.warps * any_node_bytes(S, a.C, H, fp64) + 15) / 16 * 16 : 0);
+}
+// the pre-order pass: its node table, int4 a node
+inline size_t any_down_smem(int S, int H, bool fp64, const AnyLaunch& p, const PreorderArgs& a) {
+    return any_base_smem(S, H, fp64, p, a.C, a.n_nodes, a.n_tips, a.n_codes) + (size_t)a.n_int * 16 +
+           (p.warps * any_node_bytes(S, a.C, H, fp64) + 15) / 16 * 16;
 }
 
 template <int BYTES>
@@ -103,7 +121,109 @@ __device__ __forceinline__ T row_step(T acc, T x, T p, bool first) {
     return EXACT ? add_rn(acc, mul_rn(x, p)) : fma(x, p, acc);
 }
 
-template <typename T, int S, int H, bool kRes>
+// the category weights in shared memory, FP64 and as two FP32 parts
+struct NodeWeights {
+    double w[kMaxCats];
+    float2 w2[kMaxCats];
+    __device__ __forceinline__ void load(const double* cat_w, int C) {
+        if ((int)threadIdx.x < C) {
+            const double v = cat_w[threadIdx.x];
+            w[threadIdx.x] = v;
+            w2[threadIdx.x] = make_float2((float)v, (float)(v - (double)(float)v));
+        }
+    }
+};
+
+// One node's normalised output for the warp's sites: p_s proportional to
+// sum_k w_k O[k][s] c[k][s] (O = 1 for the conditional vectors).  Every lane
+// hands its rows in (its category's, h R ..) and takes (site, state) pairs out,
+// so that a pair's sum over the categories runs in one lane and the doubles go
+// out in order.  In FP64 the sum, the total and the division are FP64, the
+// operations of the reference's order.  In FP32 they would put ten FP64
+// instructions a value on a pipe that takes 16 cycles for each (the larger part
+// of the pass); the same quantities are carried as two FP32 parts (products and
+// sums with their exact rounding errors, Dekker 1971 / Knuth's TwoSum), 2^-45
+// relative, under vectors that are good to 2^-22.
+template <typename T, int S, int H>
+struct NodeOut {
+    T* oc;         // [site * C + k][S][2]
+    double* sums;  // [site][S], then [site]
+    const double* w;  // category weights, and as two FP32 parts
+    const float2* w2;
+
+    __device__ __forceinline__ void put(int row, int s, T o, T c) const {
+        oc[(row * S + s) * 2] = o;
+        oc[(row * S + s) * 2 + 1] = c;
+    }
+    // (hi, lo) + x + y with hi's rounding error kept in lo
+    static __device__ __forceinline__ void add2(float& hi, float& lo, float x, float y) {
+        float t, e;
+        two_sum_f(hi, x, t, e);
+        hi = t;
+        lo = __fadd_rn(lo, __fadd_rn(e, y));
+    }
+    // all lanes of the warp; out = this node's doubles, site0 the warp's first site
+    __device__ __forceinline__ void write(int C, int W, int site0, int n_sites, double* out) const {
+        const int lane = threadIdx.x & 31;
+        __syncwarp();
+        if constexpr (std::is_same<T, double>::value) {
+            double* tot = sums + W * S;
+            for (int i = lane; i < W * S; i += 32) {
+                double m = 0.0;
+                for (int k = 0; k < C; ++k) {
+                    const T* v = oc + ((i / S * C + k) * S + i % S) * 2;
+                    m = fma(w[k] * v[0], v[1], m);
+                }
+                sums[i] = m;
+            }
+            __syncwarp();
+            if (lane < W) {
+                double t = 0.0;
+                for (int s = 0; s < S; ++s) t += sums[lane * S + s];
+                tot[lane] = t;
+            }
+            __syncwarp();
+            for (int i = lane; i < W * S; i += 32)
+                if (site0 + i / S < n_sites) out[(size_t)site0 * S + i] = sums[i] / tot[i / S];
+        } else {
+            float2* sum2 = reinterpret_cast<float2*>(sums);
+            float2* tot = sum2 + W * S;
+            for (int i = lane; i < W * S; i += 32) {
+                float hi = 0.0f, lo = 0.0f;
+                for (int k = 0; k < C; ++k) {
+                    const float2 v = *reinterpret_cast<const float2*>(oc + ((i / S * C + k) * S + i % S) * 2);
+                    const float wh = w2[k].x, wl = w2[k].y;
+                    // 2^40 on both keeps products of small entries off the subnormals
+                    const float o = v.x * 1099511627776.0f, c = v.y * 1099511627776.0f;
+                    const float p = __fmul_rn(o, c), pe = fmaf(o, c, -p);
+                    const float q = __fmul_rn(p, wh);
+                    const float qe = __fadd_rn(fmaf(p, wh, -q), fmaf(p, wl, __fmul_rn(pe, wh)));
+                    add2(hi, lo, q, qe);
+                }
+                sum2[i] = make_float2(hi, lo);
+            }
+            __syncwarp();
+            if (lane < W) {
+                float hi = 0.0f, lo = 0.0f;
+                for (int s = 0; s < S; ++s) add2(hi, lo, sum2[lane * S + s].x, sum2[lane * S + s].y);
+                tot[lane] = make_float2(hi, lo);
+            }
+            __syncwarp();
+            for (int i = lane; i < W * S; i += 32) {
+                const float2 m = sum2[i], t = tot[i / S];
+                // a quotient to 2^-22 and the remainder's, whose leading part is exact
+                const float inv = __fdividef(1.0f, t.x);
+                const float q1 = __fmul_rn(m.x, inv);
+                const float r = __fsub_rn(__fadd_rn(fmaf(-q1, t.x, m.x), m.y), __fmul_rn(q1, t.y));
+                const float q2 = __fmul_rn(r, inv);
+                if (site0 + i / S < n_sites) out[(size_t)site0 * S + i] = (double)q1 + (double)q2;
+            }
+        }
+        __syncwarp();  // the next node's values may be put
+    }
+};
+
+template <typename T, int S, int H, bool kRes, bool kNodes>
 __global__ void __launch_bounds__(256) prune_any_kernel(PruneArgs a, AnyLaunch pl) {
     using Sh = AnyShape<T, S, H>;
     constexpr int R = Sh::R, V = Sh::V, SX = Sh::SX;
@@ -130,7 +250,19 @@ __global__ void __launch_bounds__(256) prune_any_kernel(PruneArgs a, AnyLaunch p
     T* const stack0 = work + pl.warps * Sh::kExch;
     T* stack = stack0 + warp * R * 32 + lane;
     const int stack_slot = pl.warps * R * 32;
-    Op* const s_ops = reinterpret_cast<Op*>(stack0 + pl.depth * stack_slot);
+    unsigned char* after = reinterpret_cast<unsigned char*>(stack0 + pl.depth * stack_slot);
+    NodeOut<T, S, H> node{nullptr, nullptr, nullptr, nullptr};
+    if (kNodes && pl.nodes) {  // doubles first, then the pairs of T
+        __shared__ NodeWeights s_w;
+        s_w.load(a.cat_w, C);
+        node.w = s_w.w;
+        node.w2 = s_w.w2;
+        const int per = (32 / H) * S * 2 * (int)sizeof(T) + W * (S + 1) * 8;
+        node.sums = reinterpret_cast<double*>(after + warp * per);
+        node.oc = reinterpret_cast<T*>(after + warp * per + W * (S + 1) * 8);
+        after += (pl.warps * per + 15) / 16 * 16;
+    }
+    Op* const s_ops = reinterpret_cast<Op*>(after);
     uint8_t* const s_codes = reinterpret_cast<uint8_t*>(s_ops + n_ops);
     T* const my_row = xch + (site_l * C + k) * SX;  // this site and category's exchange row
     T* const my_row2 = my_row + (Sh::kRegX ? 0 : Sh::kRows * SX);
@@ -291,6 +423,21 @@ __global__ void __launch_bounds__(256) prune_any_kernel(PruneArgs a, AnyLaunch p
         else product(b0, x0, my_row, d0);
         if (s1 >= 0) tip_rows(s1, b1, d1);
         else if (s1 == kSrcAcc) product(b1, acc, my_row2, d1);
+        if (kNodes && pl.msg && valid) {  // the internal children's messages, for the pre-order pass
+            T* const m = static_cast<T*>(pl.msg);
+            if (s0 < 0) {
+                T* dst = m + (((size_t)(oa.z - a.n_tips) * a.n_sites + site) * C + k) * S + h * R;
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    if (kEven || h * R + r < S) dst[r] = d0[r];
+            }
+            if (s1 == kSrcAcc) {
+                T* dst = m + (((size_t)(oa.w - a.n_tips) * a.n_sites + site) * C + k) * S + h * R;
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    if (kEven || h * R + r < S) dst[r] = d1[r];
+            }
+        }
         T mx = T(0);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -311,11 +458,12 @@ __global__ void __launch_bounds__(256) prune_any_kernel(PruneArgs a, AnyLaunch p
                 scale_e += e;
             }
         }
-        if (a.cond && valid) {
-            T* dst = static_cast<T*>(a.cond) + (((size_t)oa.y * C + k) * a.n_sites + site) * S + h * R;
+        if (kNodes && pl.nodes) {
+            if (lane < W * G)
 #pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (kEven || h * R + r < S) dst[r] = acc[r];
+                for (int r = 0; r < R; ++r)
+                    if (kEven || h * R + r < S) node.put(site_l * C + k, h * R + r, T(1), acc[r]);
+            node.write(C, W, blockIdx.x * tile + warp * W, a.n_sites, pl.nodes + (size_t)oa.y * a.n_sites * S);
         }
         if (ob.z) {
 #pragma unroll
@@ -382,9 +530,269 @@ __global__ void __launch_bounds__(256) prune_any_kernel(PruneArgs a, AnyLaunch p
     if (a.grid_done) finish_grid_sum64(a.block_sum, a.grid_done, a.lnl_out);
 }
 
+// The pre-order pass and the normalised marginals (absent in the reference).
+// At node u, from the root down: cond(u) is the product of its children's
+// messages (prune_any left them in pl.msg), the output the normalised sum over
+// the categories of Out(u) x cond(u), and every internal child v gets
+//   Out(v)[b] = sum_i Out(u)[i] D_w[i] P_v[i][b],  i ascending, w its sibling,
+// rescaled like a conditional vector.  The child visited next (rank r - 1) finds
+// its vector in registers; another one's takes the place of its message, which
+// no one reads again.  Lanes, tables and codes as in prune_any_kernel; the next
+// node's messages are loaded while this one is worked on.  One thread a site
+// with vectors in local memory took 1,161 us for 100 x 10,000 (C = 4, FP32) and
+// recomputed D_w; this takes 200 us (and the pass before it 94 instead of 168).
 template <typename T, int S, int H, bool kRes>
+__global__ void __launch_bounds__(256) down_any_kernel(PreorderArgs a, AnyLaunch pl) {
+    using Sh = AnyShape<T, S, H>;
+    constexpr int R = Sh::R, SX = Sh::SX;
+    constexpr bool kEven = R * H == S;
+    constexpr bool kPre = R * (int)sizeof(T) <= 48;  // the next node's messages wait in registers
+    extern __shared__ __align__(16) unsigned char any_smem_raw[];
+    const int C = a.C, G = C * H, W = 32 / G;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int l = lane < W * G ? lane : lane - W * G;
+    const int site_l = l / G, rem = l % G, k = rem / H, h = rem % H;
+    const int tile = pl.warps * W, col = warp * W + site_l;
+    const int site = blockIdx.x * tile + col;
+    const bool valid = lane < W * G && site < a.n_sites;
+    const int n_int = a.n_int, n_tips = a.n_tips;
+    const int p_elems = C * S * S, t_elems = C * a.n_codes * S;
+    T* const tables = reinterpret_cast<T*>(any_smem_raw);
+    const int tips_at = kRes ? (a.n_nodes * p_elems + 3) & ~3 : 0;
+    const size_t table_elems = kRes ? (size_t)tips_at + (size_t)n_tips * t_elems : (size_t)pl.slots * 2 * pl.child_elems;
+    T* const work = reinterpret_cast<T*>(any_smem_raw + (table_elems * sizeof(T) + 15) / 16 * 16);
+    T* const xch = work + warp * Sh::kExch;
+    unsigned char* after = reinterpret_cast<unsigned char*>(work + pl.warps * Sh::kExch);
+    const int per = (32 / H) * S * 2 * (int)sizeof(T) + W * (S + 1) * 8;
+    __shared__ NodeWeights s_w;
+    s_w.load(a.cat_w, C);
+    const NodeOut<T, S, H> node{reinterpret_cast<T*>(after + warp * per + W * (S + 1) * 8),
+                                reinterpret_cast<double*>(after + warp * per), s_w.w, s_w.w2};
+    int4* const s_kids = reinterpret_cast<int4*>(after + (pl.warps * per + 15) / 16 * 16);  // left, right, id
+    uint8_t* const s_codes = reinterpret_cast<uint8_t*>(s_kids + n_int);
+    T* const my_row = xch + (site_l * C + k) * SX;
+    const T* P = static_cast<const T*>(a.P);
+    const T* tipT = static_cast<const T*>(a.tipT);
+    T* const msg = static_cast<T*>(pl.msg) + ((size_t)min(site, a.n_sites - 1) * C + k) * S;
+    const size_t node_elems = (size_t)a.n_sites * C * S;
+    const int code_mask = S <= 4 ? (1 << S) - 1 : 255;
+    const int p_unit = copy_unit(p_elems * (int)sizeof(T)), t_unit = copy_unit(t_elems * (int)sizeof(T));
+    const unsigned site_mask = (G == 32 ? 0xffffffffu : ((1u << G) - 1u)) << (site_l * G);
+
+    for (int r = threadIdx.x; r < n_int; r += blockDim.x) {
+        const int u = a.order[r];
+        s_kids[r] = make_int4(a.left[u], a.right[u], u, 0);
+    }
+    if constexpr (kRes) {
+        auto all = [&](T* dst, const T* src, int elems) {
+            char* d = reinterpret_cast<char*>(dst);
+            const char* g = reinterpret_cast<const char*>(src);
+            const int bytes = elems * (int)sizeof(T), whole = bytes / 16 * 16;
+#pragma unroll 8
+            for (int i = threadIdx.x * 16; i < whole; i += blockDim.x * 16) cp_async16(d + i, g + i);
+            stage_bytes(d + whole, g + whole, bytes - whole, 4);
+        };
+        all(tables, P, a.n_nodes * p_elems);
+        all(tables + tips_at, tipT, n_tips * t_elems);
+    }
+    cp_async_commit();
+    {
+        const int rows = blockDim.x / tile, s = threadIdx.x % tile;
+        const uint8_t* src = a.codes + min(blockIdx.x * tile + s, a.n_sites - 1);
+        int t = threadIdx.x / tile;
+        if (t < rows)
+#pragma unroll 4
+            for (; t < n_tips; t += rows) s_codes[t * tile + s] = src[(size_t)t * a.site_stride] & code_mask;
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    auto stage = [&](int r, int slot) {  // both children's tables of the node of rank r
+        const int4 kd = s_kids[r];
+        for (int c = 0; c < 2; ++c) {
+            const int v = c ? kd.y : kd.x;
+            char* d = reinterpret_cast<char*>(tables + (slot * 2 + c) * pl.child_elems);
+            if (v >= n_tips)
+                stage_bytes(d, reinterpret_cast<const char*>(P + (size_t)v * p_elems), p_elems * (int)sizeof(T), p_unit);
+            else if (v >= 0 && pl.stage_tips)
+                stage_bytes(d, reinterpret_cast<const char*>(tipT + (size_t)v * t_elems), t_elems * (int)sizeof(T), t_unit);
+        }
+    };
+    auto row_of = [&](int r) { return kEven ? h * R + r : min(h * R + r, S - 1); };
+    auto load_msg = [&](int v, T (&d)[R]) {
+        const T* src = msg + (size_t)(v - n_tips) * node_elems;
+#pragma unroll
+        for (int r = 0; r < R; ++r) d[r] = src[row_of(r)];
+    };
+    // x's rescale, as in prune_any_kernel
+    auto rescale = [&](T (&x)[R]) {
+        T mx = T(0);
+#pragma unroll
+        for (int r = 0; r < R; ++r) mx = fmax(mx, x[r]);
+        const unsigned high = __ballot_sync(0xffffffffu, mx >= scale_threshold<T>());
+        if (__any_sync(0xffffffffu, (high & site_mask) == 0u)) {
+            T top = mx;
+            for (int q = 0; q < G; ++q) top = fmax(top, __shfl_sync(0xffffffffu, mx, site_l * G + q));
+            if (top < scale_threshold<T>() && top > T(0)) {
+                int e;
+                T f1, f2;
+                pow2_factors(top, &e, &f1, &f2);
+#pragma unroll
+                for (int r = 0; r < R; ++r) x[r] = (x[r] * f1) * f2;
+            }
+        }
+    };
+    int slot_now = 0, slot_next = pl.slots == 3 ? 2 : 1;
+    if constexpr (!kRes) {
+        stage(n_int - 1, 0);
+        cp_async_commit();
+        if (pl.slots == 3) {
+            if (n_int > 1) stage(n_int - 2, 1);
+            cp_async_commit();
+        }
+    }
+    T ou[R], co[R];
+    bool carried = true;
+    {
+        // FP32: the root weights by the power of two that brings the largest
+        // into [0.5, 1) (it cancels), so that node_out's scaled products fit
+        T f = T(1);
+        if constexpr (!Sh::kFp64) {
+            float top = 0.0f;
+            for (int s = 0; s < S; ++s) top = fmaxf(top, fabsf((float)a.root_w[s]));
+            if (top > 0.0f && top <= 3.0e38f) f = ldexpf(1.0f, -max(-126, min(126, ilogbf(top) + 1)));
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) co[r] = (T)a.root_w[row_of(r)] * f;
+    }
+    T pl_[R], pr_[R];  // the messages of the next node's internal children
+    if constexpr (kPre) {
+        const int4 kd = s_kids[n_int - 1];
+        if (kd.x >= n_tips) load_msg(kd.x, pl_);
+        if (kd.y >= n_tips) load_msg(kd.y, pr_);
+    }
+    for (int rk = n_int - 1; rk >= 0; --rk) {
+        const int4 kd = s_kids[rk];
+        if constexpr (!kRes) {
+            if (pl.slots == 3) cp_async_wait<1>();
+            else cp_async_wait<0>();
+            __syncthreads();
+            if (rk - (pl.slots - 1) >= 0) stage(rk - (pl.slots - 1), slot_next);
+            cp_async_commit();
+        }
+        const T *b0, *b1;
+        if constexpr (kRes) {
+            b0 = tables + (kd.x < n_tips ? tips_at + max(kd.x, 0) * t_elems : kd.x * p_elems);
+            b1 = tables + (kd.y < n_tips ? tips_at + max(kd.y, 0) * t_elems : kd.y * p_elems);
+        } else {
+            b0 = tables + slot_now * 2 * pl.child_elems;
+            b1 = b0 + pl.child_elems;
+            slot_now = slot_now + 1 == pl.slots ? 0 : slot_now + 1;
+            slot_next = slot_next + 1 == pl.slots ? 0 : slot_next + 1;
+        }
+        if (carried) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) ou[r] = co[r];
+        } else {
+            load_msg(kd.z, ou);
+        }
+        carried = false;
+        // ---- the children's messages
+        T dl[R], dr[R];
+        auto child = [&](int v, const T* b, const T (&pre)[R], T (&d)[R]) {
+            if (v >= n_tips) {
+                if constexpr (kPre) {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) d[r] = pre[r];
+                } else {
+                    load_msg(v, d);
+                }
+            } else if (v >= 0) {
+                const int row = (k * a.n_codes + s_codes[v * tile + col]) * S;
+                if (kRes || pl.stage_tips) {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) d[r] = b[row + row_of(r)];
+                } else {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) d[r] = __ldg(tipT + (size_t)v * t_elems + row + row_of(r));
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r) d[r] = T(1);
+            }
+        };
+        child(kd.x, b0, pl_, dl);
+        child(kd.y, b1, pr_, dr);
+        const int next_id = rk > 0 ? s_kids[rk - 1].z : -1;
+        if constexpr (kPre) {
+            if (rk > 0) {
+                const int4 kn = s_kids[rk - 1];
+                if (kn.x >= n_tips) load_msg(kn.x, pl_);
+                if (kn.y >= n_tips) load_msg(kn.y, pr_);
+            }
+        }
+        // ---- this node's output
+        {
+            T c[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) c[r] = dl[r] * dr[r];
+            rescale(c);
+            if (lane < W * G)
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    if (kEven || h * R + r < S) node.put(site_l * C + k, h * R + r, ou[r], c[r]);
+            node.write(C, W, blockIdx.x * tile + warp * W, a.n_sites, a.out + (size_t)rk * a.n_sites * S);
+        }
+        // ---- the internal children's outside vectors
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {
+            const int v = c ? kd.y : kd.x;
+            if (v < n_tips) continue;
+            T t[R], ov[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) t[r] = ou[r] * (c ? dl[r] : dr[r]);
+            const T* Pk = (c ? b1 : b0) + k * S * S;
+            if constexpr (Sh::kRegX) {
+#pragma unroll
+                for (int b = 0; b < R; ++b) {
+                    T acc = T(0);
+#pragma unroll
+                    for (int i = 0; i < S; ++i) acc = fma(t[i], Pk[i * S + b], acc);
+                    ov[b] = acc;
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    if (kEven || h * R + r < S) my_row[h * R + r] = t[r];
+                __syncwarp();
+#pragma unroll
+                for (int r = 0; r < R; ++r) ov[r] = T(0);
+#pragma unroll 4
+                for (int i = 0; i < S; ++i) {
+                    const T x = my_row[i];
+#pragma unroll
+                    for (int r = 0; r < R; ++r) ov[r] = fma(x, Pk[i * S + row_of(r)], ov[r]);
+                }
+                __syncwarp();  // the exchange row is read before it is written again
+            }
+            rescale(ov);
+            if (v == next_id) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) co[r] = ov[r];
+                carried = true;
+            } else if (valid) {
+                T* dst = msg + (size_t)(v - n_tips) * node_elems + h * R;
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    if (kEven || h * R + r < S) dst[r] = ov[r];
+            }
+        }
+    }
+    cp_async_wait<0>();
+}
+
+template <typename T, int S, int H, bool kRes, bool kNodes>
 cudaError_t launch_any_t(const PruneArgs& a, const AnyLaunch& p, int blocks, cudaStream_t st) {
-    auto kern = prune_any_kernel<T, S, H, kRes>;
+    auto kern = prune_any_kernel<T, S, H, kRes, kNodes>;
     const size_t smem = any_smem(S, H, std::is_same<T, double>::value, p, a);
     if (smem > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -397,30 +805,62 @@ template <typename T, int S, int H>
 cudaError_t launch_any_h(const PruneArgs& a, const AnyLaunch& p, int blocks, cudaStream_t st) {
     // the tables of more than 8 states fit whole in shared memory only for a
     // handful of nodes: the ring alone there
+    const bool nodes = p.msg || p.nodes;
     if constexpr (S <= 8) {
-        if (p.slots == 0) return launch_any_t<T, S, H, true>(a, p, blocks, st);
+        if (p.slots == 0)
+            return nodes ? launch_any_t<T, S, H, true, true>(a, p, blocks, st)
+                         : launch_any_t<T, S, H, true, false>(a, p, blocks, st);
     }
-    return launch_any_t<T, S, H, false>(a, p, blocks, st);
+    return nodes ? launch_any_t<T, S, H, false, true>(a, p, blocks, st)
+                 : launch_any_t<T, S, H, false, false>(a, p, blocks, st);
 }
 
-// H is 1, 2 or 4 up to 8 states, 2 or 4 above (any_plan chooses no other)
-template <typename T, int S>
-cudaError_t launch_any_s(const PruneArgs& a, int H, const AnyLaunch& p, int blocks, cudaStream_t st) {
+template <typename T, int S, int H, bool kRes>
+cudaError_t launch_down_any_t(const PreorderArgs& a, const AnyLaunch& p, int blocks, cudaStream_t st) {
+    auto kern = down_any_kernel<T, S, H, kRes>;
+    const size_t smem = any_down_smem(S, H, std::is_same<T, double>::value, p, a);
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    kern<<<blocks, p.warps * 32, smem, st>>>(a, p);
+    return cudaGetLastError();
+}
+template <typename T, int S, int H>
+cudaError_t launch_any_h(const PreorderArgs& a, const AnyLaunch& p, int blocks, cudaStream_t st) {
+    if constexpr (S <= 8) {
+        if (p.slots == 0) return launch_down_any_t<T, S, H, true>(a, p, blocks, st);
+    }
+    return launch_down_any_t<T, S, H, false>(a, p, blocks, st);
+}
+
+// H is 1, 2 or 4 up to 8 states, 2 or 4 above (any_plan chooses no other);
+// Args: PruneArgs (post-order) or PreorderArgs
+template <typename T, int S, class Args>
+cudaError_t launch_any_s(const Args& a, int H, const AnyLaunch& p, int blocks, cudaStream_t st) {
     if constexpr (S <= 8) {
         if (H == 1) return launch_any_h<T, S, 1>(a, p, blocks, st);
     }
     if (H == 2) return launch_any_h<T, S, 2>(a, p, blocks, st);
-    if (H == 4) return launch_any_h<T, S, 4>(a, p, blocks, st);
+    if constexpr (S >= 4) {
+        if (H == 4) return launch_any_h<T, S, 4>(a, p, blocks, st);
+    }
     return cudaErrorInvalidConfiguration;
 }
 
 }  // namespace dev
 
 // the state counts of each translation unit (S = 2..12 and 13..24)
-cudaError_t launch_any32_lo(const PruneArgs& a, int S, int H, const dev::AnyLaunch& p, int blocks, cudaStream_t st);
-cudaError_t launch_any32_hi(const PruneArgs& a, int S, int H, const dev::AnyLaunch& p, int blocks, cudaStream_t st);
-cudaError_t launch_any64_lo(const PruneArgs& a, int S, int H, const dev::AnyLaunch& p, int blocks, cudaStream_t st);
-cudaError_t launch_any64_hi(const PruneArgs& a, int S, int H, const dev::AnyLaunch& p, int blocks, cudaStream_t st);
+#define PLK_ANY_DECLARE(name, Args) \
+    cudaError_t name(const Args& a, int S, int H, const dev::AnyLaunch& p, int blocks, cudaStream_t st);
+PLK_ANY_DECLARE(launch_any32_lo, PruneArgs)
+PLK_ANY_DECLARE(launch_any32_hi, PruneArgs)
+PLK_ANY_DECLARE(launch_any64_lo, PruneArgs)
+PLK_ANY_DECLARE(launch_any64_hi, PruneArgs)
+PLK_ANY_DECLARE(launch_down32_lo, PreorderArgs)
+PLK_ANY_DECLARE(launch_down32_hi, PreorderArgs)
+PLK_ANY_DECLARE(launch_down64_lo, PreorderArgs)
+PLK_ANY_DECLARE(launch_down64_hi, PreorderArgs)
 
 #define PLK_ANY_CASE(T, S) \
     case S: return dev::launch_any_s<T, S>(a, H, p, blocks, st);
