@@ -190,9 +190,10 @@ plk_status plk_kernel_times(plk_handle* h, double* ms_out, int* n_evals, int res
  * prune4p_kernel with 1 / 2 sites per thread and each op's tip codes staged
  * with its tables two ops ahead (the fast forms when the codes exceed L2),
  * 12 / 13 / 14 = prune4w_kernel (every warp walks the op list alone over its
- * own 32 x 1 / 2 / 4 sites, tables through L1, spill stack in TMEM), 15 / 16
- * / 17 = the same with the tree's tables in shared memory, 18 = two threads
- * per site pair with the tables in shared memory.  20 states: 1 / 2 =
+ * own 32 x 1 / 2 / 4 sites, tables streamed through a shared-memory ring, 1 to
+ * 8 categories, spill stack in TMEM), 15 / 16 / 17 = the same with the tree's
+ * tables in shared memory, 18 = two threads per site pair with the tables in
+ * shared memory.  20 states: 1 / 2 =
  * prune20_kernel on CUDA cores / mma.sync tensor cores with 4 warps per tile,
  * 3 / 4 = the same with 8 warps, 5 = prune20u_kernel (tcgen05 tensor cores,
  * TMEM accumulators, spill stack in TMEM), 6 = prune20v_kernel (its compact
@@ -203,8 +204,8 @@ plk_status plk_kernel_times(plk_handle* h, double* ms_out, int* n_evals, int res
 int plk_prune_variant(const plk_handle* h);
 /* Test of the failure path: the next FP32 evaluation that runs one of the
  * mbarrier-driven post-order forms -- the TMA-fed 4-state form (candidate 9),
- * the shared-table warp-independent forms (15-18: their table copy), the
- * tcgen05 20-state forms (5-7: the first MMA commit) -- withholds the first
+ * the warp-independent forms (12-14: their ring's first stage, 15-18: their
+ * table copy), the tcgen05 20-state forms (5-7: the first MMA commit) -- withholds the first
  * stage of every tile or CTA, so every bounded mbarrier wait of that launch
  * runs out; with a streamed alignment the warp-independent forms (12-18) wait
  * for an arrival no copy writes.  The tiles' sites come out NaN, the

@@ -87,7 +87,10 @@ struct plk_handle {
     std::vector<int> left, right, post, rank;
     std::vector<double> bl;
     Program prog;
+    StreamProgram sprog;
     DevBuf d_tree_block;  // the tree's arrays, one upload (upload_group)
+    DevView d_sops, d_stages, d_where;
+    DevBuf d_stream;  // the streamed forms' tables
     DevView d_ops, d_order, d_left, d_right, d_rank;
     // rate model
     bool root_quirk = true;
@@ -108,6 +111,7 @@ struct plk_handle {
     DevBuf d_site_lnl, d_block, d_lnl, d_work, d_cond, d_outside, d_nodes_out;
     DevBuf d_done;  // arrival counters (finish_grid_sum, then one per 128-site tile), zero between launches
     bool paired_written = false;  // this evaluation's P(t) kernel also wrote prune4p's layouts
+    bool stream_written = false;  // or the streamed forms' tables
     bool withhold_stage = false;  // plk_test_withhold_stage: armed for the next FP32 pass
     DevBuf d_mask_raw, d_flag;
     bool have_lnl = false;
@@ -328,7 +332,10 @@ bool tuned_tc20(const plk_handle* h) {
     return v == 5 || v == 6 || v == 7;
 }
 
-plk_status build_pmats(plk_handle* h, bool paired = false, bool tc20 = false) {
+// bytes of the streamed forms' tables (stream_program)
+size_t stream_bytes(const plk_handle* h) { return (size_t)h->sprog.units * ((h->C + 1) / 2) * 128; }
+
+plk_status build_pmats(plk_handle* h, bool paired = false, bool tc20 = false, bool streamed = false) {
     plk_status s = refresh_teff(h);
     if (s != PLK_OK) return s;
     const size_t SS = (size_t)h->S * h->S;
@@ -355,6 +362,14 @@ plk_status build_pmats(plk_handle* h, bool paired = false, bool tc20 = false) {
         PLK_CUDA(h, h->d_work.ensure(prune4p_scratch_bytes(a)), "allocate scratch");
         prune4p_scratch_parts(h->d_work.p, h->n_nodes, h->C, &m.P32p, &m.tip32p);
     }
+    m.stream = nullptr;
+    m.where = nullptr;
+    if (streamed) {
+        PLK_CUDA(h, h->d_stream.ensure(stream_bytes(h)), "allocate streamed tables");
+        m.stream = h->d_stream.as<float>();
+        m.where = h->d_where.as<int>();
+    }
+    h->stream_written = streamed;
     m.B20 = nullptr;
     m.T20 = nullptr;
     m.ncs20 = 0;
@@ -399,6 +414,10 @@ PruneArgs prune_args(plk_handle* h, int precision) {
     a.n_int = (int)h->post.size();
     a.n_tips = h->n_tips;
     a.n_nodes = h->n_nodes;
+    a.sops = h->d_sops.as<Op>();
+    a.stages = h->d_stages.as<int2>();
+    a.where = h->d_where.as<int>();
+    a.n_stages = h->S == 4 ? (int)h->sprog.stages.size() : 0;
     return a;
 }
 
@@ -498,7 +517,14 @@ plk_status autotune_prune(plk_handle* h, PruneArgs a, const std::vector<int>& ca
 bool tuned_paired(const plk_handle* h) {
     if (h->S != 4 || (h->C != 2 && h->C != 4 && h->C != 8) || !fused_kernel_applies(h, PLK_FP32S)) return false;
     const int v = tuned_variant(h);
-    return v >= 3 && v <= 18;
+    return (v >= 3 && v <= 11) || (v >= 15 && v <= 18);
+}
+
+// the same for the streamed forms and their tables
+bool tuned_stream(const plk_handle* h) {
+    if (h->S != 4 || !fused_kernel_applies(h, PLK_FP32S)) return false;
+    const int v = tuned_variant(h);
+    return v >= 12 && v <= 14;
 }
 
 // Re-arms the arrival counters of the passes' in-kernel totals (zero between
@@ -590,10 +616,15 @@ plk_status run_prune(plk_handle* h, int precision, NodePass* store, cudaEvent_t*
     }
     if (fused && !store && precision == PLK_FP32S) {
         // the paired kernels read P(t) and tip tables re-laid out in scratch
-        const bool paired = prune4p_fits(a, 1) || prune4p_fits(a, 2) || prune4w_fits(a, 1);
+        const bool paired = prune4p_fits(a, 1) || prune4p_fits(a, 2) || prune4w_fits(a, 1, 1);
         if (paired) {
             PLK_CUDA(h, h->d_work.ensure(prune4p_scratch_bytes(a)), "allocate scratch");
             a.scratch = h->d_work.p;
+        }
+        if (prune4w_fits(a, 1, 2) && (h->variant < 0 || (h->variant >= 12 && h->variant <= 14))) {
+            PLK_CUDA(h, h->d_stream.ensure(stream_bytes(h)), "allocate streamed tables");
+            a.stream = h->d_stream.as<float>();
+            a.stream_ready = h->stream_written ? 1 : 0;
         }
         if (h->variant < 0) {
             std::vector<int> cands = {0};
@@ -608,8 +639,8 @@ plk_status run_prune(plk_handle* h, int precision, NodePass* store, cudaEvent_t*
             if (prune4p_fits(a, 1, 0)) cands.push_back(9);  // TMA-fed stage ring
             for (int v = 10; v <= 11; ++v)  // codes staged with each op
                 if (prune4p_fits(a, v - 9)) cands.push_back(v);
-            for (int v = 12; v <= 18; ++v)  // warp-independent: 1/2/4 sites per thread, tables via L1 or smem
-                if (prune4w_fits(a, (v == 12 || v == 15) ? 1 : ((v == 14 || v == 17) ? 4 : 2), v >= 15 ? 1 : 0,
+            for (int v = 12; v <= 18; ++v)  // warp-independent: 1/2/4 sites per thread, tables streamed or in smem
+                if (prune4w_fits(a, (v == 12 || v == 15) ? 1 : ((v == 14 || v == 17) ? 4 : 2), v >= 15 ? 1 : 2,
                                  v == 18 ? 2 : 1))
                     cands.push_back(v);
             plk_status s = autotune_prune(h, a, cands);
@@ -938,10 +969,12 @@ plk_status plk_set_tree(plk_handle* h, int n_nodes, const int* left, const int* 
     h->n_nodes = n_nodes;
     h->tree_tips = n_leaves;
     h->prog = build_program(n_leaves, n_nodes, left, right, root, rank);
+    h->sprog = stream_program(h->prog, n_nodes);
     PLK_CUDA(h,
              upload_group(h, h->d_tree_block,
                           {part(h->d_ops, h->prog.ops), part(h->d_order, post), part(h->d_left, h->left),
-                           part(h->d_right, h->right), part(h->d_rank, rank)}),
+                           part(h->d_right, h->right), part(h->d_rank, rank), part(h->d_sops, h->sprog.ops),
+                           part(h->d_stages, h->sprog.stages), part(h->d_where, h->sprog.where)}),
              "upload tree");
     // default rate model: the reference's empty rate_model
     h->root_quirk = true;
@@ -1035,8 +1068,8 @@ plk_status plk_loglik_async(plk_handle* h, int precision) {
         ev = &h->evs[h->ev_used++];
         PLK_CUDA(h, cudaEventRecord(ev->e[0], h->stream), "cudaEventRecord");
     }
-    if ((s = build_pmats(h, precision == PLK_FP32S && tuned_paired(h), precision == PLK_FP32S && tuned_tc20(h))) !=
-        PLK_OK)
+    if ((s = build_pmats(h, precision == PLK_FP32S && tuned_paired(h), precision == PLK_FP32S && tuned_tc20(h),
+                         precision == PLK_FP32S && tuned_stream(h))) != PLK_OK)
         return s;
     if (ev) PLK_CUDA(h, cudaEventRecord(ev->e[1], h->stream), "cudaEventRecord");
     if ((s = run_prune(h, precision, nullptr, ev ? &ev->e[2] : nullptr)) != PLK_OK) return s;

@@ -435,4 +435,30 @@ Program build_program(int n_tips, int n_nodes, const int* left, const int* right
     return prog;
 }
 
+StreamProgram stream_program(const Program& prog, int n_nodes) {
+    StreamProgram sp;
+    sp.where.assign(n_nodes, -1);
+    sp.ops = prog.ops;
+    int start = 0;
+    for (size_t o = 0; o < sp.ops.size(); ++o) {
+        Op& op = sp.ops[o];
+        const int c0 = op.s0 >= 0 ? 4 : 1, c1 = op.s1 == kSrcNone ? 0 : (op.s1 >= 0 ? 4 : 1);
+        op.pad = o == 0 || sp.units - start + c0 + c1 > kStageUnits;
+        if (op.pad) {
+            if (o > 0) sp.stages.emplace_back(start, sp.units - start);
+            start = sp.units;
+        }
+        sp.where[op.e0] = sp.units;
+        op.e0 = sp.units - start;
+        sp.units += c0;
+        if (c1 > 0) {
+            sp.where[op.e1] = sp.units;
+            op.e1 = sp.units - start;
+            sp.units += c1;
+        }
+    }
+    if (!sp.ops.empty()) sp.stages.emplace_back(start, sp.units - start);
+    return sp;
+}
+
 }  // namespace plk

@@ -42,6 +42,22 @@ struct Program {
     int max_depth = 0;
 };
 
+// The program as the streamed 4-state forms read it: every op's child tables
+// lie one after another in op order, in units of one P(t) block (an internal
+// child takes one, a tip child's table of 16 codes four), cut into stages of
+// whole ops of at most kStageUnits units.  In `ops`, e0 / e1 are unit offsets
+// into the op's stage and pad is 1 for the first op of a stage; stages holds
+// (first unit, units), where[v] the first unit of node v's tables (-1: the
+// root, which has none).
+constexpr int kStageUnits = 32;
+struct StreamProgram {
+    std::vector<Op> ops;
+    std::vector<std::pair<int, int>> stages;
+    std::vector<int> where;
+    int units = 0;
+};
+StreamProgram stream_program(const Program& prog, int n_nodes);
+
 // Records msg as the handle-less error (plk_last_error(NULL)) and returns s.
 plk_status report_error(plk_status s, const std::string& msg);
 
@@ -173,6 +189,10 @@ struct DeviceModel {
     // reads (plk_prune4p.cuh), so that no relayout launch is needed
     float* P32p;
     float* tip32p;
+    // when set (4 states): the streamed forms' tables (stream_program), blocks
+    // of KP = ceil(C / 2) pairs, an odd last category paired with itself
+    float* stream;
+    const int* where;
     // when set (20 states, the tcgen05 forms tuned): also their B-operand
     // images and [state][code] tip tables (plk_prune20u.cu), ncs20 codes per
     // row (n_codes rounded up to 4)
@@ -226,8 +246,9 @@ struct PruneArgs {
     // staged in shared memory), 9 = prune4p_bulk_kernel (TMA-fed stage ring),
     // 10/11 = prune4p_kernel with 1/2 sites per thread and each op's tip
     // codes staged with its tables, 12/13/14 = prune4w_kernel (warp-
-    // independent, nothing staged) with 1/2/4 sites per thread, 15/16/17 =
-    // the same with 1/2/4 sites per thread and the tables in shared memory,
+    // independent, the tables streamed through a shared-memory ring) with
+    // 1/2/4 sites per thread, 15/16/17 = the same with the tree's tables in
+    // shared memory,
     // 18 = two sites per thread pair, each thread half of the pairs.
     // 20 states: 0 = prune_generic_kernel, 1 / 2 = prune20_kernel on CUDA
     // cores / mma.sync tensor cores (TF32, three-product split) with 4 warps
@@ -259,8 +280,16 @@ struct PruneArgs {
     int paired_ready;
     // test of the failure path (plk_test_withhold_stage): the TMA-fed form
     // never stages its first op, the shared-table form never copies its
-    // tables, so their bounded waits run out
+    // tables, the streamed form no stage, so their bounded waits run out
     int withhold_first_stage;
+    // the streamed forms (stream_program): the tables, and whether the P(t)
+    // kernel has written them
+    const Op* sops;
+    const int2* stages;
+    const int* where;
+    int n_stages;
+    float* stream;
+    int stream_ready;
     // streamed tip codes (plk_set_alignment8, 4 states): the codes of sites
     // [c chunk_sites, (c + 1) chunk_sites) have landed once arrive[c] holds
     // arrive_gen.  The warp-independent forms wait for their tile's chunk
@@ -309,12 +338,15 @@ cudaError_t launch_prune4p(const PruneArgs& a, int spt, int codes, int tps, int*
 // copies (when the P(t) kernel did not write them itself).
 cudaError_t launch_relayout4p(const PruneArgs& a, float* Pp, float* Tp, cudaStream_t st);
 // Warp-independent 4-state FP32 kernel (plk_prune4w.cu): every warp walks the
-// op list over its own 32 x spt sites (spt = 1, 2, 4 sites per thread),
-// reading the paired layouts of prune4p's scratch through L1, spills in
-// tensor memory; C = 2, 4 or 8.
-// ts = 1: the tree's tables copied into shared memory first (when they fit).
+// op list over its own 32 x spt sites (spt = 1, 2, 4 sites per thread), spills
+// in tensor memory.
+// ts = 1: the tree's paired tables (prune4p's scratch) copied into shared
+// memory first (C = 2, 4 or 8, when they fit).
+// ts = 2: the tables streamed through a ring (any tree, C = 1..8).
 // tps = 2: two threads per site, each with half of the category pairs.
-bool prune4w_fits(const PruneArgs& a, int spt, int ts = 0, int tps = 1);
+bool prune4w_fits(const PruneArgs& a, int spt, int ts, int tps = 1);
+// the streamed tables written from the P(t) kernel's FP32 copies
+cudaError_t launch_relayout_stream(const PruneArgs& a, cudaStream_t st);
 cudaError_t launch_prune4w(const PruneArgs& a, int spt, int ts, int tps, int* n_blocks, cudaStream_t st);
 // Staged 4-state FP32 kernel (plk_prune4s.cu): spt sites per thread.
 bool prune4s_fits(const PruneArgs& a, int spt);

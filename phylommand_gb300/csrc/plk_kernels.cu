@@ -39,6 +39,16 @@ __device__ __forceinline__ float tf32_rna_dev(float x) {
     return __uint_as_float(r);
 }
 
+// an entry of node v's tables in the streamed layout; the last of an odd
+// number of categories also in its missing partner's place (the next float)
+__device__ __forceinline__ void stream_store(const DeviceModel& m, int v, int k, int at, float x) {
+    const int w = m.where[v];
+    if (w < 0) return;  // the root
+    float* d = m.stream + (size_t)w * ((m.C + 1) / 2) * 32 + at;
+    d[0] = x;
+    if (k == m.C - 1 && (m.C & 1)) d[1] = x;
+}
+
 __global__ void pmat_kernel(DeviceModel m, int p_kind) {
     // a pass launched after it with programmatic stream serialization may be
     // scheduled now (it waits for this kernel's completion before reading)
@@ -152,6 +162,7 @@ __global__ void pmat_kernel(DeviceModel m, int p_kind) {
         m.P64[base + idx] = A[idx];
         m.P32[base + idx] = (float)A[idx];
         if (m.P32p) m.P32p[(size_t)v * m.C * 16 + paired_p_index(k, idx / 4, idx % 4)] = (float)A[idx];
+        if (m.stream && v >= m.n_tips) stream_store(m, v, k, paired_p_index(k, idx / 4, idx % 4), (float)A[idx]);
     }
     if (m.B20 && S == 20 && m.b20_bf16) {
         // the split-BF16 image (bf16_image_index), in the first 4 KB of the slot
@@ -201,6 +212,7 @@ __global__ void pmat_kernel(DeviceModel m, int p_kind) {
             m.tip64[tb + idx] = acc;
             m.tip32[tb + idx] = (float)acc;
             if (m.tip32p) m.tip32p[(size_t)v * m.C * kCodes * 4 + paired_tip_index(k, c, i)] = (float)acc;
+            if (m.stream) stream_store(m, v, k, paired_tip_index(k, c, i), (float)acc);
             if (m.T20) m.T20[((size_t)v * m.C + k) * (20 * m.ncs20) + (size_t)i * m.ncs20 + c] = (float)acc;
         }
         if (m.T20) {  // the padding codes of every state row
@@ -255,6 +267,7 @@ __global__ void __launch_bounds__(128) pmat4_eigen_kernel(DeviceModel m) {
         m.P64[base + j] = p[j];
         m.P32[base + j] = (float)p[j];
         if (m.P32p) m.P32p[(size_t)v * m.C * 16 + paired_p_index(k, r, j)] = (float)p[j];
+        if (m.stream && v >= m.n_tips) stream_store(m, v, k, paired_p_index(k, r, j), (float)p[j]);
     }
     if (v < m.n_tips && m.code_mask == nullptr && m.n_codes == kCodes) {
         // the 16 state sets themselves as codes: every mask known at compile
@@ -273,6 +286,7 @@ __global__ void __launch_bounds__(128) pmat4_eigen_kernel(DeviceModel m) {
             m.tip64[tb + (size_t)c * 4 + r] = acc;
             m.tip32[tb + (size_t)c * 4 + r] = (float)acc;
             if (m.tip32p) m.tip32p[(size_t)v * m.C * kCodes * 4 + paired_tip_index(k, c, r)] = (float)acc;
+            if (m.stream) stream_store(m, v, k, paired_tip_index(k, c, r), (float)acc);
         }
     } else if (v < m.n_tips) {
         const size_t tb = (size_t)it * m.n_codes * 4;
@@ -289,6 +303,7 @@ __global__ void __launch_bounds__(128) pmat4_eigen_kernel(DeviceModel m) {
             m.tip64[tb + (size_t)c * 4 + r] = acc;
             m.tip32[tb + (size_t)c * 4 + r] = (float)acc;
             if (m.tip32p) m.tip32p[(size_t)v * m.C * kCodes * 4 + paired_tip_index(k, c, r)] = (float)acc;
+            if (m.stream) stream_store(m, v, k, paired_tip_index(k, c, r), (float)acc);
         }
     }
 }
@@ -663,7 +678,7 @@ cudaError_t launch_prune(const PruneArgs& a, int S, int precision, bool store, i
         return launch_prune4p(a, a.variant - 9, 2, 1, n_blocks, st);
     if (!fp64 && !store && S == 4 && a.variant >= 12 && a.variant <= 18) {
         const int spt = (a.variant == 12 || a.variant == 15) ? 1 : ((a.variant == 14 || a.variant == 17) ? 4 : 2);
-        const int ts = a.variant >= 15 ? 1 : 0, tps = a.variant == 18 ? 2 : 1;
+        const int ts = a.variant >= 15 ? 1 : 2, tps = a.variant == 18 ? 2 : 1;
         if (prune4w_fits(a, spt, ts, tps)) return launch_prune4w(a, spt, ts, tps, n_blocks, st);
     }
     if (!fp64 && !store && S == 20 && a.variant >= 5 && a.variant <= 7 && prune20u_fits(a, a.variant - 5))

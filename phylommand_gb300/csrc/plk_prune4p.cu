@@ -15,6 +15,8 @@
 //
 // relayout4p_kernel writes the paired P(t) and tip layouts from the FP32
 // copies of the P(t) kernel.
+#include <algorithm>
+
 #include "plk_prune4p.cuh"
 
 namespace plk {
@@ -39,6 +41,29 @@ __global__ void relayout4p_kernel(const float* __restrict__ P, const float* __re
             const long long tp = t / (C * kCodes * 4);
             const int w = (int)(t % (C * kCodes * 4));
             Tp[tp * C * kCodes * 4 + paired_tip_index(w / (kCodes * 4), (w / 4) % kCodes, w % 4)] = tip[t];
+        }
+    }
+}
+
+// the streamed forms' tables from the P(t) kernel's FP32 copies: an odd last
+// category also in the place of its missing partner
+__global__ void relayout_stream_kernel(const float* __restrict__ P, const float* __restrict__ tip, int n_nodes,
+                                       int n_tips, int C, const int* __restrict__ where, float* __restrict__ stream) {
+    const int KP = (C + 1) / 2;
+    const long long n_p = (long long)(n_nodes - n_tips) * 2 * KP * 16, n_t = (long long)n_tips * 2 * KP * kCodes * 4;
+    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < n_p + n_t;
+         idx += (long long)gridDim.x * blockDim.x) {
+        if (idx < n_p) {
+            const int node = n_tips + (int)(idx / (2 * KP * 16)), w = (int)(idx % (2 * KP * 16)), k = w / 16;
+            if (where[node] < 0) continue;  // the root
+            stream[(size_t)where[node] * KP * 32 + paired_p_index(k, (w / 4) % 4, w % 4)] =
+                P[((size_t)node * C + min(k, C - 1)) * 16 + w % 16];
+        } else {
+            const long long t = idx - n_p;
+            const int tp = (int)(t / (2 * KP * kCodes * 4)), w = (int)(t % (2 * KP * kCodes * 4)), k = w / (kCodes * 4);
+            if (where[tp] < 0) continue;
+            stream[(size_t)where[tp] * KP * 32 + paired_tip_index(k, (w / 4) % kCodes, w % 4)] =
+                tip[((size_t)tp * C + min(k, C - 1)) * kCodes * 4 + w % (kCodes * 4)];
         }
     }
 }
@@ -189,6 +214,16 @@ cudaError_t launch_relayout4p(const PruneArgs& a, float* Pp, float* Tp, cudaStre
     relayout4p_kernel<<<(unsigned)blocks, 256, 0, st>>>(static_cast<const float*>(a.P),
                                                          static_cast<const float*>(a.tipT), a.n_nodes, a.n_tips, a.C,
                                                          Pp, Tp);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_relayout_stream(const PruneArgs& a, cudaStream_t st) {
+    const int KP = (a.C + 1) / 2;
+    const long long total = (long long)(a.n_nodes - a.n_tips) * KP * 32 + (long long)a.n_tips * KP * kCodes * 8;
+    const long long blocks = std::min<long long>((total + 255) / 256, 152 * 8);
+    relayout_stream_kernel<<<(unsigned)blocks, 256, 0, st>>>(static_cast<const float*>(a.P),
+                                                             static_cast<const float*>(a.tipT), a.n_nodes, a.n_tips,
+                                                             a.C, a.where, a.stream);
     return cudaGetLastError();
 }
 

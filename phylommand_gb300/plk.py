@@ -415,9 +415,9 @@ class Handle:
             9: "prune4p_bulk_kernel (category pairs on FP32x2, TMA bulk-copy stage ring, mbarrier pipeline)",
             10: "prune4p_kernel (category pairs on FP32x2, 1 site/thread, tip codes staged with each op)",
             11: "prune4p_kernel (category pairs on FP32x2, 2 sites/thread, tip codes staged with each op)",
-            12: "prune4w_kernel (category pairs on FP32x2, warp-independent, 1 site/thread, spills in TMEM)",
-            13: "prune4w_kernel (category pairs on FP32x2, warp-independent, 2 sites/thread, spills in TMEM)",
-            14: "prune4w_kernel (category pairs on FP32x2, warp-independent, 4 sites/thread, spills in TMEM)",
+            12: "prune4w_kernel (category pairs on FP32x2, warp-independent, 1 site/thread, streamed tables)",
+            13: "prune4w_kernel (category pairs on FP32x2, warp-independent, 2 sites/thread, streamed tables)",
+            14: "prune4w_kernel (category pairs on FP32x2, warp-independent, 4 sites/thread, streamed tables)",
             15: "prune4w_kernel (category pairs on FP32x2, warp-independent, 1 site/thread, tables in shared memory)",
             16: "prune4w_kernel (category pairs on FP32x2, warp-independent, 2 sites/thread, tables in shared memory)",
             17: "prune4w_kernel (category pairs on FP32x2, warp-independent, 4 sites/thread, tables in shared memory)",
