@@ -697,23 +697,28 @@ template <class PointFn>
 plk_status set_gtr_models(plk_batch* b, const double* freqs, PointFn point, std::vector<char>& in_domain) {
     const int n_items = (int)b->items.size();
     const int C = b->C;
-    const int n_threads = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+    // A model takes about 4 us and starting a thread about 18, one after another,
+    // so n threads beside this one make n x 18 + items x 4 / (n + 1) us, least at
+    // n + 1 = sqrt(items / 4.5).  48 items: two, 100 us, where always sixteen
+    // took 600.
+    const int n_threads = std::max(1, std::min({(int)std::sqrt(n_items / 4.5), 16, (int)std::thread::hardware_concurrency()}));
     std::vector<plk_status> st(n_threads, PLK_OK);
     std::vector<std::thread> pool;
-    for (int t = 0; t < n_threads; ++t)
-        pool.emplace_back([&, t]() {
-            std::vector<double> Q(16), cr(C), cw(C);
-            for (int i = t; i < n_items; i += n_threads) {
-                const double* x = point(i);
-                if (!x) continue;
-                double scale = 1.0;
-                in_domain[i] = gtr_model_from_x(4, x, C, freqs + (size_t)i * 4, Q.data(), cr.data(), cw.data(), &scale);
-                if (!in_domain[i]) continue;
-                for (int k = 0; k < C; ++k) cr[k] *= scale;
-                const plk_status s = plk_batch_set_model(b, i, Q.data(), freqs + (size_t)i * 4, cr.data(), cw.data());
-                if (s != PLK_OK) st[t] = s;
-            }
-        });
+    auto run = [&](int t) {
+        std::vector<double> Q(16), cr(C), cw(C);
+        for (int i = t; i < n_items; i += n_threads) {
+            const double* x = point(i);
+            if (!x) continue;
+            double scale = 1.0;
+            in_domain[i] = gtr_model_from_x(4, x, C, freqs + (size_t)i * 4, Q.data(), cr.data(), cw.data(), &scale);
+            if (!in_domain[i]) continue;
+            for (int k = 0; k < C; ++k) cr[k] *= scale;
+            const plk_status s = plk_batch_set_model(b, i, Q.data(), freqs + (size_t)i * 4, cr.data(), cw.data());
+            if (s != PLK_OK) st[t] = s;
+        }
+    };
+    for (int t = 1; t < n_threads; ++t) pool.emplace_back(run, t);
+    run(0);
     for (auto& th : pool) th.join();
     for (plk_status s : st)
         if (s != PLK_OK) return s;
