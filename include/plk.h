@@ -69,7 +69,7 @@ typedef int plk_status;
 #define PLK_P_TAYLOR20 0 /* the reference's (I + Q t / 2^20)^(2^20),
                             src/marth/marth.cpp:129-140, same operation order */
 #define PLK_P_EXACT 1    /* exp(Q t): eigendecomposition for a reversible Q
-                            (FP64 Jacobi on the host, FP64 P on the device),
+                            (FP64 eigen system on the host, FP64 P on the device),
                             scaling and squaring for a non-reversible Q */
 
 /* node-state outputs */
@@ -285,9 +285,10 @@ plk_status plk_batch_device_ms(const plk_batch* b, double* loglik_ms, double* nn
 plk_status plk_batch_tuning(const plk_batch* b, int* sites_per_thread, int* grid, double* ms,
                             int* uses_graph);
 /* The autotuned form of the post-order kernel: paired = 1 when categories
- * go in pairs on the packed FP32x2 pipe (2, 4 or 8 categories; same per-site
- * bits as one at a time), codes_smem = 1 when each tile's tip codes are
- * staged in shared memory rather than read from global memory. */
+ * go in pairs on the packed FP32x2 pipe (2, 4 or 8 categories, or any count in
+ * the form with streamed tables; same per-site bits as one at a time),
+ * codes_smem = 1 when each tile's tip codes are staged in shared memory (whole,
+ * or as the ops need them) rather than read from global memory. */
 plk_status plk_batch_form(const plk_batch* b, int* paired, int* codes_smem);
 
 /* NNI neighbours of every item: the trees one nearest-neighbour interchange

@@ -10,6 +10,8 @@
 //                      it; one compensated partial sum per unit.
 //  batch_prune4p_kernel the same over the paired-category tile body of
 //                      plk_prune4p.cuh (C = 2, 4, 8; same per-site bits).
+//  batch_prune4w_kernel the warps of a unit walk its op list alone, tables
+//                      streamed (plk_batch4w.cu).
 //  batch_reduce_kernel one warp per item sums its units in a fixed order
 //                      (TwoSum), so results do not depend on scheduling.
 #include "plk_batch.h"
@@ -47,6 +49,10 @@ __global__ void batch_pmat_kernel(BatchDev b) {
             for (int m = 0; m < 4; ++m) acc = fma(L[i * 4 + m] * ex[m], R[m * 4 + j], acc);
             P[i * 4 + j] = acc;
         }
+    const int v = nm.y, last = (k == C - 1 && (C & 1)) ? 2 : 1;  // an odd last category also in its partner's place
+    const bool tip = v < it.n_tips;
+    const int w = b.stream ? b.where[g] : -1;
+    float* const sd = w >= 0 ? b.stream + (size_t)w * ((C + 1) / 2) * 32 : nullptr;
     if (b.write_std) {
         float* dst = b.P32 + ((size_t)g * C + k) * 16;
 #pragma unroll
@@ -59,20 +65,31 @@ __global__ void batch_pmat_kernel(BatchDev b) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) dst[paired_p_index(k, i, j)] = (float)P[i * 4 + j];
     }
-    const int v = nm.y;
-    if (v < it.n_tips) {
-        float* tt = b.write_std ? b.tip32 + (((size_t)(it.tip_off + v) * C + k) * kCodes) * 4 : nullptr;
-        float* tp = b.tip32p ? b.tip32p + (size_t)(it.tip_off + v) * C * kCodes * 4 : nullptr;
-        for (int code = 0; code < kCodes; ++code)
+    if (sd && !tip) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                double acc = 0.0;
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if ((code >> j) & 1) acc += P[i * 4 + j];
-                if (tt) tt[code * 4 + i] = (float)acc;
-                if (tp) tp[paired_tip_index(k, code, i)] = (float)acc;
-            }
+            for (int j = 0; j < 4; ++j)
+                for (int q = 0; q < last; ++q) sd[paired_p_index(k, i, j) + q] = (float)P[i * 4 + j];
+    }
+    if (!tip) return;
+    // a code's sum over its states, ascending: that of the code without its
+    // highest state plus one term
+    float* tt = b.write_std ? b.tip32 + (((size_t)(it.tip_off + v) * C + k) * kCodes) * 4 : nullptr;
+    float* tp = b.tip32p ? b.tip32p + (size_t)(it.tip_off + v) * C * kCodes * 4 : nullptr;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        double sum[kCodes];
+        sum[0] = 0.0;
+#pragma unroll
+        for (int code = 0; code < kCodes; ++code) {
+            const int top = code >= 8 ? 3 : (code >= 4 ? 2 : (code >= 2 ? 1 : 0));
+            if (code > 0) sum[code] = sum[code ^ (1 << top)] + P[i * 4 + top];
+            if (tt) tt[code * 4 + i] = (float)sum[code];
+            if (tp) tp[paired_tip_index(k, code, i)] = (float)sum[code];
+            if (sd)
+                for (int q = 0; q < last; ++q) sd[paired_tip_index(k, code, i) + q] = (float)sum[code];
+        }
     }
 }
 
@@ -197,7 +214,7 @@ BatchKernel form_kernel(int C, const BatchForm& f, int max_ops, int max_tips, in
 }  // namespace
 
 bool batch_form_valid(int C, const BatchForm& f) {
-    if (f.spt != 1 && f.spt != 2) return false;
+    if (f.stream || (f.spt != 1 && f.spt != 2)) return false;
     if (C < 1 || C > 8) return false;
     return !f.paired || C == 2 || C == 4 || C == 8;
 }

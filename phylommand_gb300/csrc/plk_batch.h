@@ -20,7 +20,8 @@ struct BatchItemDev {
     int model_off;        // doubles into model: lam[4] L[16] R[16] root_w[4] cat_rate[C] cat_w[C]
     int n_moves, move_out_off;  // NNI rearrangements of this tree, into the NNI output
     int n_int;            // internal nodes (the root is n_tips + n_int - 1)
-    int pad[3];
+    int stage_off, n_stages;  // into stages (streamed tables)
+    int pad;
 };
 static_assert(sizeof(BatchItemDev) == 64, "BatchItemDev is 64 bytes");
 
@@ -38,6 +39,12 @@ struct BatchDev {
     float* tip32;             // [n_tips_total][C][16][4]
     float* P32p;              // paired layout of P32 (plk_prune4p.cuh), or null
     float* tip32p;            // paired layout of tip32, or null
+    // streamed tables (plk_batch4w.cu, stream_program): per item's ops in their
+    // order, its stages, every node's place, the tables; or null
+    const Op* sops;           // as ops
+    const int2* stages;       // (first unit, units) of every item's stages
+    const int* where;         // [n_nodes_total] first unit of a node's tables, -1 for a root
+    float* stream;            // [units][KP][32]
     int write_std, pad2;      // batch_pmat_kernel writes P32 / tip32 when non-zero
     const int2* units;        // [n_units] (item, tile index), largest trees first
     double* unit_sums;        // [n_units][2]
@@ -62,11 +69,13 @@ inline int batch_model_stride(int C) { return 40 + 2 * C; }
 
 // One form of the batch post-order kernel: sites per thread, tip codes staged
 // in shared memory or read from global, categories in pairs on the FP32x2
-// pipe (C = 2, 4, 8; reads P32p / tip32p) or one at a time.
+// pipe (C = 2, 4, 8; reads P32p / tip32p) or one at a time; or the streamed
+// form (in pairs, any C).
 struct BatchForm {
     int spt = 1;
     bool codes_smem = false;
     bool paired = false;
+    bool stream = false;
 };
 bool batch_form_valid(int C, const BatchForm& f);
 size_t batch_smem_bytes(int C, const BatchForm& f, int max_ops, int max_tips, int max_depth);
@@ -74,6 +83,16 @@ int batch_occupancy(int C, const BatchForm& f, size_t smem);
 cudaError_t launch_batch_pmat(const BatchDev& b, cudaStream_t st);
 cudaError_t launch_batch_prune(const BatchDev& b, const BatchForm& f, int grid, size_t smem, cudaStream_t st);
 cudaError_t launch_batch_reduce(const BatchDev& b, cudaStream_t st);
+
+// The streamed form (plk_batch4w.cu) with per_sm CTAs of four warps an SM: their
+// tensor-memory columns and stack entries in them, byte offsets in shared memory.
+struct BatchStreamShape {
+    int tmem_cols, levels;
+    int ops_at, codes_at, over_at, ops_in_smem;
+    size_t smem;  // 0: does not fit
+};
+BatchStreamShape batch_stream_shape(int C, int spt, int max_ops, int max_depth, int per_sm);
+cudaError_t launch_batch_prune4w(const BatchDev& b, const BatchStreamShape& sh, int spt, int grid, cudaStream_t st);
 
 // NNI scoring and branch-length derivatives (plk_nni.cu): work units of `warps`
 // warps of down_sites_per_warp sites; the tables of an item in shared memory

@@ -43,6 +43,11 @@ struct BBuf {
         if (e == cudaSuccess) bytes = n;
         return e;
     }
+    void release() {
+        if (p) cudaFree(p);
+        p = nullptr;
+        bytes = 0;
+    }
     template <typename T>
     T* as() const { return static_cast<T*>(p); }
 };
@@ -96,6 +101,7 @@ struct plk_batch {
     // device layout
     BBuf d_items, d_codes, d_ops, d_teff, d_node_item, d_child, d_model, d_P32, d_tip32, d_lnl, d_counter;
     BBuf d_P32p, d_tip32p;  // paired layouts (C = 2, 4, 8)
+    BBuf d_sops, d_stages, d_where, d_stream;  // streamed tables
     // NNI scoring and branch-length derivatives
     BBuf d_kids, d_Pn, d_tipn, d_records, d_nni_out, d_scr, d_scr_e;
     BBuf d_blen_out, d_blen_ex;
@@ -109,6 +115,7 @@ struct plk_batch {
     BatchForm form;
     int grid = 0;
     size_t smem = 0;
+    BatchStreamShape shape{};  // of the streamed form
     double tuned_ms = 0.0;
     bool tuned = false;
     // optimiser of plk_batch_fit_gtr
@@ -164,6 +171,10 @@ BatchDev device_view(plk_batch* b, const UnitSet& us) {
     d.tip32 = b->d_tip32.as<float>();
     d.P32p = nullptr;  // the plain layout only, unless lnl_view asks for the paired one
     d.tip32p = nullptr;
+    d.sops = nullptr;  // likewise
+    d.stages = nullptr;
+    d.where = nullptr;
+    d.stream = nullptr;
     d.write_std = 1;
     d.units = us.units.as<int2>();
     d.unit_sums = us.sums.as<double>();
@@ -179,11 +190,17 @@ BatchDev device_view(plk_batch* b, const UnitSet& us) {
 BatchDev lnl_view(plk_batch* b, const BatchForm* form) {
     BatchDev d = device_view(b, b->lnl_units);
     const bool has_paired = b->d_P32p.p != nullptr && (b->C == 2 || b->C == 4 || b->C == 8);
-    if (has_paired && (!form || form->paired)) {
+    if (b->d_stream.p != nullptr && (!form || form->stream)) {
+        d.sops = b->d_sops.as<Op>();
+        d.stages = b->d_stages.as<int2>();
+        d.where = b->d_where.as<int>();
+        d.stream = b->d_stream.as<float>();
+    }
+    if (has_paired && (!form || (form->paired && !form->stream))) {
         d.P32p = b->d_P32p.as<float>();
         d.tip32p = b->d_tip32p.as<float>();
     }
-    if (form && form->paired) d.write_std = 0;
+    if (form && (form->paired || form->stream)) d.write_std = 0;
     return d;
 }
 
@@ -230,6 +247,10 @@ plk_status build_layout(plk_batch* b) {
     std::vector<double> teff;
     std::vector<int2> node_item, child;
     std::vector<int4> kids;
+    std::vector<Op> sops;
+    std::vector<int2> stages;
+    std::vector<int> where;
+    size_t stream_units = 0;
     size_t codes_bytes = 0;
     int tips_total = 0, total_moves = 0;
     b->max_ops = b->max_tips = b->max_depth = b->max_int = 0;
@@ -249,6 +270,13 @@ plk_status build_layout(plk_batch* b) {
         d.n_moves = h.n_moves();
         d.move_out_off = total_moves;
         d.n_int = h.n_int;
+        const StreamProgram sp = stream_program(h.prog, h.n_nodes);
+        d.stage_off = (int)stages.size();
+        d.n_stages = (int)sp.stages.size();
+        sops.insert(sops.end(), sp.ops.begin(), sp.ops.end());
+        for (const auto& st : sp.stages) stages.push_back(make_int2((int)stream_units + st.first, st.second));
+        for (int w : sp.where) where.push_back(w < 0 ? -1 : (int)stream_units + w);
+        stream_units += sp.units;
         codes_bytes += h.codes.size();
         ops.insert(ops.end(), h.prog.ops.begin(), h.prog.ops.end());
         teff.insert(teff.end(), h.t_eff.begin(), h.t_eff.end());
@@ -281,6 +309,19 @@ plk_status build_layout(plk_batch* b) {
         PLK_BCUDA(b, b->d_P32p.ensure((size_t)b->n_nodes_total * C * 16 * sizeof(float)), "allocate P");
         PLK_BCUDA(b, b->d_tip32p.ensure((size_t)tips_total * C * 16 * 4 * sizeof(float)), "allocate tip tables");
     }
+    // the streamed form's buffers: without them (no memory, or more units than an
+    // int counts) the staged forms remain
+    const size_t stream_bytes = stream_units * ((C + 1) / 2) * 128;
+    bool stream_ok = C <= 8 && stream_units > 0 && stream_units < (1u << 30);
+    for (auto [buf, bytes] : {std::pair<BBuf*, size_t>{&b->d_sops, sops.size() * sizeof(Op)},
+                              {&b->d_stages, stages.size() * sizeof(int2)},
+                              {&b->d_where, where.size() * sizeof(int)},
+                              {&b->d_stream, stream_bytes}})
+        if (stream_ok && buf->ensure(bytes) != cudaSuccess) {
+            cudaGetLastError();
+            stream_ok = false;
+        }
+    if (!stream_ok) b->d_stream.release();
     PLK_BCUDA(b, b->d_lnl.ensure(it.size() * sizeof(double)), "allocate lnL");
     PLK_BCUDA(b, b->d_counter.ensure(sizeof(int)), "allocate counter");
     PLK_BCUDA(b, b->d_kids.ensure(kids.size() * sizeof(int4)), "allocate node table");
@@ -292,6 +333,13 @@ plk_status build_layout(plk_batch* b) {
         off += h.codes.size();
     }
     PLK_BCUDA(b, cudaMemcpy(b->d_ops.p, ops.data(), ops.size() * sizeof(Op), cudaMemcpyHostToDevice), "upload programs");
+    if (stream_ok) {
+        PLK_BCUDA(b, cudaMemcpy(b->d_sops.p, sops.data(), sops.size() * sizeof(Op), cudaMemcpyHostToDevice), "upload programs");
+        PLK_BCUDA(b, cudaMemcpy(b->d_stages.p, stages.data(), stages.size() * sizeof(int2), cudaMemcpyHostToDevice),
+                  "upload programs");
+        PLK_BCUDA(b, cudaMemcpy(b->d_where.p, where.data(), where.size() * sizeof(int), cudaMemcpyHostToDevice),
+                  "upload programs");
+    }
     PLK_BCUDA(b, cudaMemcpy(b->d_teff.p, teff.data(), teff.size() * sizeof(double), cudaMemcpyHostToDevice), "upload lengths");
     PLK_BCUDA(b, cudaMemcpy(b->d_node_item.p, node_item.data(), node_item.size() * sizeof(int2), cudaMemcpyHostToDevice),
               "upload node map");
@@ -324,6 +372,11 @@ plk_status build_layout(plk_batch* b) {
     return PLK_OK;
 }
 
+cudaError_t launch_form(plk_batch* b, const BatchDev& d, const BatchForm& f, int grid, size_t smem,
+                        const BatchStreamShape& shape) {
+    return f.stream ? launch_batch_prune4w(d, shape, f.spt, grid, b->stream) : launch_batch_prune(d, f, grid, smem, b->stream);
+}
+
 // The evaluation sequence (graph body).
 plk_status enqueue_eval(plk_batch* b) {
     const BatchDev d = lnl_view(b, &b->form);
@@ -332,7 +385,7 @@ plk_status enqueue_eval(plk_batch* b) {
     PLK_BCUDA(b, cudaMemcpyAsync(b->d_model.p, b->h_model, mn * sizeof(double), cudaMemcpyHostToDevice, b->stream),
               "upload models");
     PLK_BCUDA(b, launch_batch_pmat(d, b->stream), "batch P(t) launch");
-    PLK_BCUDA(b, launch_batch_prune(d, b->form, b->grid, b->smem, b->stream), "batch post-order launch");
+    PLK_BCUDA(b, launch_form(b, d, b->form, b->grid, b->smem, b->shape), "batch post-order launch");
     PLK_BCUDA(b, launch_batch_reduce(d, b->stream), "batch reduce launch");
     PLK_BCUDA(b, cudaMemcpyAsync(b->h_lnl, b->d_lnl.p, b->items.size() * sizeof(double), cudaMemcpyDeviceToHost,
                                  b->stream),
@@ -342,9 +395,11 @@ plk_status enqueue_eval(plk_batch* b) {
 
 // Autotuner over the kernel forms -- categories in pairs or one at a time,
 // sites per thread 1 or 2, tip codes staged in shared memory (where they fit)
-// or read from global -- times CTAs per SM 1 .. occupancy, two launches of
-// the persistent kernel after a warm-up each.  PLK_BATCH_SPT and
-// PLK_BATCH_PAIRED (0 / 1) pin those choices.
+// or read from global, the streamed form -- times CTAs per SM, two launches of
+// the persistent kernel after a warm-up each.  Fewer CTAs an SM than fit were
+// slower for every form of every batch measured (streamed, 48 items: 1 to 4 CTAs
+// 902, 532, 428, 392 us), so the count goes down only while that is faster.  PLK_BATCH_SPT
+// and PLK_BATCH_PAIRED (0 / 1, 2 = streamed) pin those choices.
 plk_status tune(plk_batch* b) {
     cudaEvent_t e0, e1;
     PLK_BCUDA(b, cudaEventCreate(&e0), "cudaEventCreate");
@@ -353,6 +408,7 @@ plk_status tune(plk_batch* b) {
     BatchForm best_form;
     int best_grid = 0;
     size_t best_smem = 0;
+    BatchStreamShape best_shape{};
     const char* force_spt = getenv("PLK_BATCH_SPT");
     const char* force_paired = getenv("PLK_BATCH_PAIRED");
     std::vector<BatchForm> forms;
@@ -371,23 +427,40 @@ plk_status tune(plk_batch* b) {
                 if (f.codes_smem && smem > 160 * 1024) continue;
                 forms.push_back(f);
             }
+    for (int spt = 1; spt <= 2 && b->d_stream.p != nullptr; ++spt) {
+        if (force_spt && atoi(force_spt) != spt) continue;
+        if (force_paired && atoi(force_paired) != 2) continue;
+        BatchForm f;
+        f.spt = spt;
+        f.codes_smem = f.paired = f.stream = true;
+        forms.push_back(f);
+    }
     for (const BatchForm& f : forms) {
-        const size_t smem = batch_smem_bytes(b->C, f, b->max_ops, b->max_tips, b->max_depth);
-        const int occ = batch_occupancy(b->C, f, smem);
+        const size_t smem = f.stream ? 0 : batch_smem_bytes(b->C, f, b->max_ops, b->max_tips, b->max_depth);
+        int occ = 0;
+        if (f.stream)
+            while (occ < 8 && batch_stream_shape(b->C, f.spt, b->max_ops, b->max_depth, occ + 1).smem > 0) ++occ;
+        else occ = batch_occupancy(b->C, f, smem);
         if (occ < 1) continue;
         if (b->lnl_units.spt != f.spt) {
             plk_status s = build_units(b, b->lnl_units, f.spt);
             if (s != PLK_OK) return s;
         }
         const BatchDev d = lnl_view(b, nullptr);
-        for (int per_sm = 1; per_sm <= occ; ++per_sm) {
+        // from the most CTAs an SM down, while that gets faster
+        float form_best = 1e30f;
+        int last_grid = 0;
+        for (int per_sm = occ; per_sm >= 1; --per_sm) {
             const int grid = std::min(b->lnl_units.n_units, per_sm * b->n_sms);
-            if (grid < 1) continue;
+            if (grid < 1 || grid == last_grid) continue;
+            last_grid = grid;
+            const BatchStreamShape shape =
+                f.stream ? batch_stream_shape(b->C, f.spt, b->max_ops, b->max_depth, per_sm) : BatchStreamShape{};
             float ms = 0.f;
             for (int rep = 0; rep < 3; ++rep) {  // warm-up, then two timed launches
                 PLK_BCUDA(b, cudaMemsetAsync(b->d_counter.p, 0, sizeof(int), b->stream), "clear work queue");
                 if (rep == 1) PLK_BCUDA(b, cudaEventRecord(e0, b->stream), "cudaEventRecord");
-                PLK_BCUDA(b, launch_batch_prune(d, f, grid, smem, b->stream), "batch post-order launch");
+                PLK_BCUDA(b, launch_form(b, d, f, grid, smem, shape), "batch post-order launch");
             }
             PLK_BCUDA(b, cudaEventRecord(e1, b->stream), "cudaEventRecord");
             PLK_BCUDA(b, cudaEventSynchronize(e1), "tune");
@@ -397,8 +470,10 @@ plk_status tune(plk_batch* b) {
                 best_form = f;
                 best_grid = grid;
                 best_smem = smem;
+                best_shape = shape;
             }
-            if (grid == b->lnl_units.n_units) break;
+            if (ms > form_best) break;
+            form_best = ms;
         }
     }
     cudaEventDestroy(e0);
@@ -407,6 +482,7 @@ plk_status tune(plk_batch* b) {
     b->form = best_form;
     b->grid = best_grid;
     b->smem = best_smem;
+    b->shape = best_shape;
     b->tuned_ms = best / 2.0;
     if (b->lnl_units.spt != best_form.spt) {
         plk_status s = build_units(b, b->lnl_units, best_form.spt);

@@ -124,7 +124,7 @@ __global__ void __maxnreg__(prune4w_maxnreg(KP, SPT, TPS, TS)) prune4w_kernel(Pr
         tab.ops = smem0 + pb + tb;
     } else {
         // [control][ring][ops, where they fit]
-        ring_init<KP>(tab, smem0, smem0 + kRingCtlBytes, tid == 0);
+        ring_init(tab, smem0, smem0 + kRingCtlBytes, tid == 0);
         tab.ops = a.sops;
         if (ops_smem) {
             int4* d = reinterpret_cast<int4*>(wtab + kRingCtlBytes + kRingSlots * RingTables<KP>::kSlotBytes);

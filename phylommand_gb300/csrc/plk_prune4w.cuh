@@ -83,11 +83,12 @@ struct SmemTables {
 // fills it next, so nothing waits for a free slot and no thread is set aside to
 // produce.  A wait for a stage is bounded: one that runs out stops further
 // copies and leaves ok false, and the caller makes its sites NaN.
-constexpr int kRingSlots = 4;
+constexpr int kRingSlots = 4;      // at most, and where one group has the SM
 constexpr int kRingCtlBytes = 64;  // per group: 4 mbarriers, 4 counters, the abort flag
 
-template <int KP>
+template <int KP, int SLOTS = kRingSlots>
 struct RingTables {
+    static_assert(SLOTS <= kRingSlots, "the control words hold four slots");
     static constexpr bool kOver = true;  // stack entries above the TMEM's in shared memory
     static constexpr uint32_t kSlotBytes = kStageUnits * KP * 128;
     uint32_t ring, ctl;   // shared-memory addresses of the slots and of the control words
@@ -99,10 +100,11 @@ struct RingTables {
     uint32_t base;        // its slot's address
     uint32_t phases;      // parity of every slot's next fill, kept from tree to tree
     bool ok;
+    int drain;            // stages that may be in flight after a wait ran out
 
     __device__ __forceinline__ void issue(int gg) const {  // one thread
         const int2 st = __ldg(stages + gg);
-        const uint32_t slot = (uint32_t)gg % kRingSlots, bar = ctl + 8 * slot, bytes = (uint32_t)st.y * (KP * 128);
+        const uint32_t slot = (uint32_t)gg % SLOTS, bar = ctl + 8 * slot, bytes = (uint32_t)st.y * (KP * 128);
         if (withhold) return;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
         asm volatile(
@@ -112,10 +114,12 @@ struct RingTables {
             : "memory");
     }
     __device__ __forceinline__ void start() const {  // one thread, all slots free
-        for (int i = 0; i < kRingSlots && i < n_stages; ++i) issue(i);
+        int stop;
+        asm volatile("ld.shared.s32 %0, [%1];\n" : "=r"(stop) : "r"(ctl + 48) : "memory");
+        for (int i = 0; !stop && i < SLOTS && i < n_stages; ++i) issue(i);
     }
     __device__ __forceinline__ void release() const {
-        const uint32_t cnt = ctl + 32 + 4 * ((uint32_t)g % kRingSlots);
+        const uint32_t cnt = ctl + 32 + 4 * ((uint32_t)g % SLOTS);
         __syncwarp();
         if ((threadIdx.x & 31) == 0) {
             int old, stop;
@@ -123,7 +127,7 @@ struct RingTables {
             if (old == warps - 1) {  // every warp has left the slot
                 asm volatile("st.shared.s32 [%0], 0;\nfence.acq_rel.cta;\n" ::"r"(cnt) : "memory");
                 asm volatile("ld.shared.s32 %0, [%1];\n" : "=r"(stop) : "r"(ctl + 48) : "memory");
-                if (!stop && g + kRingSlots < n_stages) issue(g + kRingSlots);
+                if (!stop && g + SLOTS < n_stages) issue(g + SLOTS);
             }
         }
     }
@@ -131,11 +135,15 @@ struct RingTables {
         if (!first_of_stage) return;
         if (g >= 0) release();
         ++g;
-        const uint32_t slot = (uint32_t)g % kRingSlots, bar = ctl + 8 * slot, par = (phases >> slot) & 1u;
+        const uint32_t slot = (uint32_t)g % SLOTS, bar = ctl + 8 * slot, par = (phases >> slot) & 1u;
         if (ok && !mbar_try_wait_bounded(bar, par)) {
             ok = false;
+            drain = withhold ? 0 : SLOTS;
             asm volatile("st.shared.s32 [%0], 1;\n" ::"r"(ctl + 48) : "memory");
-            if (!withhold) mbar_try_wait_bounded(bar, par);  // for a copy still in flight
+        }
+        if (!ok && drain > 0) {  // copies still in flight, this one and those issued ahead
+            --drain;
+            mbar_try_wait_bounded(bar, par);
         }
         phases ^= 1u << slot;
         base = ring + slot * kSlotBytes;
@@ -171,8 +179,8 @@ struct RingTables {
 
 // A group's control words at ctl, its slots at ring; one thread initialises
 // them, a barrier of the group follows before their use.
-template <int KP>
-__device__ __forceinline__ void ring_init(RingTables<KP>& tab, uint32_t ctl, uint32_t ring, bool leader) {
+template <int KP, int SLOTS>
+__device__ __forceinline__ void ring_init(RingTables<KP, SLOTS>& tab, uint32_t ctl, uint32_t ring, bool leader) {
     if (leader) {
         for (int i = 0; i < kRingSlots; ++i)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\nst.shared.s32 [%1], 0;\n" ::"r"(ctl + 8 * i),
@@ -186,6 +194,7 @@ __device__ __forceinline__ void ring_init(RingTables<KP>& tab, uint32_t ctl, uin
     tab.base = ring;
     tab.phases = 0;
     tab.ok = true;
+    tab.drain = 0;
 }
 
 // out[i] = sum_j r[j][i] x[j], j ascending, the first term a product (the
