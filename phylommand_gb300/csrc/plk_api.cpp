@@ -435,7 +435,7 @@ bool fused_kernel_applies(const plk_handle* h, int precision) {
 // alignment or model changes.  4 states: prune4_kernel and prune4s_kernel
 // with 1 and 2 sites per thread; 20 states: prune20_kernel on CUDA cores and
 // on tensor cores.  PLK_PRUNE_VARIANT=<n> forces candidate n where it applies.
-plk_status autotune_prune(plk_handle* h, PruneArgs a, const std::vector<int>& cands) {
+plk_status autotune_prune(plk_handle* h, PruneArgs a, std::vector<int> cands) {
     if (cands.empty()) return fail(h, PLK_ERR_STATE, "no post-order kernel applies");
     if (const char* f = getenv("PLK_PRUNE_VARIANT")) {
         const int v = atoi(f);
@@ -450,6 +450,19 @@ plk_status autotune_prune(plk_handle* h, PruneArgs a, const std::vector<int>& ca
     if (hit != h->tune_cache.end()) {
         h->variant = hit->second;
         return PLK_OK;
+    }
+    // Not timed: the warp-independent forms with two (four) sites a thread where
+    // one (two) leave no SM with a second warp.  There they have half the warps,
+    // each with more to do; a candidate costs a first evaluation 50 us and more
+    // (its kernel is loaded).
+    if (h->S == 4) {
+        const int sms = device_sm_count();
+        cands.erase(std::remove_if(cands.begin(), cands.end(),
+                                   [&](int v) {
+                                       return ((v == 13 || v == 16) && a.n_sites <= 32 * sms) ||
+                                              ((v == 14 || v == 17) && a.n_sites <= 64 * sms);
+                                   }),
+                    cands.end());
     }
     if (cands.size() == 1) {
         h->variant = cands[0];

@@ -216,6 +216,8 @@ cudaError_t launch_arena_copy(void* dst, const void* src_mapped, size_t bytes, c
 cudaError_t launch_check_codes(const uint8_t* codes, int n_tips, int n_sites, int stride, uint32_t all, int* bad,
                                int gen, cudaStream_t st);
 
+// SMs of the current device (of the first one asked; the engine's devices are alike)
+int device_sm_count();
 struct PruneArgs {
     const Op* ops;
     int n_ops;

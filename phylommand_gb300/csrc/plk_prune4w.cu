@@ -48,6 +48,17 @@ namespace plk {
 using namespace dev;
 using namespace dev4w;
 
+int device_sm_count() {
+    static std::atomic<int> n{0};
+    int v = n.load();
+    if (v > 0) return v;
+    int dev = 0, c = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || c <= 0) c = 1;
+    n.store(c);
+    return c;
+}
+
 namespace {
 
 constexpr int kWMinWarps = 4;
@@ -315,17 +326,6 @@ int prune4w_ctas_per_sm(int KP, int SPT, int TS, int warps, size_t smem, int TPS
     return n;
 }
 
-int sm_count() {
-    static std::atomic<int> n{0};
-    int v = n.load();
-    if (v > 0) return v;
-    int dev = 0, c = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || c <= 0) c = 1;
-    n.store(c);
-    return c;
-}
-
 // warps per CTA: enough that every SM's CTA has a tile per warp where the
 // tiles allow, at most what keeps the stacks within the TMEM and the
 // registers (and, for TS = 1, the tables) within one CTA per SM (0: no size
@@ -393,7 +393,7 @@ cudaError_t launch_prune4w(const PruneArgs& a, int spt, int ts, int tps, int* n_
                                   : kRingCtlBytes + (size_t)kRingSlots * kStageUnits * KP * 128 + (ops_smem ? op_bytes : 0);
     const int ws = 32 / tps * spt;  // sites per warp tile
     const int tiles = (a.n_sites + ws - 1) / ws;
-    const int sms = sm_count();
+    const int sms = device_sm_count();
     const int warps = prune4w_warps(KP, spt, ts, tps, tables, a.max_depth, tiles, sms);
     if (warps == 0) return cudaErrorInvalidConfiguration;
     const int levels = prune4w_levels(KP, spt, ts, warps, a.max_depth, tps);
