@@ -308,7 +308,69 @@ __global__ void __launch_bounds__(128) pmat4_eigen_kernel(DeviceModel m) {
     }
 }
 
+// P(t) of the reference's series for 4 states, two (node, category) matrices a
+// warp: lane 16 w + 4 i + j holds entry (i, j) of matrix w, through all 20
+// squarings.  What bounds it is their latency, one after another: a multiplication
+// and three additions of the FP64 pipe and an exchange through shared memory.
+// pmat_kernel, a matrix a CTA with a barrier and index divisions a squaring, took
+// 12.0 us for 31 matrices as for 205; here 7.7.  Operations and their order
+// are pmat_kernel's (p_kind 0), so are the bits.
+__global__ void __launch_bounds__(128) pmat4_series_kernel(DeviceModel m) {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    __shared__ double s_a[2][8][16];
+    const int w = threadIdx.x >> 4, e = threadIdx.x & 15, i = e >> 2, j = e & 3;
+    const int item = blockIdx.x * 8 + w;  // (node, category)
+    const int n_items = m.n_nodes * m.C;
+    const bool live = item < n_items;
+    const int it = live ? item : n_items - 1;  // lanes past the end repeat the last item, store nothing
+    const int v = it / m.C, k = it % m.C;
+    const double t = __dmul_rn(m.t_eff[v], m.cat_rate[k]);
+    const double q = __ddiv_rn(__dmul_rn(m.Q[e], t), 1048576.0);
+    double p = i == j ? __dadd_rn(1.0, q) : q;
+#pragma unroll 2
+    for (int n = 0; n < 20; ++n) {
+        double* a = s_a[n & 1][w];
+        a[e] = p;
+        __syncwarp();
+        const double2 r0 = *reinterpret_cast<const double2*>(a + 4 * i), r1 = *reinterpret_cast<const double2*>(a + 4 * i + 2);
+        p = __dmul_rn(r0.x, a[j]);
+        p = __dadd_rn(p, __dmul_rn(r0.y, a[4 + j]));
+        p = __dadd_rn(p, __dmul_rn(r1.x, a[8 + j]));
+        p = __dadd_rn(p, __dmul_rn(r1.y, a[12 + j]));
+    }
+    double* a = s_a[0][w];  // last read two squarings ago
+    a[e] = p;
+    __syncwarp();
+    if (!live) return;
+    const size_t base = (size_t)it * 16;
+    m.P64[base + e] = p;
+    m.P32[base + e] = (float)p;
+    if (m.P32p) m.P32p[(size_t)v * m.C * 16 + paired_p_index(k, i, j)] = (float)p;
+    if (m.stream && v >= m.n_tips) stream_store(m, v, k, paired_p_index(k, i, j), (float)p);
+    if (v >= m.n_tips) return;
+    const size_t tb = (size_t)it * m.n_codes * 4;
+    for (int c = j; c < m.n_codes; c += 4) {
+        const uint32_t mask = m.code_mask ? m.code_mask[c] : (uint32_t)c;
+        double acc = 0.0;
+        bool first = true;
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj)
+            if ((mask >> jj) & 1u) {
+                acc = first ? a[4 * i + jj] : __dadd_rn(acc, a[4 * i + jj]);
+                first = false;
+            }
+        m.tip64[tb + (size_t)c * 4 + i] = acc;
+        m.tip32[tb + (size_t)c * 4 + i] = (float)acc;
+        if (m.tip32p) m.tip32p[(size_t)v * m.C * kCodes * 4 + paired_tip_index(k, c, i)] = (float)acc;
+        if (m.stream) stream_store(m, v, k, paired_tip_index(k, c, i), (float)acc);
+    }
+}
+
 cudaError_t launch_pmat(const DeviceModel& m, int p_kind, cudaStream_t st) {
+    if (m.S == 4 && p_kind == 0 && m.B20 == nullptr) {
+        pmat4_series_kernel<<<(m.n_nodes * m.C + 7) / 8, 128, 0, st>>>(m);
+        return cudaGetLastError();
+    }
     if (m.S == 4 && p_kind == 1 && m.B20 == nullptr) {
         const int lanes = m.n_nodes * m.C * 4;
         pmat4_eigen_kernel<<<(lanes + 127) / 128, 128, 0, st>>>(m);
