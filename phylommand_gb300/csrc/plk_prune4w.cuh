@@ -371,6 +371,7 @@ struct CodeRing {
         cp_async_commit();
         c0 = get(o, 0), c1 = get(o, 1);
     }
+    __device__ __forceinline__ void next() {}
     __device__ __forceinline__ void finish() { cp_async_wait<0>(); }
 };
 
@@ -380,6 +381,7 @@ struct CodeRegs {
     const uint8_t* colp;  // the alignment's rows at this thread's sites
     int stride;
     int a0, a1, b0, b1;   // codes of the ops o, o + 1
+    int m0, m1;           // and o + 2, on their way
 
     template <class Tab>
     __device__ __forceinline__ void load(const Tab& tab, int n_ops, int o, int& c0, int& c1) const {
@@ -396,9 +398,12 @@ struct CodeRegs {
     }
     template <class Tab>
     __device__ __forceinline__ void step(const Tab& tab, int n_ops, int o, int& c0, int& c1) {
+        load(tab, n_ops, o + 2, m0, m1);
         c0 = a0, c1 = a1;
+    }
+    __device__ __forceinline__ void next() {
         a0 = b0, a1 = b1;
-        load(tab, n_ops, o + 2, b0, b1);
+        b0 = m0, b1 = m1;
     }
     __device__ __forceinline__ void finish() {}
 };
@@ -685,6 +690,7 @@ __device__ __forceinline__ void walk4w(Tab& tab, int n_ops, Codes codes, uint32_
             }
             ++sp;
         }
+        codes.next();
     }
     codes.finish();
     tab.finish();
