@@ -108,7 +108,7 @@ struct plk_handle {
     // P(t) and tip tables
     DevBuf d_P64, d_P32, d_tip64, d_tip32;
     // results and scratch
-    DevBuf d_site_lnl, d_block, d_lnl, d_work, d_cond, d_outside, d_nodes_out;
+    DevBuf d_site_lnl, d_block, d_work, d_cond, d_outside, d_nodes_out;
     DevBuf d_done;  // arrival counters (finish_grid_sum, then one per 128-site tile), zero between launches
     bool paired_written = false;  // this evaluation's P(t) kernel also wrote prune4p's layouts
     bool stream_written = false;  // or the streamed forms' tables
@@ -135,6 +135,11 @@ struct plk_handle {
     size_t arena_off = 0;
     cudaEvent_t arena_done = nullptr;
     int* h_flag = nullptr;
+    // the lnL: a mapped word that the pass (or the weighted sum) writes itself, so
+    // that reading a result is a synchronisation alone (its copy took
+    // 7 of 46 us of a small evaluation)
+    double* h_lnl = nullptr;
+    double* d_lnl = nullptr;  // its device address
     bool flag_pending = false;
     int flag_gen = 0;  // value the encode kernel stores for an empty cell of the current alignment
     // the tip masks' copy and encode run on copy_stream, so that the tree and
@@ -158,6 +163,7 @@ struct plk_handle {
         if (arena) cudaFreeHost(arena);
         if (arena_done) cudaEventDestroy(arena_done);
         if (h_flag) cudaFreeHost(h_flag);
+        if (h_lnl) cudaFreeHost(h_lnl);
         if (h_gen) cudaFreeHost(h_gen);
         if (main_done) cudaEventDestroy(main_done);
         if (codes_ready) cudaEventDestroy(codes_ready);
@@ -577,7 +583,10 @@ plk_status run_prune(plk_handle* h, int precision, NodePass* store, cudaEvent_t*
     const int blocks = std::max((h->n_sites + 63) / 64, any_blocks);
     PLK_CUDA(h, h->d_site_lnl.ensure(sizeof(double) * h->n_sites), "allocate site lnL");
     PLK_CUDA(h, h->d_block.ensure(sizeof(double) * 2 * (size_t)blocks), "allocate block sums");
-    PLK_CUDA(h, h->d_lnl.ensure(sizeof(double)), "allocate lnL");
+    if (!h->h_lnl) {
+        PLK_CUDA(h, cudaHostAlloc(&h->h_lnl, sizeof(double), cudaHostAllocMapped), "allocate lnL");
+        PLK_CUDA(h, cudaHostGetDevicePointer(&h->d_lnl, h->h_lnl, 0), "map lnL");
+    }
     // arrival counters, zero between launches: the grid's, then one per
     // 128-site tile (the 20-state compact form's in-kernel combine)
     const size_t counters = (1 + (size_t)(h->n_sites + 127) / 128) * sizeof(unsigned);
@@ -587,10 +596,10 @@ plk_status run_prune(plk_handle* h, int precision, NodePass* store, cudaEvent_t*
     }
     PruneArgs a = prune_args(h, precision);
     // the last CTA of the post-order pass (or of its per-site combine) adds
-    // up the block sums into d_lnl: no separate reduction launch
+    // up the block sums into the lnL word: no separate reduction launch
     a.grid_done = h->d_done.as<unsigned>();
     a.tile_done = h->d_done.as<unsigned>() + 1;
-    a.lnl_out = h->d_lnl.as<double>();
+    a.lnl_out = h->d_lnl;
     a.paired_ready = (precision == PLK_FP32S && h->paired_written) ? 1 : 0;
     a.withhold_first_stage = (precision == PLK_FP32S && h->withhold_stage) ? 1 : 0;
     if (precision == PLK_FP32S) h->withhold_stage = false;
@@ -1088,7 +1097,7 @@ plk_status plk_loglik_async(plk_handle* h, int precision) {
     if ((s = run_prune(h, precision, nullptr, ev ? &ev->e[2] : nullptr)) != PLK_OK) return s;
     if (h->patterns)  // every pattern's lnL counts once per site showing it
         PLK_CUDA(h, launch_weighted_sum(h->d_site_lnl.as<double>(), h->d_pattern_w.as<double>(), h->n_sites,
-                                        h->d_lnl.as<double>(), h->stream),
+                                        h->d_lnl, h->stream),
                  "weighted sum kernel launch");
     if (ev) PLK_CUDA(h, cudaEventRecord(ev->e[3], h->stream), "cudaEventRecord");
     h->lnl_pending = true;
@@ -1100,9 +1109,8 @@ plk_status plk_loglik_result(plk_handle* h, double* lnl_out) {
     if (!lnl_out) return fail(h, PLK_ERR_ARG, "lnl_out is NULL");
     *lnl_out = 0.0;
     if (!h->lnl_pending) return fail(h, PLK_ERR_STATE, "no evaluation enqueued (plk_loglik_async)");
-    double v = 0.0;
-    PLK_CUDA(h, cudaMemcpyAsync(&v, h->d_lnl.p, sizeof(double), cudaMemcpyDeviceToHost, h->stream), "copy lnL");
     PLK_CUDA(h, cudaStreamSynchronize(h->stream), "likelihood kernels");
+    const double v = *static_cast<volatile double*>(h->h_lnl);
     h->lnl_pending = false;
     if (h->flag_pending) {  // the alignment's empty-cell check, read back with this result
         h->flag_pending = false;
