@@ -110,7 +110,6 @@ __device__ __forceinline__ TileJob unit_job(const BatchDev& b, int2 unit, int ti
     j.C = b.C;
     j.tile_base = unit.y * tile;
     j.site_lnl = nullptr;
-    j.max_depth = b.max_depth;
     return j;
 }
 

@@ -964,9 +964,9 @@ bool down_takes(const plk_batch* b) {
 }
 
 // Plan of the down kernel for the batch's layout.  Warps per CTA: the fewest
-// (a power of two, up to 16) with which every warp tile of the batch is
+// (a power of two, or 12, the most) with which every warp tile of the batch is
 // resident at once, since an item's tables are then brought in for as few
-// idle warps as possible; 16 where there are more tiles than that.
+// idle warps as possible; 12 where there are more tiles than that.
 plk_status plan_down(plk_batch* b, DownPlan& p, bool blen) {
     if (p.ready) return PLK_OK;
     if (!down_takes(b))

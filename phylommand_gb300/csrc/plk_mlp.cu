@@ -3,8 +3,8 @@
 // from fixed values, src/treeator.cpp:612-615).
 //
 //  rows_kernel       (networks up to 256 wide) the whole forward pass, the loss
-//                    and the chain of activation gradients of 128 rows in one
-//                    CTA, activations staying in shared memory.
+//                    and the chain of activation gradients of a row block in one
+//                    cluster of four CTAs, activations staying on chip.
 //  update_kernel     weight and bias gradients of a tile over the whole batch,
 //                    and on them, still in registers, the Adam step.
 // Wider networks run layer by layer:

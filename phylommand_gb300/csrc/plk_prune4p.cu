@@ -86,7 +86,6 @@ __global__ void __launch_bounds__(kPruneThreads) prune4p_kernel(PruneArgs a, con
     j.C = 2 * KP;
     j.tile_base = blockIdx.x * tile4p_sites<SPT, TPS>();
     j.site_lnl = a.site_lnl;
-    j.max_depth = a.max_depth;
     SiteSum32 sum;
     run_tile4p<KP, SPT, CODES, TPS>(j, sm, sum);
     const SiteSum32 bsum = block_sum_site32f(sum);
@@ -125,7 +124,6 @@ __global__ void __launch_bounds__(kPruneThreads) prune4p_bulk_kernel(PruneArgs a
     j.C = 2 * KP;
     j.tile_base = blockIdx.x * kPruneThreads;
     j.site_lnl = a.site_lnl;
-    j.max_depth = a.max_depth;
     SiteSum32 sum;
     run_tile4p_bulk<KP>(j, sm, bars, &s_abort, sum, a.withhold_first_stage != 0);
     const SiteSum32 bsum = block_sum_site32f(sum);

@@ -42,7 +42,6 @@ __global__ void __launch_bounds__(kPruneThreads) prune4s_kernel(PruneArgs a) {
     j.C = a.C;
     j.tile_base = blockIdx.x * kPruneThreads * SPT;
     j.site_lnl = a.site_lnl;
-    j.max_depth = a.max_depth;
     SiteSum32 sum;
     run_tile<CM, SPT, CODES_SMEM>(j, sm, sum);
     const SiteSum32 bsum = block_sum_site32f(sum);
