@@ -47,6 +47,14 @@ def test_same_bits_several_tiles_and_deep_stacks(monkeypatch, n_tips, n_sites, v
     np.testing.assert_array_equal(_sites(monkeypatch, case, variant), want)
 
 
+def test_an_op_list_above_shared_memory(monkeypatch):
+    # more than 96 KB of ops: read from global memory
+    case = _random_case(np.random.default_rng(3), 3300, 70, C=4, shape="yule", missing=0.02)
+    want = _sites(monkeypatch, case, "1")
+    for v in ("12", "13", "14"):
+        np.testing.assert_array_equal(_sites(monkeypatch, case, v), want, err_msg=v)
+
+
 def test_a_withheld_stage_times_out_and_the_handle_recovers(monkeypatch):
     rng = np.random.default_rng(79)
     left, right, bl, masks, Q, f, cr, cw = _random_case(rng, 40, 700, C=4)
