@@ -59,12 +59,17 @@ __global__ void __launch_bounds__(32 * kUnitWarps, ctas_per_sm(KP, SPT)) batch_p
     const uint32_t over =
         smem0 + (uint32_t)(sh.over_at + warp * max(b.max_depth - sh.levels, 0) * KP * 8 * SPT * 128 + lane * 4);
     Op* const s_ops = reinterpret_cast<Op*>(sm + sh.ops_at);
+    bool dead = false;  // a stage did not arrive (a bounded wait ran out)
     for (;;) {
         __syncthreads();  // every slot is free, the last unit's ops are no longer read
         if (tid == 0) s_unit = atomicAdd(b.counter, 1);
         __syncthreads();
         const int u = s_unit;
         if (u >= b.n_units) break;
+        if (dead) {  // no unit keeps an earlier evaluation's sum
+            if (tid == 0) b.unit_sums[2 * u] = b.unit_sums[2 * u + 1] = (double)__int_as_float(0x7fc00000);
+            continue;
+        }
         const int2 unit = b.units[u];
         const BatchItemDev it = b.items[unit.x];
         const Op* ops = b.sops + it.ops_off;
@@ -102,7 +107,7 @@ __global__ void __launch_bounds__(32 * kUnitWarps, ctas_per_sm(KP, SPT)) batch_p
             b.unit_sums[2 * u] = ts;
             b.unit_sums[2 * u + 1] = tc;
         }
-        if (__syncthreads_or(!tab.ok)) break;  // the units that are left go to the other CTAs
+        dead = __syncthreads_or(!tab.ok) != 0;
     }
     tmem_wait_st();  // every warp is done with its stack: free the TMEM
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
