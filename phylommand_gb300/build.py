@@ -24,7 +24,7 @@ CU_SOURCES = ["plk_kernels.cu", "plk_prune4s.cu", "plk_prune4p.cu", "plk_prune4w
               "plk_prune_any.cu", "plk_any32_lo.cu", "plk_any32_hi.cu", "plk_any64_lo.cu", "plk_any64_hi.cu",
               "plk_down32_lo.cu", "plk_down32_hi.cu", "plk_down64_lo.cu", "plk_down64_hi.cu", "plk_batch.cu",
               "plk_batch4w.cu", "plk_nni.cu", "plk_features.cu", "plk_mlp.cu", "plk_noalloc.cu", "plk_peak.cu"]
-CPP_SOURCES = ["plk_api.cpp", "plk_host.cpp", "plk_fit.cpp", "plk_batch_api.cpp", "plk_sim.cpp", "plk_io.cpp"]
+CPP_SOURCES = ["plk_api.cpp", "plk_launch.cpp", "plk_host.cpp", "plk_fit.cpp", "plk_batch_api.cpp", "plk_sim.cpp", "plk_io.cpp"]
 
 
 def _cuda_home() -> str:

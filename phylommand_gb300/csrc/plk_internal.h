@@ -208,6 +208,10 @@ cudaError_t launch_pmat(const DeviceModel& m, int p_kind, cudaStream_t st);
 // unique id of the current CUDA context (0 when it cannot be had): launch
 // set-up caches key on it, since a device reset resets kernel attributes
 unsigned long long current_ctx_id();
+// Dynamic shared memory that a CTA of kernel fn may have on the current device:
+// the limit of a CTA less the kernel's own static shared memory (0 where it
+// cannot be had).
+size_t smem_limit(const void* fn);
 // copies bytes (both addresses 16-byte aligned) from mapped pinned host
 // memory with loads over the host link instead of a DMA copy
 cudaError_t launch_arena_copy(void* dst, const void* src_mapped, size_t bytes, cudaStream_t st);

@@ -314,14 +314,20 @@ int prune4w_ctas_per_sm(int KP, int SPT, int TS, int warps, size_t smem, int TPS
     std::lock_guard<std::mutex> lock(mu);
     size_t& allowed = attr[std::make_tuple(dev, ctx, fn)];
     if (smem > allowed) {
-        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+            cudaGetLastError();  // a size that does not fit is no error of the next launch
+            return 0;
+        }
         allowed = smem;
     }
     const auto key = std::make_tuple(dev, ctx, fn, warps, smem);
     const auto it = occ.find(key);
     if (it != occ.end()) return it->second;
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, warps * 32, smem) != cudaSuccess) n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, warps * 32, smem) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
     occ[key] = n;
     return n;
 }
@@ -332,10 +338,11 @@ int prune4w_ctas_per_sm(int KP, int SPT, int TS, int warps, size_t smem, int TPS
 // works)
 int prune4w_warps(int KP, int SPT, int TS, int TPS, size_t smem, int depth, int tiles, int sms) {
     int hi = 0;
+    const size_t limit = smem_limit(prune4w_fn_of(KP, SPT, TS, TPS));
     for (int w = kWMaxWarps; w >= kWMinWarps; --w) {
         const int levels = prune4w_levels(KP, SPT, TS, w, depth, TPS);
         const size_t warp_bytes = prune4w_code_bytes(TS, SPT, TPS) + prune4w_over_bytes(KP, SPT, levels, depth, TPS);
-        if (levels > 0 && smem + w * warp_bytes <= kMaxSmem &&
+        if (levels > 0 && smem + w * warp_bytes <= limit &&
             prune4w_ctas_per_sm(KP, SPT, TS, w, smem + w * warp_bytes, TPS) >= 1) {
             hi = w;
             break;
