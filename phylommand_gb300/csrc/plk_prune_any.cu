@@ -8,7 +8,7 @@ namespace plk {
 
 namespace {
 
-constexpr size_t kAnySmem = 227 * 1024;
+constexpr size_t kAnySmem = 227 * 1024;  // of a CTA, the kernel's static bytes among them
 constexpr int kAnyWarps = 8;  // per CTA at most
 
 int any_sm_count() {
@@ -30,9 +30,9 @@ struct AnyPlan {
 };
 
 // H, warps per CTA and the tables' place for these counts; H = 0 where
-// nothing fits.  smem(H, launch): the bytes of a CTA.
+// nothing fits.  smem(H, launch): the dynamic bytes of a CTA, fixed: its static ones.
 template <class Smem>
-AnyPlan any_plan(int S, int C, bool fp64, int n_sites, int n_codes, int max_depth, int sms, Smem smem) {
+AnyPlan any_plan(int S, int C, bool fp64, int n_sites, int n_codes, int max_depth, int sms, size_t fixed, Smem smem) {
     AnyPlan best;
     const int tsz = fp64 ? 8 : 4;
     for (int H = 1; H <= 4; H *= 2) {
@@ -57,14 +57,14 @@ AnyPlan any_plan(int S, int C, bool fp64, int n_sites, int n_codes, int max_dept
         p.launch.warps = want;
         if (S <= 8) {
             const size_t need = smem(H, p.launch);
-            fits = need <= (per_sm <= kAnyWarps ? kAnySmem : kAnySmem / 2);
+            fits = need <= (per_sm <= kAnyWarps ? kAnySmem - fixed : kAnySmem / 2);
         }
         for (int slots = 3; slots >= 2 && !fits; --slots)
             for (int w = want; w >= 1 && !fits; --w) {
                 if (slots == 3 && w < (want + 1) / 2) break;  // rather two slots than half the warps
                 p.launch.slots = slots;
                 p.launch.warps = w;
-                fits = smem(H, p.launch) <= kAnySmem;
+                fits = smem(H, p.launch) <= kAnySmem - fixed;
             }
         if (!fits) continue;
         // FP64: the SM's FP64 pipe takes 16 cycles a warp instruction; FP32:
@@ -77,15 +77,18 @@ AnyPlan any_plan(int S, int C, bool fp64, int n_sites, int n_codes, int max_dept
     return best;
 }
 
-AnyPlan up_plan(const PruneArgs& a, int S, bool fp64, bool cond_nodes, int sms) {
-    return any_plan(S, a.C, fp64, a.n_sites, a.n_codes, a.max_depth, sms, [&](int H, dev::AnyLaunch p) {
-        static double some;
-        p.nodes = cond_nodes ? &some : nullptr;  // only its presence counts
-        return dev::any_smem(S, H, fp64, p, a);
-    });
+// node_pass: a pass for the node states (of conditional vectors, or of messages)
+AnyPlan up_plan(const PruneArgs& a, int S, bool fp64, bool node_pass, bool cond_nodes, int sms) {
+    return any_plan(S, a.C, fp64, a.n_sites, a.n_codes, a.max_depth, sms,
+                    dev::kSumStatic + (node_pass ? dev::kWeightStatic : 0),
+                    [&](int H, dev::AnyLaunch p) {
+                        static double some;
+                        p.nodes = cond_nodes ? &some : nullptr;  // only its presence counts
+                        return dev::any_smem(S, H, fp64, p, a);
+                    });
 }
 AnyPlan down_plan(const PreorderArgs& a, int S, bool fp64, int sms) {
-    return any_plan(S, a.C, fp64, a.n_sites, a.n_codes, 0, sms,
+    return any_plan(S, a.C, fp64, a.n_sites, a.n_codes, 0, sms, dev::kWeightStatic,
                     [&](int H, const dev::AnyLaunch& p) { return dev::any_down_smem(S, H, fp64, p, a); });
 }
 
@@ -96,7 +99,7 @@ int prune_any_blocks(const PruneArgs& a, int S, int precision, bool nodes, bool 
     if (S < 2 || S > kMaxStates || a.C > kMaxCats || a.n_ops < 1) return 0;
     if (!fp64 && !nodes && ((S == 4 && a.C <= 8) || S == 20)) return 0;  // the tuned FP32 forms
     const int sms = any_sm_count();
-    const AnyPlan p = up_plan(a, S, fp64, nodes && !marginal, sms);
+    const AnyPlan p = up_plan(a, S, fp64, nodes, nodes && !marginal, sms);
     if (p.H == 0) return 0;
     if (marginal) {
         PreorderArgs d{};
@@ -117,7 +120,7 @@ int prune_any_blocks(const PruneArgs& a, int S, int precision, bool nodes, bool 
 
 cudaError_t launch_prune_any(const PruneArgs& a, int S, int precision, int* n_blocks, cudaStream_t st) {
     const bool fp64 = precision == PLK_FP64;
-    AnyPlan p = up_plan(a, S, fp64, a.nodes != nullptr, any_sm_count());
+    AnyPlan p = up_plan(a, S, fp64, a.nodes || a.msg, a.nodes != nullptr, any_sm_count());
     if (p.H == 0) return cudaErrorInvalidConfiguration;
     p.launch.msg = a.msg;
     p.launch.nodes = a.nodes;

@@ -144,6 +144,13 @@ struct NodeWeights {
 // of the pass); the same quantities are carried as two FP32 parts (products and
 // sums with their exact rounding errors, Dekker 1971 / Knuth's TwoSum), 2^-45
 // relative, under vectors that are good to 2^-22.
+// Static shared memory of the kernels, which counts towards a CTA's limit: the
+// site sum's words and the last CTA's flag (post-order), the category weights
+// (node states).
+constexpr size_t kSumStatic = 32 * 2 * 8 + 32 * 4 + 16, kWeightStatic = sizeof(NodeWeights);
+// what a kernel gets without asking for more, static bytes taken off
+constexpr size_t kAnyUnasked = 48 * 1024 - kSumStatic - kWeightStatic;
+
 template <typename T, int S, int H>
 struct NodeOut {
     T* oc;         // [site * C + k][S][2]
@@ -794,7 +801,7 @@ template <typename T, int S, int H, bool kRes, bool kNodes>
 cudaError_t launch_any_t(const PruneArgs& a, const AnyLaunch& p, int blocks, cudaStream_t st) {
     auto kern = prune_any_kernel<T, S, H, kRes, kNodes>;
     const size_t smem = any_smem(S, H, std::is_same<T, double>::value, p, a);
-    if (smem > 48 * 1024) {
+    if (smem > kAnyUnasked) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
@@ -819,7 +826,7 @@ template <typename T, int S, int H, bool kRes>
 cudaError_t launch_down_any_t(const PreorderArgs& a, const AnyLaunch& p, int blocks, cudaStream_t st) {
     auto kern = down_any_kernel<T, S, H, kRes>;
     const size_t smem = any_down_smem(S, H, std::is_same<T, double>::value, p, a);
-    if (smem > 48 * 1024) {
+    if (smem > kAnyUnasked) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }

@@ -7,6 +7,7 @@ those of the staged form with one site a thread (variant 1)."""
 import numpy as np
 import pytest
 
+from oracle import oracle as O
 from phylommand_gb300 import plk
 from test_gpu_parity import _engine, _random_case
 
@@ -28,3 +29,44 @@ def test_streamed_tables_beside_a_full_shared_memory(monkeypatch, C, tips):
             with _engine(left, right, bl, masks, 4, Q, f, cr, cw) as h:
                 assert h.loglik(plk.PLK_FP32S) == pytest.approx(lnl, rel=1e-12)
                 np.testing.assert_array_equal(h.site_loglik(), site, err_msg=f"{n_tips} tips")
+
+
+# The first two shapes need just less than the 48 KB that a kernel has without
+# asking for more, static bytes left out; the others just less than 227 KB.
+# FP64 1e-11 (P(t) of the eigen form); FP32 2 S roundings an op, two vectors a
+# marginal.
+@pytest.mark.parametrize("S, C, n_tips, n_sites, shape, precision", [
+    (4, 1, 561, 5000, "caterpillar", plk.PLK_FP64), (5, 4, 327, 5000, "balanced", plk.PLK_FP32S),
+    (4, 1, 284, 200, "balanced", plk.PLK_FP64), (4, 1, 286, 200, "caterpillar", plk.PLK_FP64),
+    (5, 4, 158, 5000, "balanced", plk.PLK_FP32S), (5, 4, 174, 500, "balanced", plk.PLK_FP32S),
+    (20, 8, 207, 5000, "balanced", plk.PLK_FP64), (24, 4, 393, 5000, "balanced", plk.PLK_FP64)])
+def test_any_state_lnl_beside_a_full_shared_memory(S, C, n_tips, n_sites, shape, precision):
+    left, right, bl, masks, Q, f, cr, cw = _random_case(np.random.default_rng(S + n_tips), n_tips, n_sites, S=S, C=C,
+                                                        shape=shape)
+    some = np.linspace(0, n_sites - 1, 16).astype(int)  # the oracle's sites
+    orc = O.loglik(left, right, masks[:, some], plk.effective_lengths(left, right, bl, False), Q, f, cr, cw,
+                   p_mode=O.P_EXACT)
+    with _engine(left, right, bl, masks, S, Q, f, cr, cw) as h:
+        h.loglik(precision)
+        tol = 1e-11 if precision == plk.PLK_FP64 else 6e-8 * 2 * S * n_tips
+        np.testing.assert_allclose(h.site_loglik()[some], orc.site_lnl, rtol=1e-11, atol=tol)
+
+
+@pytest.mark.parametrize("S, C, n_tips, n_sites, shape, precision, mode", [
+    (4, 4, 31, 200, "caterpillar", plk.PLK_FP32S, plk.PLK_NODES_COND),
+    (4, 4, 31, 500, "caterpillar", plk.PLK_FP32S, plk.PLK_NODES_MARGINAL),
+    (4, 4, 147, 500, "caterpillar", plk.PLK_FP32S, plk.PLK_NODES_COND),
+    (4, 4, 147, 500, "yule", plk.PLK_FP32S, plk.PLK_NODES_MARGINAL),
+    (4, 2, 294, 500, "balanced", plk.PLK_FP32S, plk.PLK_NODES_MARGINAL),
+    (7, 2, 92, 1000, "caterpillar", plk.PLK_FP64, plk.PLK_NODES_MARGINAL),
+    (3, 1, 588, 1000, "balanced", plk.PLK_FP64, plk.PLK_NODES_COND)])
+def test_node_states_beside_a_full_shared_memory(S, C, n_tips, n_sites, shape, precision, mode):
+    left, right, bl, masks, Q, f, cr, cw = _random_case(np.random.default_rng(S + n_tips), n_tips, n_sites, S=S, C=C,
+                                                        shape=shape)
+    some = np.linspace(0, n_sites - 1, 16).astype(int)
+    orc = O.loglik(left, right, masks[:, some], plk.effective_lengths(left, right, bl, False), Q, f, cr, cw,
+                   p_mode=O.P_EXACT, want_cond_norm=True, want_marginal=True)
+    want = orc.cond_norm if mode == plk.PLK_NODES_COND else orc.marginal
+    with _engine(left, right, bl, masks, S, Q, f, cr, cw) as h:
+        got = h.node_states(mode, precision)[:, some]
+        np.testing.assert_allclose(got, want, rtol=0, atol=1e-11 if precision == plk.PLK_FP64 else 6e-8 * 4 * S * n_tips)
