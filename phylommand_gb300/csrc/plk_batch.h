@@ -109,6 +109,8 @@ struct DownSize {              // warps per CTA; the largest item whose tables s
 constexpr int kDownWarps = 12;  // per CTA at most
 int down_sites_per_warp(int C);
 int down_smem_bytes(int C, bool blen, bool in_smem, const DownSize& z);
+// the most a CTA may have of them
+size_t down_smem_limit(int C, bool blen, bool in_smem);
 // resident CTAs per SM
 int down_occupancy(int C, bool blen, bool in_smem, const DownSize& z);
 cudaError_t launch_down_tables(const BatchDev& b, const BlenDev& bd, cudaStream_t st);

@@ -981,6 +981,7 @@ plk_status plan_down(plk_batch* b, DownPlan& p, bool blen) {
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return b->items[x].n_nodes > b->items[y].n_nodes; });
     // the largest items whose tables do not fit read them through L1
     int far = 0, occ = 0;
+    const size_t limit = down_smem_limit(b->C, blen, true);
     DownSize& z = p.size;
     auto split = [&]() {
         for (far = 0; far < n_items; ++far) {
@@ -991,7 +992,7 @@ plk_status plan_down(plk_batch* b, DownPlan& p, bool blen) {
                 z.tips = std::max(z.tips, h.n_tips);
                 z.ints = std::max(z.ints, h.n_int);
             }
-            if ((size_t)down_smem_bytes(b->C, blen, true, z) <= kSmemLimit) return;
+            if ((size_t)down_smem_bytes(b->C, blen, true, z) <= limit) return;
         }
         z.nodes = z.tips = z.ints = 0;
     };

@@ -734,8 +734,11 @@ template <int KP, bool kSmem, int MODE>
 int occupancy_t(const Shape& sh) {
     auto kern = batch_down_kernel<KP, kSmem, MODE>;
     int n = 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sh.smem) != cudaSuccess) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, sh.warps * 32, sh.smem) != cudaSuccess) return 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sh.smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, sh.warps * 32, sh.smem) != cudaSuccess) {
+        cudaGetLastError();  // a size that does not fit is no error of the next launch
+        return 0;
+    }
     return n;
 }
 
@@ -760,6 +763,10 @@ struct ShapeOf {
     template <int KP, bool kSmem, int MODE>
     Shape operator()() const { return down_shape<KP, kSmem>(mode, warps, nodes, tips, ints); }
 };
+struct LimitOf {
+    template <int KP, bool kSmem, int MODE>
+    size_t operator()() const { return smem_limit(reinterpret_cast<const void*>(batch_down_kernel<KP, kSmem, MODE>)); }
+};
 struct OccOf {
     Shape sh;
     template <int KP, bool kSmem, int MODE>
@@ -782,6 +789,8 @@ int down_sites_per_warp(int C) { return 32 / ((C + 1) / 2); }
 int down_smem_bytes(int C, bool blen, bool in_smem, const DownSize& z) {
     return dispatch(C, in_smem, blen, ShapeOf{blen ? kBlen : kNni, z.warps, z.nodes, z.tips, z.ints}).smem;
 }
+
+size_t down_smem_limit(int C, bool blen, bool in_smem) { return dispatch(C, in_smem, blen, LimitOf{}); }
 
 int down_occupancy(int C, bool blen, bool in_smem, const DownSize& z) {
     const Shape sh = dispatch(C, in_smem, blen, ShapeOf{blen ? kBlen : kNni, z.warps, z.nodes, z.tips, z.ints});

@@ -9,6 +9,8 @@ import pytest
 
 from oracle import oracle as O
 from phylommand_gb300 import plk
+from phylommand_gb300.nni import neighbour_tree
+from test_gpu_batch import _single
 from test_gpu_parity import _engine, _random_case
 
 pytestmark = pytest.mark.gpu
@@ -70,3 +72,30 @@ def test_node_states_beside_a_full_shared_memory(S, C, n_tips, n_sites, shape, p
     with _engine(left, right, bl, masks, S, Q, f, cr, cw) as h:
         got = h.node_states(mode, precision)[:, some]
         np.testing.assert_allclose(got, want, rtol=0, atol=1e-11 if precision == plk.PLK_FP64 else 6e-8 * 4 * S * n_tips)
+
+
+# One item whose tables take the last 64 of 227 KB: they go through L1 instead.
+# Tolerances as in test_gpu_down.
+@pytest.mark.parametrize("C, n_tips, n_sites", [(5, 253, 700), (1, 464, 38000)])
+def test_nni_beside_a_full_shared_memory(C, n_tips, n_sites):
+    left, right, bl, masks, Q, f, cr, cw = _random_case(np.random.default_rng(C), n_tips, n_sites, C=C)
+    with plk.Batch(C) as b:
+        b.set_model(b.add(masks, left, right, bl), Q, f, cr, cw)
+        got, moves = b.nni_loglik()[0], b.nni_moves(0)
+    for m in (0, 1, len(moves) // 2, len(moves) - 1):
+        L, R = neighbour_tree(left, right, int(moves[m][0]), int(moves[m][1]))
+        assert got[m] == pytest.approx(_single(masks, L, R, bl, Q, f, cr, cw, plk.PLK_FP64), rel=1e-6)
+
+
+def test_edge_derivatives_beside_a_full_shared_memory():
+    C, n_tips, n_sites = 6, 226, 20000
+    left, right, bl, masks, Q, f, cr, cw = _random_case(np.random.default_rng(C), n_tips, n_sites, C=C)
+    with plk.Batch(C) as b:
+        b.set_model(b.add(masks, left, right, bl), Q, f, cr, cw)
+        d = b.edge_derivatives()[0]
+    for v in (0, n_tips // 2, n_tips + 7):
+        eps = 1e-4 * max(bl[v], 1e-2)
+        lp, lm = (_single(masks, left, right, np.where(np.arange(len(bl)) == v, x, bl), Q, f, cr, cw, plk.PLK_FP64)
+                  for x in (bl[v] + eps, bl[v] - eps))
+        d1 = (lp - lm) / (2 * eps)
+        assert abs(d[v, 0] - d1) <= 2e-4 * (abs(d1) + n_sites), (v, d[v], d1)
