@@ -228,8 +228,11 @@ int batch_occupancy(int C, const BatchForm& f, size_t smem) {
     const BatchKernel kern = form_kernel(C, f, 0, 0, 0, &unused);
     int n = 0;
     if (!kern) return 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, kPruneThreads, smem) != cudaSuccess) return 0;
+    if (allow_smem(reinterpret_cast<const void*>(kern), smem) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, kPruneThreads, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
     return n;
 }
 
@@ -246,7 +249,7 @@ cudaError_t launch_batch_prune(const BatchDev& b, const BatchForm& f, int grid, 
     size_t unused = 0;
     const BatchKernel kern = form_kernel(b.C, f, 0, 0, 0, &unused);
     if (!kern || (f.paired && (!b.P32p || !b.tip32p))) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), smem);
     if (e != cudaSuccess) return e;
     kern<<<grid, kPruneThreads, smem, st>>>(b);
     return cudaGetLastError();

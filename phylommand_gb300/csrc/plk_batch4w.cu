@@ -167,7 +167,7 @@ BatchStreamShape batch_stream_shape(int C, int spt, int max_ops, int max_depth, 
     if (at > 227 * 1024 || cudaGetDevice(&dev) != cudaSuccess || cudaFuncGetAttributes(&fa, kern) != cudaSuccess ||
         cudaDeviceGetAttribute(&sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess ||
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)at) != cudaSuccess) {
+        allow_smem(reinterpret_cast<const void*>(kern), at) != cudaSuccess) {
         cudaGetLastError();
         return s;
     }
@@ -180,7 +180,7 @@ BatchStreamShape batch_stream_shape(int C, int spt, int max_ops, int max_depth, 
 cudaError_t launch_batch_prune4w(const BatchDev& b, const BatchStreamShape& sh, int spt, int grid, cudaStream_t st) {
     const StreamKernel kern = stream_kernel(b.C, spt);
     if (!kern || !b.stream || sh.smem == 0) return cudaErrorInvalidValue;
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
+    const cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), sh.smem);
     if (e != cudaSuccess) return e;
     kern<<<grid, 32 * kUnitWarps, sh.smem, st>>>(b, sh);
     return cudaGetLastError();

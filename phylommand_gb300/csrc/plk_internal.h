@@ -212,6 +212,9 @@ unsigned long long current_ctx_id();
 // the limit of a CTA less the kernel's own static shared memory (0 where it
 // cannot be had).
 size_t smem_limit(const void* fn);
+// Lets launches of kernel fn on the current device have at least `bytes` of
+// dynamic shared memory; a refusal leaves no error pending.  Thread-safe.
+cudaError_t allow_smem(const void* fn, size_t bytes);
 // copies bytes (both addresses 16-byte aligned) from mapped pinned host
 // memory with loads over the host link instead of a DMA copy
 cudaError_t launch_arena_copy(void* dst, const void* src_mapped, size_t bytes, cudaStream_t st);

@@ -710,12 +710,12 @@ static cudaError_t launch_prune4(const PruneArgs& a, bool store, int blocks, cud
     cudaError_t err;
     if (store) {
         auto kern = prune4_kernel<T, CM, EXACT, true>;
-        err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        err = allow_smem(reinterpret_cast<const void*>(kern), smem);
         if (err != cudaSuccess) return err;
         kern<<<blocks, kPruneThreads, smem, st>>>(a);
     } else {
         auto kern = prune4_kernel<T, CM, EXACT, false>;
-        err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        err = allow_smem(reinterpret_cast<const void*>(kern), smem);
         if (err != cudaSuccess) return err;
         kern<<<blocks, kPruneThreads, smem, st>>>(a);
     }

@@ -724,7 +724,7 @@ template <int KP, bool kSmem, int MODE>
 cudaError_t launch_t(const BatchDev& b, const BlenDev& bd, const Shape& sh, int unit0, int unit1, int grid,
                      cudaStream_t st) {
     auto kern = batch_down_kernel<KP, kSmem, MODE>;
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sh.smem);
+    const cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), sh.smem);
     if (e != cudaSuccess) return e;
     kern<<<grid, sh.warps * 32, sh.smem, st>>>(b, bd, sh, unit0, unit1);
     return cudaGetLastError();
@@ -734,7 +734,7 @@ template <int KP, bool kSmem, int MODE>
 int occupancy_t(const Shape& sh) {
     auto kern = batch_down_kernel<KP, kSmem, MODE>;
     int n = 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sh.smem) != cudaSuccess ||
+    if (allow_smem(reinterpret_cast<const void*>(kern), sh.smem) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, sh.warps * 32, sh.smem) != cudaSuccess) {
         cudaGetLastError();  // a size that does not fit is no error of the next launch
         return 0;

@@ -577,7 +577,7 @@ cudaError_t launch_prune20(const PruneArgs& a, int n_nodes, int variant, void* s
     dim3 grid((a.n_sites + kTile - 1) / kTile, a.C);
     cudaError_t e;
     auto run = [&](auto kern) -> cudaError_t {
-        cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t r = allow_smem(reinterpret_cast<const void*>(kern), smem);
         if (r != cudaSuccess) return r;
         kern<<<grid, 32 * warps, smem, st>>>(g);
         return cudaGetLastError();

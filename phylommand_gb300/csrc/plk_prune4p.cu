@@ -136,7 +136,7 @@ cudaError_t launch4p_bulk(const PruneArgs& a, const float* Pp, const float* Tp, 
     const size_t smem = tile4p_bulk_smem_bytes<KP>(a.n_ops, a.max_depth);
     if (smem > 227 * 1024) return cudaErrorInvalidConfiguration;
     auto kern = prune4p_bulk_kernel<KP>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), smem);
     if (e != cudaSuccess) return e;
     const int blocks = (a.n_sites + kPruneThreads - 1) / kPruneThreads;
     *n_blocks = blocks;
@@ -149,7 +149,7 @@ cudaError_t launch4p(const PruneArgs& a, const float* Pp, const float* Tp, int* 
     const size_t smem = tile4p_smem_bytes<KP, SPT, CODES, TPS>(a.n_ops, a.n_tips, a.max_depth);
     if (smem > 227 * 1024) return cudaErrorInvalidConfiguration;
     auto kern = prune4p_kernel<KP, SPT, CODES, TPS>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), smem);
     if (e != cudaSuccess) return e;
     constexpr int TILE = tile4p_sites<SPT, TPS>();
     const int blocks = (a.n_sites + TILE - 1) / TILE;

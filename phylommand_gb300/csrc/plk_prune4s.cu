@@ -54,7 +54,7 @@ cudaError_t launch_one(const PruneArgs& a, int* n_blocks, cudaStream_t st) {
     const size_t smem = tile_smem_bytes<CM, SPT, CODES_SMEM>(a.n_ops, a.n_tips, a.max_depth);
     if (smem > kMaxSmem) return cudaErrorInvalidConfiguration;
     auto kern = prune4s_kernel<CM, SPT, CODES_SMEM>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), smem);
     if (e != cudaSuccess) return e;
     const int blocks = (a.n_sites + kPruneThreads * SPT - 1) / (kPruneThreads * SPT);
     *n_blocks = blocks;

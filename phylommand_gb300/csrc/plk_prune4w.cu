@@ -310,16 +310,8 @@ int prune4w_ctas_per_sm(int KP, int SPT, int TS, int warps, size_t smem, int TPS
     const unsigned long long ctx = current_ctx_id();  // a device reset starts the caches over
     static std::mutex mu;
     static std::map<std::tuple<int, unsigned long long, const void*, int, size_t>, int> occ;
-    static std::map<std::tuple<int, unsigned long long, const void*>, size_t> attr;  // the largest size allowed
+    if (allow_smem(fn, smem) != cudaSuccess) return 0;
     std::lock_guard<std::mutex> lock(mu);
-    size_t& allowed = attr[std::make_tuple(dev, ctx, fn)];
-    if (smem > allowed) {
-        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-            cudaGetLastError();  // a size that does not fit is no error of the next launch
-            return 0;
-        }
-        allowed = smem;
-    }
     const auto key = std::make_tuple(dev, ctx, fn, warps, smem);
     const auto it = occ.find(key);
     if (it != occ.end()) return it->second;

@@ -148,8 +148,6 @@ struct NodeWeights {
 // site sum's words and the last CTA's flag (post-order), the category weights
 // (node states).
 constexpr size_t kSumStatic = 32 * 2 * 8 + 32 * 4 + 16, kWeightStatic = sizeof(NodeWeights);
-// what a kernel gets without asking for more, static bytes taken off
-constexpr size_t kAnyUnasked = 48 * 1024 - kSumStatic - kWeightStatic;
 
 template <typename T, int S, int H>
 struct NodeOut {
@@ -801,10 +799,8 @@ template <typename T, int S, int H, bool kRes, bool kNodes>
 cudaError_t launch_any_t(const PruneArgs& a, const AnyLaunch& p, int blocks, cudaStream_t st) {
     auto kern = prune_any_kernel<T, S, H, kRes, kNodes>;
     const size_t smem = any_smem(S, H, std::is_same<T, double>::value, p, a);
-    if (smem > kAnyUnasked) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), smem);
+    if (e != cudaSuccess) return e;
     kern<<<blocks, p.warps * 32, smem, st>>>(a, p);
     return cudaGetLastError();
 }
@@ -826,10 +822,8 @@ template <typename T, int S, int H, bool kRes>
 cudaError_t launch_down_any_t(const PreorderArgs& a, const AnyLaunch& p, int blocks, cudaStream_t st) {
     auto kern = down_any_kernel<T, S, H, kRes>;
     const size_t smem = any_down_smem(S, H, std::is_same<T, double>::value, p, a);
-    if (smem > kAnyUnasked) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), smem);
+    if (e != cudaSuccess) return e;
     kern<<<blocks, p.warps * 32, smem, st>>>(a, p);
     return cudaGetLastError();
 }
