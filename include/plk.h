@@ -373,6 +373,13 @@ plk_status plk_mlp_gradients(plk_mlp* m, int batch, const float* x, const float*
  * the step into *loss (may be NULL). */
 plk_status plk_mlp_train_step(plk_mlp* m, int batch, const float* x, const float* t, float lr,
                               float* loss);
+/* Every device wait of the networks up to 256 wide is bounded; a pass in which
+ * one runs out returns PLK_ERR_TIMEOUT, a train step then with the weights as
+ * they were (the row kernel gave up) or in part updated (the update kernel did;
+ * the message says which), and the network stays usable.  Test of that path:
+ * the next pass's row kernel (where = 1) does not get its last weights, or its
+ * update kernel (2) not the signal of its last tile's products. */
+plk_status plk_mlp_test_withhold(plk_mlp* m, int where);
 
 /* ---- branch lengths (no counterpart in the reference: its branch lengths
  * are fixed inputs, src/tree.cpp:136, 176) ------------------------------------

@@ -280,8 +280,11 @@ __global__ void __launch_bounds__(128, 1) gemm_tc_kernel(GemmArgs g) {
 // this in 29.  update_kernel then has a CTA per 128 x 32 tile of every
 // weight matrix, the batch as K; its operands are transposed on the way by
 // ldmatrix.trans / stmatrix.  A step, with the host's part, 525 -> 65 us.
-// Every wait on an mbarrier is bounded; one that runs out raises the network's
-// fail flag, so the loss is NaN and the weights stay as they were.
+// Every wait on an mbarrier is bounded.  One that runs out in rows_kernel raises
+// `fail`, on which update_kernel leaves the weights as they were, and the host's
+// word; one that runs out in update_kernel raises the host's other word (that
+// tile's weights stay as they were, other tiles' do not).  The host reads both
+// after the pass and reports PLK_ERR_TIMEOUT.
 // ---------------------------------------------------------------------------
 constexpr int kNetWide = 256;   // widest layer (padded to 16)
 constexpr int kNetLayers = 8;   // weight layers
@@ -306,7 +309,9 @@ struct NetArgs {
     float* y;                         // [batch][n_out]
     float* loss_part;                 // [CTAs]
     float* loss;
-    int* fail;
+    int* fail;                        // rows_kernel gave up
+    volatile int* gave_up;            // the same for the host [rows_kernel, update_kernel]
+    int withhold;                     // test of the failure path (plk_mlp_test_withhold)
     float *p, *g, *m, *v;
     float lr, b1, b2, eps, c1, c2;
 };
@@ -320,8 +325,9 @@ __device__ __forceinline__ size_t net_image_at(int n, int k, int N, int K) {
     return ((size_t)(n / w * (K / 8) + (k >> 3)) * w + n % w) * 8 + (k & 7);
 }
 
+constexpr int kNetWaitLimit = 1 << 18;  // about a second
 __device__ __forceinline__ bool net_wait(uint32_t mbar, uint32_t parity) {
-    for (int it = 0; it < kGWaitLimit; ++it) {
+    for (int it = 0; it < kNetWaitLimit; ++it) {
         uint32_t ok;
         asm volatile(
             "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
@@ -335,7 +341,8 @@ __device__ __forceinline__ bool net_wait(uint32_t mbar, uint32_t parity) {
 }
 
 // the MMAs of a K-deep product, A [K / 8][128][8] and B [K / 8][N][8], committed to mbar
-__device__ __forceinline__ void net_mma(uint32_t tmem, uint32_t a, uint32_t b, int N, int K, bool first, uint32_t mbar) {
+__device__ __forceinline__ void net_mma(uint32_t tmem, uint32_t a, uint32_t b, int N, int K, bool first, uint32_t mbar,
+                                        bool commit = true) {
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((kGM >> 4) << 24);
     // one thread issues them: a step of K is an addition to each descriptor's
     // address (16-byte units; the operands lie below 256 KB, so nothing carries)
@@ -351,7 +358,8 @@ __device__ __forceinline__ void net_mma(uint32_t tmem, uint32_t a, uint32_t b, i
         bd += 2 * N;
         accum = 1u;
     }
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar) : "memory");
+    if (commit)
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar) : "memory");
 }
 
 __device__ __forceinline__ void net_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
@@ -387,7 +395,7 @@ __device__ __forceinline__ uint4 net_pack8(const float* v) {
 
 // TMEM and the mbarriers of a CTA (all threads call it)
 constexpr int kNetBars = 5;
-__device__ __forceinline__ uint32_t net_begin(uint32_t* s_tmem, uint64_t* s_bar, int* s_fail, int cols) {
+__device__ __forceinline__ uint32_t net_begin(uint32_t* s_tmem, uint64_t* s_bar, int cols) {
     const uint32_t bar = static_cast<uint32_t>(__cvta_generic_to_shared(s_bar));
     if (threadIdx.x < 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
@@ -400,7 +408,6 @@ __device__ __forceinline__ uint32_t net_begin(uint32_t* s_tmem, uint64_t* s_bar,
         for (int i = 0; i < kNetBars; ++i)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar + 8 * i) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-        *s_fail = 0;
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
@@ -430,7 +437,6 @@ __global__ void __cluster_dims__(kNetCtas, 1, 1) __launch_bounds__(kNetThreads, 
     // MMAs done, weights landed (two buffers), the other CTAs' slices of A landed (two)
     __shared__ __align__(8) uint64_t s_bar[kNetBars];
     __shared__ uint32_t s_tmem;
-    __shared__ int s_fail;
     __shared__ float s_red[kNetThreads];
     __shared__ __align__(16) float s_bias[kNetLayers][net_share(kNetWide)];
     __shared__ uint32_t s_pos[kNetLayers][kNetThreads];  // ReLU: the positive ones of a thread's 32 columns
@@ -438,12 +444,13 @@ __global__ void __cluster_dims__(kNetCtas, 1, 1) __launch_bounds__(kNetThreads, 
     const int rank = blockIdx.x % kNetCtas, row0 = blockIdx.x / kNetCtas * kGM;
     const uint32_t a_sm = static_cast<uint32_t>(__cvta_generic_to_shared(net_sm)), w_sm = a_sm + 2 * kRowsA;
     const uint32_t bar = static_cast<uint32_t>(__cvta_generic_to_shared(s_bar));
-    const uint32_t tmem = net_begin(&s_tmem, s_bar, &s_fail, net_share(kNetWide));
+    const uint32_t tmem = net_begin(&s_tmem, s_bar, net_share(kNetWide));
     const int L = n.L, steps = n.backward ? 2 * L - 1 : L;
     // step st: layer l forward (st < L) or back (layers L - 1 .. 1)
     auto layer_of = [&](int st) { return st < L ? st : 2 * L - 1 - st; };
     // thread 0: this CTA's slice of step st's weights, in 32 KB copies
     auto load_w = [&](int st) {
+        if (n.withhold == 1 && blockIdx.x == kNetCtas - 1 && st == steps - 1) return;
         const NetLayer& ly = n.layer[layer_of(st)];
         const int N = st < L ? ly.pout : ly.pin, K = st < L ? ly.pin : ly.pout;
         const uint32_t bytes = (uint32_t)(net_share(N) * K * 2), to = w_sm + (st & 1) * kRowsW, b = bar + 8 + 8 * (st & 1);
@@ -506,33 +513,37 @@ __global__ void __cluster_dims__(kNetCtas, 1, 1) __launch_bounds__(kNetThreads, 
     const uint32_t trow = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
     float sq = 0.0f;
     uint32_t mma_phase = 0;
+    // failed: a wait ran out; the CTA then multiplies and loads no more but keeps
+    // step, as the others wait for its slices.  loaded: this step's weights were asked for.
+    bool failed = false, loaded = true;
     for (int st = 0; st < steps; ++st) {
         const bool fwd = st < L, last = st == L - 1;
         const int l = layer_of(st);
         const NetLayer& ly = n.layer[l];
         const int N = fwd ? ly.pout : ly.pin, K = fwd ? ly.pin : ly.pout, share = net_share(N), n0 = rank * share;
-        if (!net_wait(bar + 8 + 8 * (st & 1), (st >> 1) & 1)) {
+        if (loaded && !net_wait(bar + 8 + 8 * (st & 1), (st >> 1) & 1)) {
             net_wait(bar + 8 + 8 * (st & 1), (st >> 1) & 1);  // a last bounded wait for the copy in flight
-            s_fail = 1;
+            failed = true;
         }
         if (st > 0 && !net_wait(bar + 24 + 8 * (st & 1), ((st - 1) >> 1) & 1)) {
             net_wait(bar + 24 + 8 * (st & 1), ((st - 1) >> 1) & 1);
-            s_fail = 1;
+            failed = true;
         }
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-        __syncthreads();
-        const bool go = s_fail == 0 && n0 < N;  // a CTA past the last columns only keeps step
+        failed = __syncthreads_or(failed) != 0;
+        loaded = !failed;
+        const bool go = !failed && n0 < N;  // a CTA past the last columns only keeps step
         if (go && tid == 0) {
             asm volatile("fence.proxy.async;\n" ::: "memory");
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             net_mma(tmem, a_sm + (st & 1) * kRowsA, w_sm + (st & 1) * kRowsW, share, K, true, bar);
         }
         // the other buffer's products were waited for in the step before
-        if (tid == 32 && st + 1 < steps) load_w(st + 1);
+        if (tid == 32 && st + 1 < steps && loaded) load_w(st + 1);
         bool done = false;
         if (go) {
             done = net_wait(bar, mma_phase) || net_wait(bar, mma_phase);
-            if (!done) s_fail = 1;
+            if (!done) failed = true;
             mma_phase ^= 1u;
         }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -637,12 +648,7 @@ __global__ void __cluster_dims__(kNetCtas, 1, 1) __launch_bounds__(kNetThreads, 
         }
     }
     cluster_barrier();  // every copy from and into this CTA's shared memory has landed
-    if (s_fail) {
-        if (tid == 0) *n.fail = 1;
-        if (n.y && warp < 4 && row < n.batch && rank == 0)
-            for (int c = 0; c < n.layer[L - 1].out; ++c)
-                n.y[(size_t)row * n.layer[L - 1].out + c] = __int_as_float(0x7fc00000);
-    }
+    if (__syncthreads_or(failed) && tid == 0) *n.fail = n.gave_up[0] = 1;
     if (n.backward) {
         s_red[tid] = sq;
         __syncthreads();
@@ -711,11 +717,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) update_kernel(const __grid_con
     extern __shared__ __align__(128) unsigned char net_sm[];
     __shared__ __align__(8) uint64_t s_bar[kNetBars];
     __shared__ uint32_t s_tmem;
-    __shared__ int s_fail;
-    if (*n.fail) {  // a row block gave up: no update, and the loss says so
-        if (blockIdx.x == 0 && threadIdx.x == 0) *n.loss = __int_as_float(0x7fc00000);
-        return;
-    }
+    if (*n.fail) return;  // a row block gave up (nothing in this launch writes the flag): no update
     int l = 0;
     while (l + 1 < n.L && (int)blockIdx.x >= n.layer[l + 1].tile0) ++l;
     const NetLayer& ly = n.layer[l];
@@ -724,7 +726,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) update_kernel(const __grid_con
     unsigned char *stA = net_sm + kUpOpA + kUpOpB, *stB = stA + kUpStageA;
     const uint32_t a_sm = static_cast<uint32_t>(__cvta_generic_to_shared(net_sm));
     const uint32_t bar = static_cast<uint32_t>(__cvta_generic_to_shared(s_bar));
-    const uint32_t tmem = net_begin(&s_tmem, s_bar, &s_fail, kUpN);
+    const uint32_t tmem = net_begin(&s_tmem, s_bar, kUpN);
     float bias = 0.0f;  // thread o < 128 of the tiles with n0 = 0: the bias gradient of output m0 + o
     bool ok = true;
     uint32_t phase = 0;
@@ -741,19 +743,15 @@ __global__ void __launch_bounds__(kNetThreads, 1) update_kernel(const __grid_con
         __syncthreads();
         if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            net_mma(tmem, a_sm, a_sm + kUpOpA, kUpN, K, k0 == 0, bar);
+            net_mma(tmem, a_sm, a_sm + kUpOpA, kUpN, K, k0 == 0, bar, n.withhold != 2 || blockIdx.x + 1 < gridDim.x);
         }
         if (n0 == 0 && tid < kGM)
 #pragma unroll 16
             for (int r = 0; r < K; ++r)
                 bias += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(stA + (size_t)r * kUpPitchA + 2 * tid));
-        if (!net_wait(bar, phase)) {
-            net_wait(bar, phase);
-            s_fail = 1;
-        }
+        const bool done = net_wait(bar, phase) || net_wait(bar, phase);
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        __syncthreads();
-        ok = s_fail == 0;
+        ok = __syncthreads_and(done) != 0;
         if (!ok) break;
     }
     // the tile's gradient through shared memory, so that the parameters and
@@ -833,12 +831,12 @@ __global__ void __launch_bounds__(kNetThreads, 1) update_kernel(const __grid_con
             n.g[i] = bias;
         }
     }
-    if (tid == 0 && !ok) *n.fail = 1;
+    if (tid == 0 && !ok) n.gave_up[1] = 1;
     if (blockIdx.x == 0 && tid == 0) {
         float s = 0.0f;
         for (int i = 0; i < row_ctas; ++i) s += n.loss_part[i];
         const NetLayer& top = n.layer[n.L - 1];
-        *n.loss = ok ? s / ((float)n.batch * top.out) : __int_as_float(0x7fc00000);
+        *n.loss = s / ((float)n.batch * top.out);
     }
     net_end(tmem, kUpN);
 }
@@ -891,6 +889,7 @@ struct plk_mlp {
     int* fail = nullptr;
     char *host = nullptr, *host_dev = nullptr;
     size_t host_bytes = 0;
+    int withhold = 0;  // armed by plk_mlp_test_withhold for the next pass
     ~plk_mlp() {
         for (auto* v : {&wf, &wt, &n_act, &n_dz})
             for (auto* q : *v) cudaFree(q);
@@ -960,8 +959,8 @@ plk_status net_images(plk_mlp* m) {
     return PLK_OK;
 }
 
-// Room for `batch` rows, and the pinned block: [loss][x][t], read and written
-// by the kernels in place.
+// Room for `batch` rows, and the pinned block: [loss, the kernels' gave-up
+// words][x][t], read and written by the kernels in place.
 plk_status net_ensure(plk_mlp* m, int batch, bool train) {
     const int rows = (batch + kGM - 1) / kGM * kGM;
     const size_t xb = (size_t)batch * m->dims.front() * sizeof(float), tb = (size_t)batch * m->dims.back() * sizeof(float);
@@ -1006,7 +1005,7 @@ plk_status net_ensure(plk_mlp* m, int batch, bool train) {
 }
 
 // One pass over `batch` rows: forward (t null), gradients, or an Adam step.
-// The loss is in the pinned block once the stream has drained (net_loss).
+// The loss is in the pinned block once the stream has drained (net_finish).
 plk_status net_pass(plk_mlp* m, int batch, const float* x, const float* t, bool adam, float lr, float* y_dev) {
     plk_status s = net_ensure(m, batch, t != nullptr);
     if (s != PLK_OK) return s;
@@ -1034,6 +1033,10 @@ plk_status net_pass(plk_mlp* m, int batch, const float* x, const float* t, bool 
     n.loss_part = m->loss_part;
     n.loss = reinterpret_cast<float*>(m->host_dev);
     n.fail = m->fail;
+    n.gave_up = reinterpret_cast<int*>(m->host_dev) + 1;
+    reinterpret_cast<int*>(m->host)[1] = reinterpret_cast<int*>(m->host)[2] = 0;
+    n.withhold = m->withhold;
+    m->withhold = 0;
     n.p = m->p; n.g = m->g; n.m = m->m; n.v = m->v;
     int tiles = 0;
     for (int l = 0; l < L; ++l) {
@@ -1063,12 +1066,22 @@ plk_status net_pass(plk_mlp* m, int batch, const float* x, const float* t, bool 
     return PLK_OK;
 }
 
-// The last pass's loss; a pass that gave up (NaN) leaves its flag cleared for
-// the next one.
-float net_loss(plk_mlp* m) {
-    const float v = *reinterpret_cast<const float*>(m->host);
-    if (std::isnan(v)) cudaMemsetAsync(m->fail, 0, sizeof(int), m->stream);
-    return v;
+// Waits for the last pass (`trained`: one with an Adam step) and gives its loss,
+// or PLK_ERR_TIMEOUT where a kernel gave up, with the flag cleared for the next.
+plk_status net_finish(plk_mlp* m, bool trained, const char* what, float* loss) {
+    if (loss) *loss = NAN;
+    PLK_MCUDA(m, cudaStreamSynchronize(m->stream), what);
+    const volatile int* gave_up = reinterpret_cast<const volatile int*>(m->host) + 1;
+    if (gave_up[0]) {
+        if (trained) --m->step;  // no update was made
+        PLK_MCUDA(m, cudaMemsetAsync(m->fail, 0, sizeof(int), m->stream), "clear flag");
+        return mfail(m, PLK_ERR_TIMEOUT, std::string(what) + ": a bounded wait of the row kernel ran out");
+    }
+    if (gave_up[1])
+        return mfail(m, PLK_ERR_TIMEOUT, std::string(what) + ": a bounded wait of the update kernel ran out" +
+                                             (trained ? "; only a part of the weights was updated" : ""));
+    if (loss) *loss = *reinterpret_cast<const volatile float*>(m->host);
+    return PLK_OK;
 }
 
 plk_status refresh_bf16(plk_mlp* m) {
@@ -1279,8 +1292,8 @@ plk_status plk_mlp_forward(plk_mlp* m, int batch, const float* x, float* y) {
         if ((s = net_pass(m, batch, x, nullptr, false, 0.0f, m->y_dev)) != PLK_OK) return s;
         PLK_MCUDA(m, cudaMemcpyAsync(y, m->y_dev, (size_t)batch * m->dims.back() * sizeof(float), cudaMemcpyDeviceToHost,
                                      m->stream), "download outputs");
-        PLK_MCUDA(m, cudaStreamSynchronize(m->stream), "forward");
-        return PLK_OK;
+        if ((s = net_finish(m, false, "forward", nullptr)) != PLK_OK) std::fill(y, y + (size_t)batch * m->dims.back(), NAN);
+        return s;
     }
     if ((s = ensure_batch(m, batch)) != PLK_OK) return s;
     PLK_MCUDA(m, cudaMemcpyAsync(m->xin, x, (size_t)batch * m->dims.front() * sizeof(float), cudaMemcpyHostToDevice,
@@ -1302,10 +1315,7 @@ plk_status plk_mlp_gradients(plk_mlp* m, int batch, const float* x, const float*
         if (grad)
             PLK_MCUDA(m, cudaMemcpyAsync(grad, m->g, m->n_params * sizeof(float), cudaMemcpyDeviceToHost, m->stream),
                       "download gradients");
-        PLK_MCUDA(m, cudaStreamSynchronize(m->stream), "gradients");
-        const float v = net_loss(m);
-        if (loss) *loss = v;
-        return PLK_OK;
+        return net_finish(m, false, "gradients", loss);
     }
     if ((s = ensure_batch(m, batch)) != PLK_OK) return s;
     PLK_MCUDA(m, cudaMemcpyAsync(m->xin, x, (size_t)batch * m->dims.front() * sizeof(float), cudaMemcpyHostToDevice,
@@ -1322,15 +1332,20 @@ plk_status plk_mlp_gradients(plk_mlp* m, int batch, const float* x, const float*
     return PLK_OK;
 }
 
+plk_status plk_mlp_test_withhold(plk_mlp* m, int where) {
+    if (!m) return PLK_ERR_ARG;
+    if (!m->narrow || where < 1 || where > 2)
+        return mfail(m, PLK_ERR_ARG, "plk_mlp_test_withhold: 1 or 2, networks up to 256 wide");
+    m->withhold = where;
+    return PLK_OK;
+}
+
 plk_status plk_mlp_train_step(plk_mlp* m, int batch, const float* x, const float* t, float lr, float* loss) {
     plk_status s;
     if (m && m->narrow && batch >= 1 && x && t) {
         PLK_MCUDA(m, cudaSetDevice(m->device), "cudaSetDevice");
         if ((s = net_pass(m, batch, x, t, true, lr, nullptr)) != PLK_OK) return s;
-        PLK_MCUDA(m, cudaStreamSynchronize(m->stream), "train step");
-        const float v = net_loss(m);
-        if (loss) *loss = v;
-        return PLK_OK;
+        return net_finish(m, true, "train step", loss);
     }
     if ((s = plk_mlp_gradients(m, batch, x, t, nullptr, nullptr)) != PLK_OK) return s;
     ++m->step;

@@ -53,6 +53,7 @@ EXPORTS = [
     "plk_parse_alignment", "plk_parse_newick",
     "plk_mlp_create", "plk_mlp_destroy", "plk_mlp_last_error", "plk_mlp_n_params", "plk_mlp_get_params",
     "plk_mlp_set_params", "plk_mlp_forward", "plk_mlp_gradients", "plk_mlp_train_step",
+    "plk_mlp_test_withhold",
     "plk_measure_fp32_peak", "plk_loglik_err", "plk_node_states_err", "plk_batch_device_ms",
 ]
 
@@ -155,6 +156,7 @@ def lib() -> ctypes.CDLL:
     L.plk_mlp_forward.argtypes = [hp, c_int, fp, fp]
     L.plk_mlp_gradients.argtypes = [hp, c_int, fp, fp, fp, fp]
     L.plk_mlp_train_step.argtypes = [hp, c_int, fp, fp, ctypes.c_float, fp]
+    L.plk_mlp_test_withhold.argtypes = [hp, c_int]
     no_status = ("plk_destroy", "plk_last_error", "plk_status_string", "plk_batch_destroy", "plk_batch_last_error",
                  "plk_mlp_destroy", "plk_mlp_last_error")
     for name in EXPORTS:
@@ -746,6 +748,11 @@ class MLP:
         self._check(lib().plk_mlp_gradients(self._m, xa.shape[0], _p(xa, ctypes.c_float), _p(ta, ctypes.c_float),
                                             _p(g, ctypes.c_float), ctypes.byref(loss)))
         return g, float(loss.value)
+
+    def test_withhold(self, where: int) -> None:
+        """Test of the failure path: a bounded wait of the next pass's row kernel
+        (1) or update kernel (2) runs out (see plk_mlp_test_withhold)."""
+        self._check(lib().plk_mlp_test_withhold(self._m, int(where)))
 
     def train_step(self, x, t, lr: float) -> float:
         xa = np.ascontiguousarray(x, dtype=np.float32).reshape(-1, self.n_in)
