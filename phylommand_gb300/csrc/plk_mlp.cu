@@ -915,9 +915,11 @@ plk_status mfail(plk_mlp* m, plk_status s, const std::string& msg) {
 #define PLK_MCUDA(m, expr, what)                                                                        \
     do {                                                                                                \
         cudaError_t _e = (expr);                                                                        \
-        if (_e != cudaSuccess)                                                                          \
+        if (_e != cudaSuccess) {                                                                        \
+            cudaGetLastError(); /* reported here, not by the next launch */                             \
             return mfail(m, _e == cudaErrorMemoryAllocation ? PLK_ERR_ALLOC : PLK_ERR_CUDA,              \
                          std::string(what) + ": " + cudaGetErrorString(_e));                            \
+        }                                                                                               \
     } while (0)
 
 int n_layers(const plk_mlp* m) { return (int)m->dims.size() - 1; }
@@ -993,14 +995,25 @@ plk_status net_ensure(plk_mlp* m, int batch, bool train) {
         PLK_MCUDA(m, cudaMalloc(&m->tin, (size_t)rows * m->dims.back() * sizeof(float)), "allocate targets");
         m->n_cap = rows;
     }
-    if (train && m->n_act.empty())
-        for (int l = 0; l < n_layers(m); ++l) {
-            __nv_bfloat16* q = nullptr;
-            PLK_MCUDA(m, cudaMalloc(&q, (size_t)m->n_cap * m->pdims[l] * sizeof(__nv_bfloat16)), "allocate activations");
-            m->n_act.push_back(q);
-            PLK_MCUDA(m, cudaMalloc(&q, (size_t)m->n_cap * m->pdims[l + 1] * sizeof(__nv_bfloat16)), "allocate gradients");
-            m->n_dz.push_back(q);
+    if (train && m->n_act.empty()) {
+        // all of them or none: a later pass takes what is there for whole, and a
+        // smaller batch may fit where this one did not
+        m->n_act.assign(n_layers(m), nullptr);
+        m->n_dz.assign(n_layers(m), nullptr);
+        cudaError_t e = cudaSuccess;
+        for (int l = 0; e == cudaSuccess && l < n_layers(m); ++l) {
+            e = cudaMalloc(&m->n_act[l], (size_t)m->n_cap * m->pdims[l] * sizeof(__nv_bfloat16));
+            if (e == cudaSuccess) e = cudaMalloc(&m->n_dz[l], (size_t)m->n_cap * m->pdims[l + 1] * sizeof(__nv_bfloat16));
         }
+        if (e != cudaSuccess) {
+            for (auto* v : {&m->n_act, &m->n_dz}) {
+                for (auto* q : *v) cudaFree(q);
+                v->clear();
+            }
+            m->n_cap = 0;
+            PLK_MCUDA(m, e, "allocate activations and gradients");
+        }
+    }
     return PLK_OK;
 }
 

@@ -54,3 +54,16 @@ def test_an_update_kernel_that_gives_up():
         np.testing.assert_array_equal(got[w].reshape(64, 256)[:, 224:], p[w].reshape(64, 256)[:, 224:])
         np.testing.assert_array_equal(got[:w.start], ref.get_params()[:w.start])
         assert np.isfinite(net.train_step(x, t, 1e-3))
+
+
+def test_a_batch_that_does_not_fit_leaves_the_network_usable():
+    # 2^26 rows: 34 GB a hidden layer, twice, so an allocation in the middle fails
+    rows = 1 << 26
+    big = np.zeros((rows, 1), dtype=np.float32)
+    x, t = _case(1, 1, 40)
+    with plk.MLP(1, 1, 256, 7, seed=1) as net, plk.MLP(1, 1, 256, 7, seed=1) as ref:
+        for _ in range(2):
+            with pytest.raises(plk.PlkError) as err:
+                net.gradients(big, big)
+            assert err.value.status == plk.PLK_ERR_ALLOC
+        np.testing.assert_array_equal(net.gradients(x, t)[0], ref.gradients(x, t)[0])
