@@ -290,6 +290,7 @@ constexpr int kNetWide = 256;   // widest layer (padded to 16)
 constexpr int kNetLayers = 8;   // weight layers
 constexpr int kNetThreads = 256;
 constexpr int kNetCtas = 4;     // of a row block's cluster
+constexpr uint32_t kNetToken = 16;  // bytes a CTA without columns sends
 constexpr int kUpN = 32, kUpK = 256;  // update tile: inputs, batch rows per pass
 
 struct NetLayer {
@@ -439,6 +440,7 @@ __global__ void __cluster_dims__(kNetCtas, 1, 1) __launch_bounds__(kNetThreads, 
     __shared__ uint32_t s_tmem;
     __shared__ float s_red[kNetThreads];
     __shared__ __align__(16) float s_bias[kNetLayers][net_share(kNetWide)];
+    __shared__ __align__(16) unsigned char s_token[kNetToken];  // its contents mean nothing
     __shared__ uint32_t s_pos[kNetLayers][kNetThreads];  // ReLU: the positive ones of a thread's 32 columns
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = blockIdx.x % kNetCtas, row0 = blockIdx.x / kNetCtas * kGM;
@@ -622,20 +624,24 @@ __global__ void __cluster_dims__(kNetCtas, 1, 1) __launch_bounds__(kNetThreads, 
                 g[1] = o1;
             }
         }
-        // the slice to the other CTAs; theirs arrive on this one's barrier.  A
-        // buffer is free by then: a CTA reaches this point only with the slices
-        // that every other CTA sent after its products of the step before.
+        // the slice to the other CTAs, or a token from one without columns; theirs
+        // arrive on this one's barrier.  So a CTA reaches this point only when
+        // every other one has been here in the step before: their products that
+        // read the buffer are done, and their barrier, which serves every other
+        // step, is in this step's phase.  (Remote arrivals instead of tokens cost
+        // 5 % of a training step: three more cluster operations a layer.)
         asm volatile("fence.proxy.async;\n" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
         __syncthreads();
         if (tid == 0 && st + 1 < steps) {
-            const int own = max(0, min(share, N - n0));
-            const uint32_t b = bar + 24 + 8 * ((st + 1) & 1), bytes = (uint32_t)own * kGM * 2;
-            const uint32_t at = a_sm + ((st + 1) & 1) * kRowsA + (uint32_t)(n0 / 8 * kGM) * 16;
+            const int own = max(0, min(share, N - n0)), idle = kNetCtas - (N + share - 1) / share;  // CTAs without columns
+            const uint32_t b = bar + 24 + 8 * ((st + 1) & 1), bytes = own > 0 ? (uint32_t)own * kGM * 2 : kNetToken;
+            const uint32_t at = own > 0 ? a_sm + ((st + 1) & 1) * kRowsA + (uint32_t)(n0 / 8 * kGM) * 16
+                                        : static_cast<uint32_t>(__cvta_generic_to_shared(s_token));
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(b),
-                         "r"((uint32_t)(N - own) * kGM * 2)
+                         "r"((uint32_t)(N - own) * kGM * 2 + (idle - (own > 0 ? 0 : 1)) * kNetToken)
                          : "memory");
-            for (int d = 1; d < kNetCtas && own > 0; ++d) {
+            for (int d = 1; d < kNetCtas; ++d) {
                 const int cta = (rank + d) % kNetCtas;
                 uint32_t to, tb;
                 asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(to) : "r"(at), "r"(cta));
