@@ -160,15 +160,13 @@ __global__ void __maxnreg__(prune4w_maxnreg(KP, SPT, TPS, TS)) prune4w_kernel(Pr
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     // TS = 1: the tables have landed (a bounded wait; one that runs out
-    // leaves this thread's sum NaN, so the evaluation reports a non-finite
+    // leaves this warp's sums NaN, so the evaluation reports a non-finite
     // value, after a second bounded wait for copies still in flight)
     bool tables_ok = true;
     if constexpr (TS == 1) {
         const uint32_t bar = static_cast<uint32_t>(__cvta_generic_to_shared(&s_bar));
-        if (!mbar_try_wait_bounded(bar, 0)) {
-            tables_ok = false;
-            if (!a.withhold_first_stage) mbar_try_wait_bounded(bar, 0);
-        }
+        tables_ok = __all_sync(0xffffffffu, mbar_try_wait_bounded(bar, 0));
+        if (!tables_ok && !a.withhold_first_stage) mbar_try_wait_bounded(bar, 0);
     }
     // this warp's stack: its lanes, its column range
     const uint32_t tstack =
@@ -212,7 +210,7 @@ __global__ void __maxnreg__(prune4w_maxnreg(KP, SPT, TPS, TS)) prune4w_kernel(Pr
         codes.stride = stride;
         walk4w<KP, SPT, TPS>(tab, n_ops, codes, tstack, levels, over, q0, acc, scale_e);
         if constexpr (TS == 2) {
-            if (!tab.ok) {  // a stage did not arrive
+            if (!__all_sync(0xffffffffu, tab.ok)) {  // a stage did not arrive
                 site_sum_add(sum, __int_as_float(0x7fc00000), 0);
                 continue;
             }

@@ -99,7 +99,7 @@ struct RingTables {
     int g;                // the stage being read, -1 before the first
     uint32_t base;        // its slot's address
     uint32_t phases;      // parity of every slot's next fill, kept from tree to tree
-    bool ok;
+    bool ok;              // of this lane; a caller that branches on it votes first
     int drain;            // stages that may be in flight after a wait ran out
 
     __device__ __forceinline__ void issue(int gg) const {  // one thread
@@ -275,7 +275,7 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 // The arrival of a streamed tile's codes: arrive[c] reaching gen (written by a
 // copy after the chunk's copy on the alignment's copy stream).  Every lane
 // reads the flag with acquire semantics, so its code loads that follow see
-// the chunk.  Bounded: false after kArriveLimitNs of waiting.
+// the chunk.  Bounded: false, for the whole warp, where a lane waited kArriveLimitNs.
 constexpr unsigned long long kArriveLimitNs = 2000000000ull;  // 2 s: far above any chunk's copy time
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
     int v;
@@ -287,7 +287,7 @@ __device__ __forceinline__ unsigned long long global_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t));
     return t;
 }
-__device__ __forceinline__ bool wait_arrival(const int* flag, int gen) {
+__device__ __forceinline__ bool lane_arrival(const int* flag, int gen) {
     if (ld_acquire_gpu(flag) == gen) return true;
     const unsigned long long t0 = global_ns();
     for (;;) {
@@ -295,6 +295,9 @@ __device__ __forceinline__ bool wait_arrival(const int* flag, int gen) {
         if (ld_acquire_gpu(flag) == gen) return true;
         if (global_ns() - t0 > kArriveLimitNs) return false;
     }
+}
+__device__ __forceinline__ bool wait_arrival(const int* flag, int gen) {
+    return __all_sync(0xffffffffu, lane_arrival(flag, gen));
 }
 
 // this thread's tip codes (SPT adjacent sites, one load of SPT bytes),
