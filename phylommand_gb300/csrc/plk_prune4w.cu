@@ -28,7 +28,8 @@
 //    a lane of the warp falls below the threshold does the warp take the full
 //    maximum (the same decision and factors);
 //  * a streamed alignment's codes land while the pass runs: a warp waits
-//    (bounded) for its tile's chunk flag before its walk;
+//    (bounded) for its tile's chunk flag before its walk, with TS = 2 the CTA's
+//    warps together before a round of tiles;
 //  * the launch overlaps the P(t) kernel before it (programmatic stream
 //    serialization; griddepcontrol.wait before any read of its tables).
 // The arithmetic is run_tile4p's (plk_prune4p.cuh) in the same order -- every
@@ -179,19 +180,20 @@ __global__ void __maxnreg__(prune4w_maxnreg(KP, SPT, TPS, TS)) prune4w_kernel(Pr
     for (int round = 0; tables_ok && round < rounds; ++round) {
         const int wtile = warp * gridDim.x + blockIdx.x + round * total_warps;
         bool sites = wtile < n_wtiles;
-        if constexpr (TS == 2) {
-            // every slot is free again; the tree's first stages
-            if (round > 0) __syncthreads();
-            if (tid == 0) tab.start();
-        } else if (!sites) {
-            break;
-        }
+        if (TS == 1 && !sites) break;
         if (sites && a.arrive) {  // a streamed alignment: this tile's chunk of codes first (the test hook withholds it)
             const int want = a.withhold_first_stage ? (a.arrive_gen ^ 0x40000000) : a.arrive_gen;
             if (!wait_arrival(a.arrive + (wtile * WS * SPT) / a.chunk_sites, want)) {
                 site_sum_add(sum, __int_as_float(0x7fc00000), 0);  // NaN: the evaluation reports a numeric error
                 sites = false;
             }
+        }
+        if constexpr (TS == 2) {
+            // every slot is free again, and every warp has its tile's codes (a warp
+            // that still waited for them would hold up the ring, whose waits have
+            // a bound of their own): the tree's first stages
+            if (round > 0 || a.arrive) __syncthreads();
+            if (tid == 0) tab.start();
         }
         if (!sites) {
             if constexpr (TS == 2) tab.skip();
