@@ -212,6 +212,10 @@ int plk_prune_variant(const plk_handle* h);
  * evaluation fails with PLK_ERR_NUMERIC, and the handle stays usable.  No
  * effect on the other forms. */
 plk_status plk_test_withhold_stage(plk_handle* h);
+/* The same for the arrivals of a streamed alignment alone: the next FP32
+ * evaluation in a warp-independent form (12-18) waits for an arrival no copy
+ * writes, and gets its tables and stages. */
+plk_status plk_test_withhold_arrival(plk_handle* h);
 /* Per-site log-likelihoods of the last plk_loglik (n_sites doubles). */
 plk_status plk_site_loglik(plk_handle* h, double* out);
 /* Node-state output for every internal node: out[(rank * n_sites + site) *

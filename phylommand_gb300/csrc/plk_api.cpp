@@ -113,6 +113,7 @@ struct plk_handle {
     bool paired_written = false;  // this evaluation's P(t) kernel also wrote prune4p's layouts
     bool stream_written = false;  // or the streamed forms' tables
     bool withhold_stage = false;  // plk_test_withhold_stage: armed for the next FP32 pass
+    bool withhold_arrival = false;  // plk_test_withhold_arrival: likewise
     DevBuf d_mask_raw, d_flag;
     bool have_lnl = false;
     bool lnl_pending = false;
@@ -602,7 +603,8 @@ plk_status run_prune(plk_handle* h, int precision, NodePass* store, cudaEvent_t*
     a.lnl_out = h->d_lnl;
     a.paired_ready = (precision == PLK_FP32S && h->paired_written) ? 1 : 0;
     a.withhold_first_stage = (precision == PLK_FP32S && h->withhold_stage) ? 1 : 0;
-    if (precision == PLK_FP32S) h->withhold_stage = false;
+    a.withhold_arrival = (precision == PLK_FP32S && (h->withhold_stage || h->withhold_arrival)) ? 1 : 0;
+    if (precision == PLK_FP32S) h->withhold_stage = h->withhold_arrival = false;
     a.use_any = any_blocks > 0 ? 1 : 0;
     const bool fused = fused_kernel_applies(h, precision);
     std::vector<int> cands20;
@@ -1189,6 +1191,12 @@ int plk_prune_variant(const plk_handle* h) { return h ? h->variant : -1; }
 plk_status plk_test_withhold_stage(plk_handle* h) {
     if (!h) return PLK_ERR_ARG;
     h->withhold_stage = true;
+    return PLK_OK;
+}
+
+plk_status plk_test_withhold_arrival(plk_handle* h) {
+    if (!h) return PLK_ERR_ARG;
+    h->withhold_arrival = true;
     return PLK_OK;
 }
 

@@ -293,6 +293,7 @@ struct PruneArgs {
     // never stages its first op, the shared-table form never copies its
     // tables, the streamed form no stage, so their bounded waits run out
     int withhold_first_stage;
+    int withhold_arrival;  // and the warp-independent forms wait for an arrival no copy writes
     // the streamed forms (stream_program): the tables, and whether the P(t)
     // kernel has written them
     const Op* sops;

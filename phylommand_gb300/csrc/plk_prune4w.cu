@@ -182,7 +182,7 @@ __global__ void __maxnreg__(prune4w_maxnreg(KP, SPT, TPS, TS)) prune4w_kernel(Pr
         bool sites = wtile < n_wtiles;
         if (TS == 1 && !sites) break;
         if (sites && a.arrive) {  // a streamed alignment: this tile's chunk of codes first (the test hook withholds it)
-            const int want = a.withhold_first_stage ? (a.arrive_gen ^ 0x40000000) : a.arrive_gen;
+            const int want = a.withhold_arrival ? (a.arrive_gen ^ 0x40000000) : a.arrive_gen;
             if (!wait_arrival(a.arrive + (wtile * WS * SPT) / a.chunk_sites, want)) {
                 site_sum_add(sum, __int_as_float(0x7fc00000), 0);  // NaN: the evaluation reports a numeric error
                 sites = false;
