@@ -307,7 +307,9 @@ plk_status plk_batch_form(const plk_batch* b, int* paired, int* codes_smem);
  *   1  swap left(v)  with v's sibling          (parent of v not the root)
  *   2  swap right(v) with left(c)              (v, c the root's children)
  *   3  swap right(v) with right(c)
- * plk_batch_nni_loglik writes, item after item, the lnL of every move. */
+ * plk_batch_nni_loglik writes, item after item, the lnL of every move: -inf
+ * where a site's likelihood is zero under it, NaN where one is not a positive
+ * number (the call itself succeeds; the other moves are not affected). */
 /* Summary statistics of every item (the warm-start network's inputs), 43
  * floats per item: base frequencies (4), mean pairwise proportions of the
  * substitution types A<->G, A<->C, A<->T, G<->C, G<->T, C<->T (6), histogram of

@@ -389,7 +389,11 @@ __global__ void __maxnreg__(kDownRegs) batch_down_kernel(BatchDev b, BlenDev bd,
                 if constexpr (MODE == kNni) {
                     const float2 v = reinterpret_cast<const float2*>(vals)[s * (W + 1) + c];
                     const int bits = __float_as_int(v.x);
-                    const float lm = logf(__int_as_float((bits & 0x007fffff) | 0x3f800000));
+                    // zero, a negative one (rounding noise of P(0)), infinity and NaN keep
+                    // logf's own result (-inf, NaN, inf, NaN), as in site_log32
+                    const float lm = v.x > 0.0f && v.x <= 3.40282347e38f
+                                         ? logf(__int_as_float((bits & 0x007fffff) | 0x3f800000))
+                                         : logf(v.x);
                     float ns, er;
                     two_sum_f(h1, lm, ns, er);
                     h1 = ns;
@@ -660,7 +664,9 @@ __global__ void __launch_bounds__(32 * kFoldWarps) batch_down_reduce_kernel(Batc
         else add(h2, l2, v.z, v.w);
     }
     if constexpr (MODE == kNni) {
-        b.nni_out[it.move_out_off + m] = fma((double)e, 0.69314718055994530942, (double)h1 + (double)l1);
+        // an infinite sum is what it is (its low part is not a number)
+        b.nni_out[it.move_out_off + m] =
+            isinf(h1) ? (double)h1 : fma((double)e, 0.69314718055994530942, (double)h1 + (double)l1);
     } else {
         const int g = bd.item_edge_off[blk.x] + m;
         bd.edge_out[2 * g] = (double)h1 + (double)l1;
