@@ -620,6 +620,22 @@ __global__ void __maxnreg__(kDownRegs) batch_down_kernel(BatchDev b, BlenDev bd,
     }
 }
 
+// A running sum of FP32 pairs in three parts, h + l + ll: the rounding errors of
+// h and of l are kept, so it is no less exact than FP64 sums (whose adds would
+// cost the derivatives' batch 2 % on GB300's FP64 pipe); in two parts a sum of
+// 3,000 tiles was off by 1e-14 of its terms.
+struct Sum3 {
+    float h = 0.0f, l = 0.0f, ll = 0.0f;
+    __device__ __forceinline__ void add(float oh, float ol, float oll) {
+        float e, e1, e2;
+        two_sum_f(h, oh, h, e);
+        two_sum_f(l, ol, l, e1);
+        two_sum_f(l, e, l, e2);
+        ll = __fadd_rn(ll, __fadd_rn(__fadd_rn(e1, e2), oll));
+    }
+    __device__ __forceinline__ double value() const { return (double)h + ((double)l + (double)ll); }
+};
+
 constexpr int kFoldWarps = 32;
 // One CTA per (item, 32 outputs): its warps fold the records of the item's
 // warp tiles, each every 32nd tile in order, a lane per output; then the
@@ -628,49 +644,64 @@ constexpr int kFoldWarps = 32;
 // batch from 83 us (eight warps) to 30 us.
 template <int MODE>
 __global__ void __launch_bounds__(32 * kFoldWarps) batch_down_reduce_kernel(BatchDev b, BlenDev bd, int W) {
-    __shared__ float4 part[kFoldWarps][32];
     const int2 blk = b.reduce_blocks[blockIdx.x];
     const BatchItemDev it = b.items[blk.x];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n_out = MODE == kNni ? it.n_moves : 2 * it.n_int, m = blk.y + lane;
     const int tiles = (it.n_sites + W - 1) / W;
     const float4* rec = b.records + b.rec_off[blk.x] + m;
-    float h1 = 0.0f, l1 = 0.0f, h2 = 0.0f, l2 = 0.0f;
-    long long e = 0;
-    auto add = [](float& h, float& l, float oh, float ol) {
-        float ns, er;
-        two_sum_f(h, oh, ns, er);
-        h = ns;
-        l = __fadd_rn(l, __fadd_rn(ol, er));
-    };
-    if (m < n_out) {
+    if constexpr (MODE == kBlen) {
+        __shared__ Sum3 part[2][kFoldWarps][32];
+        Sum3 d1, d2;
+        if (m < n_out) {
 #pragma unroll 4
-        for (int t = warp; t < tiles; t += kFoldWarps) {
-            const float4 v = rec[(size_t)t * n_out];
-            add(h1, l1, v.x, v.y);
-            if constexpr (MODE == kNni) e += __float_as_int(v.z);
-            else add(h2, l2, v.z, v.w);
+            for (int t = warp; t < tiles; t += kFoldWarps) {
+                const float4 v = rec[(size_t)t * n_out];
+                d1.add(v.x, v.y, 0.0f);
+                d2.add(v.z, v.w, 0.0f);
+            }
         }
-    }
-    __shared__ long long part_e[kFoldWarps][32];
-    part[warp][lane] = make_float4(h1, l1, h2, l2);
-    part_e[warp][lane] = e;
-    __syncthreads();
-    if (warp != 0 || m >= n_out) return;
-    for (int w = 1; w < kFoldWarps; ++w) {
-        const float4 v = part[w][lane];
-        add(h1, l1, v.x, v.y);
-        if constexpr (MODE == kNni) e += part_e[w][lane];
-        else add(h2, l2, v.z, v.w);
-    }
-    if constexpr (MODE == kNni) {
-        // an infinite sum is what it is (its low part is not a number)
-        b.nni_out[it.move_out_off + m] =
-            isinf(h1) ? (double)h1 : fma((double)e, 0.69314718055994530942, (double)h1 + (double)l1);
-    } else {
+        part[0][warp][lane] = d1;
+        part[1][warp][lane] = d2;
+        __syncthreads();
+        if (warp != 0 || m >= n_out) return;
+        for (int w = 1; w < kFoldWarps; ++w) {
+            const Sum3 a = part[0][w][lane], c = part[1][w][lane];
+            d1.add(a.h, a.l, a.ll);
+            d2.add(c.h, c.l, c.ll);
+        }
         const int g = bd.item_edge_off[blk.x] + m;
-        bd.edge_out[2 * g] = (double)h1 + (double)l1;
-        bd.edge_out[2 * g + 1] = (double)h2 + (double)l2;
+        bd.edge_out[2 * g] = d1.value();
+        bd.edge_out[2 * g + 1] = d2.value();
+    } else {
+        __shared__ float2 part[kFoldWarps][32];
+        __shared__ long long part_e[kFoldWarps][32];
+        float h = 0.0f, l = 0.0f;
+        long long e = 0;
+        auto add = [&](float oh, float ol) {
+            float ns, er;
+            two_sum_f(h, oh, ns, er);
+            h = ns;
+            l = __fadd_rn(l, __fadd_rn(ol, er));
+        };
+        if (m < n_out) {
+#pragma unroll 4
+            for (int t = warp; t < tiles; t += kFoldWarps) {
+                const float4 v = rec[(size_t)t * n_out];
+                add(v.x, v.y);
+                e += __float_as_int(v.z);
+            }
+        }
+        part[warp][lane] = make_float2(h, l);
+        part_e[warp][lane] = e;
+        __syncthreads();
+        if (warp != 0 || m >= n_out) return;
+        for (int w = 1; w < kFoldWarps; ++w) {
+            add(part[w][lane].x, part[w][lane].y);
+            e += part_e[w][lane];
+        }
+        // an infinite sum is what it is (its low part is not a number)
+        b.nni_out[it.move_out_off + m] = isinf(h) ? (double)h : fma((double)e, 0.69314718055994530942, (double)h + (double)l);
     }
 }
 
