@@ -227,30 +227,31 @@ __device__ inline void finish_grid_sum32(const double* bs, unsigned* counter, do
 // Sum of FP64 site log-likelihoods in integers.  A warp-wide FP64 instruction
 // occupies GB300's FP64 pipe for 16 cycles of its SM and a chain of TwoSum
 // shuffle steps waits on each, which put about 13 us at the end of a short
-// pass; integer adds do not.  A value x is split exactly into hi 2^-20 + lo
-// 2^-60 (hi, lo 64-bit; nothing of x is lost while |x| >= 2^-8, and 2^-61 at
+// pass; integer adds do not.  A value x is split exactly into hi 2^-26 + lo
+// 2^-78 (hi, lo 64-bit; nothing of x is lost while |x| >= 2^-26, and 2^-79 at
 // most below), the parts are summed as integers, so the total is exact until
 // its one rounding at the end and does not depend on the order.  A value that
-// is not finite, or 2^40 and more, makes the sum NaN.
+// is not finite, or 2^36 and more (a site's exponent is an int: it stays below
+// 2^31), makes the sum NaN; the total may reach 2^37.
 struct SiteSum64 {
     long long hi = 0, lo = 0;
     int bad = 0;
 };
 
 __device__ __forceinline__ void site_sum64_add(SiteSum64& a, double x) {
-    if (!(fabs(x) < 1099511627776.0)) {
+    if (!(fabs(x) < 68719476736.0)) {
         a.bad = 1;
         return;
     }
-    const long long h = __double2ll_rn(x * 1048576.0);
+    const long long h = __double2ll_rn(x * 67108864.0);
     a.hi += h;
-    a.lo += __double2ll_rn(fma((double)h, -9.5367431640625e-07, x) * 1152921504606846976.0);
+    a.lo += __double2ll_rn(fma((double)h, -1.4901161193847656e-08, x) * 3.0223145490365729e23);
 }
 
-// carries lo beyond 40 bits into hi, leaving 0 <= lo < 2^40
+// carries lo beyond 52 bits into hi, leaving 0 <= lo < 2^52
 __device__ __forceinline__ void site_sum64_carry(SiteSum64& a) {
-    a.hi += a.lo >> 40;
-    a.lo &= (1ll << 40) - 1;
+    a.hi += a.lo >> 52;
+    a.lo &= (1ll << 52) - 1;
 }
 
 __device__ __forceinline__ void warp_sum_site64(SiteSum64& a) {
@@ -319,9 +320,9 @@ __device__ inline void finish_grid_sum64(const double* bs, unsigned* counter, do
         site_sum64_carry(t);
         // hi may need more than 53 bits: its rounding error goes with lo
         const double h = (double)t.hi;
-        const double rest = (double)(t.hi - (long long)h) * 9.5367431640625e-07 +
-                            (double)t.lo * 8.6736173798840355e-19;
-        *out = t.bad ? __longlong_as_double(0x7ff8000000000000ll) : h * 9.5367431640625e-07 + rest;
+        const double rest = (double)(t.hi - (long long)h) * 1.4901161193847656e-08 +
+                            (double)t.lo * 3.3087224502121107e-24;
+        *out = t.bad ? __longlong_as_double(0x7ff8000000000000ll) : h * 1.4901161193847656e-08 + rest;
         *counter = 0u;
     }
 }
