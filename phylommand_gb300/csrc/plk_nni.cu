@@ -620,22 +620,6 @@ __global__ void __maxnreg__(kDownRegs) batch_down_kernel(BatchDev b, BlenDev bd,
     }
 }
 
-// A running sum of FP32 pairs in three parts, h + l + ll: the rounding errors of
-// h and of l are kept, so it is no less exact than FP64 sums (whose adds would
-// cost the derivatives' batch 2 % on GB300's FP64 pipe); in two parts a sum of
-// 3,000 tiles was off by 1e-14 of its terms.
-struct Sum3 {
-    float h = 0.0f, l = 0.0f, ll = 0.0f;
-    __device__ __forceinline__ void add(float oh, float ol, float oll) {
-        float e, e1, e2;
-        two_sum_f(h, oh, h, e);
-        two_sum_f(l, ol, l, e1);
-        two_sum_f(l, e, l, e2);
-        ll = __fadd_rn(ll, __fadd_rn(__fadd_rn(e1, e2), oll));
-    }
-    __device__ __forceinline__ double value() const { return (double)h + ((double)l + (double)ll); }
-};
-
 constexpr int kFoldWarps = 32;
 // One CTA per (item, 32 outputs): its warps fold the records of the item's
 // warp tiles, each every 32nd tile in order, a lane per output; then the

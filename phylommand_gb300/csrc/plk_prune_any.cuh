@@ -68,7 +68,7 @@ struct AnyShape {
 // [warps] pairs of vectors and sums of the node output (node_out) | ops or node
 // table | tip codes [tip][sites of the CTA].
 inline size_t any_node_bytes(int S, int C, int H, bool fp64) {  // of a warp
-    return (size_t)(32 / H) * S * (fp64 ? 16 : 8) + (size_t)(32 / (C * H)) * (S + 1) * 8;
+    return (size_t)(32 / H) * S * (fp64 ? 16 : 8) + (size_t)(32 / (C * H)) * (S + 2) * 8;
 }
 inline size_t any_base_smem(int S, int H, bool fp64, const AnyLaunch& p, int C, int n_nodes, int n_tips, int n_codes) {
     const int V = fp64 ? (S % 2 == 0 ? 2 : 1) : (S % 4 == 0 ? 4 : (S % 2 == 0 ? 2 : 1));
@@ -141,9 +141,14 @@ struct NodeWeights {
 // out in order.  In FP64 the sum, the total and the division are FP64, the
 // operations of the reference's order.  In FP32 they would put ten FP64
 // instructions a value on a pipe that takes 16 cycles for each (the larger part
-// of the pass); the same quantities are carried as two FP32 parts (products and
-// sums with their exact rounding errors, Dekker 1971 / Knuth's TwoSum), 2^-45
-// relative, under vectors that are good to 2^-22.
+// of the pass); there the sums over the categories are carried as two FP32 parts
+// (products and sums with their exact rounding errors, Dekker 1971 / Knuth's
+// TwoSum), 2^-47 relative, under vectors that are good to 2^-22.  The total is kept
+// in three parts and the quotient rounded at 2^-50, so that a site's outputs sum
+// to one within 1.3e-15; a quotient in two rough parts left them up to 3e-13 from
+// it.  Conditionals and marginals with their copy, rough and now: 4 states, 100 x
+// 10,000, C = 4, 379 and 490 -> 365 and 492 us (FP64 for total and quotient: 501
+// and 605); 20 states, 40 x 2,000, 192 and 257 -> 216 and 280.
 // Static shared memory of the kernels, which counts towards a CTA's limit: the
 // site sum's words and the last CTA's flag (post-order), the category weights
 // (node states).
@@ -152,7 +157,7 @@ constexpr size_t kSumStatic = 32 * 2 * 8 + 32 * 4 + 16, kWeightStatic = sizeof(N
 template <typename T, int S, int H>
 struct NodeOut {
     T* oc;         // [site * C + k][S][2]
-    double* sums;  // [site][S], then [site]
+    double* sums;  // [site][S], then [site][2]
     const double* w;  // category weights, and as two FP32 parts
     const float2* w2;
 
@@ -209,19 +214,26 @@ struct NodeOut {
             }
             __syncwarp();
             if (lane < W) {
-                float hi = 0.0f, lo = 0.0f;
-                for (int s = 0; s < S; ++s) add2(hi, lo, sum2[lane * S + s].x, sum2[lane * S + s].y);
-                tot[lane] = make_float2(hi, lo);
+                Sum3 t;
+                for (int s = 0; s < S; ++s) t.add(sum2[lane * S + s].x, sum2[lane * S + s].y, 0.0f);
+                tot[2 * lane] = make_float2(t.h, t.l);
+                tot[2 * lane + 1] = make_float2(t.ll, __frcp_rn(t.h));
             }
             __syncwarp();
             for (int i = lane; i < W * S; i += 32) {
-                const float2 m = sum2[i], t = tot[i / S];
-                // a quotient to 2^-22 and the remainder's, whose leading part is exact
-                const float inv = __fdividef(1.0f, t.x);
-                const float q1 = __fmul_rn(m.x, inv);
-                const float r = __fsub_rn(__fadd_rn(fmaf(-q1, t.x, m.x), m.y), __fmul_rn(q1, t.y));
-                const float q2 = __fmul_rn(r, inv);
-                if (site0 + i / S < n_sites) out[(size_t)site0 * S + i] = (double)q1 + (double)q2;
+                // long division: q1, rounded as a division would be, leaves a
+                // remainder that is exact, q2 and q3 one in two parts; then the
+                // quotient's two parts, the first one rounded
+                const float2 m = sum2[i], t = tot[2 * (i / S)], u = tot[2 * (i / S) + 1];
+                const float q0 = __fmul_rn(m.x, u.y), q1 = fmaf(fmaf(-q0, t.x, m.x), u.y, q0), c = __fmul_rn(q1, t.y);
+                float r, e1, e2;
+                two_sum_f(fmaf(-q1, t.x, m.x), m.y, r, e1);
+                two_sum_f(r, -c, r, e2);
+                const float low = __fadd_rn(__fadd_rn(e1, e2), fmaf(-q1, u.x, -fmaf(q1, t.y, -c)));
+                const float q2 = __fmul_rn(r, u.y);
+                const float q3 = __fmul_rn(__fadd_rn(fmaf(-q2, t.x, r), fmaf(-q2, t.y, low)), u.y);
+                const float p1 = __fadd_rn(q1, q2), p2 = __fadd_rn(__fsub_rn(q2, __fsub_rn(p1, q1)), q3);
+                if (site0 + i / S < n_sites) out[(size_t)site0 * S + i] = (double)p1 + (double)p2;
             }
         }
         __syncwarp();  // the next node's values may be put
@@ -262,9 +274,9 @@ __global__ void __launch_bounds__(256) prune_any_kernel(PruneArgs a, AnyLaunch p
         s_w.load(a.cat_w, C);
         node.w = s_w.w;
         node.w2 = s_w.w2;
-        const int per = (32 / H) * S * 2 * (int)sizeof(T) + W * (S + 1) * 8;
+        const int per = (32 / H) * S * 2 * (int)sizeof(T) + W * (S + 2) * 8;
         node.sums = reinterpret_cast<double*>(after + warp * per);
-        node.oc = reinterpret_cast<T*>(after + warp * per + W * (S + 1) * 8);
+        node.oc = reinterpret_cast<T*>(after + warp * per + W * (S + 2) * 8);
         after += (pl.warps * per + 15) / 16 * 16;
     }
     Op* const s_ops = reinterpret_cast<Op*>(after);
@@ -568,10 +580,10 @@ __global__ void __launch_bounds__(256) down_any_kernel(PreorderArgs a, AnyLaunch
     T* const work = reinterpret_cast<T*>(any_smem_raw + (table_elems * sizeof(T) + 15) / 16 * 16);
     T* const xch = work + warp * Sh::kExch;
     unsigned char* after = reinterpret_cast<unsigned char*>(work + pl.warps * Sh::kExch);
-    const int per = (32 / H) * S * 2 * (int)sizeof(T) + W * (S + 1) * 8;
+    const int per = (32 / H) * S * 2 * (int)sizeof(T) + W * (S + 2) * 8;
     __shared__ NodeWeights s_w;
     s_w.load(a.cat_w, C);
-    const NodeOut<T, S, H> node{reinterpret_cast<T*>(after + warp * per + W * (S + 1) * 8),
+    const NodeOut<T, S, H> node{reinterpret_cast<T*>(after + warp * per + W * (S + 2) * 8),
                                 reinterpret_cast<double*>(after + warp * per), s_w.w, s_w.w2};
     int4* const s_kids = reinterpret_cast<int4*>(after + (pl.warps * per + 15) / 16 * 16);  // left, right, id
     uint8_t* const s_codes = reinterpret_cast<uint8_t*>(s_kids + n_int);
