@@ -75,13 +75,19 @@ struct UnitSet {
 
 // Plan of NNI scoring or of the branch-length derivatives (plk_nni.cu) for
 // the current layout: warps per CTA, the units whose item's tables do not fit
-// in shared memory first, the records and the CTAs that fold them.
+// in shared memory first, the records and the CTAs that fold them.  Items whose
+// records together pass kRecordBytes go in several groups, one after another
+// over the same records.
+struct DownGroup {
+    int unit0, unit1, block0, block1;
+};
 struct DownPlan {
     bool ready = false;
     int n_units = 0, n_far = 0;  // units [0, n_far) read their tables through L1
     DownSize size;
-    int grid_far = 0, grid_near = 0, n_blocks = 0, total_out = 0;
-    size_t n_records = 0;
+    int grid_far = 0, grid_near = 0, total_out = 0;
+    size_t n_records = 0;  // of the largest group
+    std::vector<DownGroup> groups;
     std::vector<int> out_off;                   // first output of every item
     BBuf units, rec_off, blocks, d_out_off;
 };
@@ -954,6 +960,9 @@ plk_status plk_batch_nni_moves(const plk_batch* b, int item, int* moves) {
 namespace {
 
 constexpr size_t kSmemLimit = 227 * 1024;
+// A record takes 16 bytes per output and warp tile, up to four times the tip codes
+// of its item: a batch whose codes fit has to fit with them.
+constexpr size_t kRecordBytes = (size_t)8 << 30;
 
 // The trees NNI scoring and the derivatives take: those whose op list and
 // spill stack (of a staged tile of 128 sites) fit in a CTA's shared memory.
@@ -1007,26 +1016,36 @@ plk_status plan_down(plk_batch* b, DownPlan& p, bool blen) {
     std::vector<int2> blocks;
     p.out_off.assign(n_items, 0);
     p.total_out = 0;
-    long long records = 0;
+    auto n_out = [&](int i) { return blen ? 2 * b->items[i].n_int : b->items[i].n_moves(); };
     for (int i = 0; i < n_items; ++i) {
-        const ItemHost& h = b->items[i];
-        const int n_out = blen ? 2 * h.n_int : h.n_moves();
         p.out_off[i] = p.total_out;
-        p.total_out += n_out;
-        rec_off[i] = records;
-        records += (long long)n_out * ((h.n_sites + W - 1) / W);
-        for (int m = 0; m < n_out; m += 32) blocks.push_back(make_int2(i, m));
+        p.total_out += n_out(i);
     }
     p.n_far = 0;
+    p.n_records = 1;
+    p.groups.clear();
+    size_t most = kRecordBytes;
+    if (const char* e = getenv("PLK_BATCH_RECORD_BYTES")) most = (size_t)std::max(0ll, atoll(e));
+    long long records = 0;
     const int tile = z.warps * W;
     for (int k = 0; k < n_items; ++k) {
+        const int i = order[k], n_sites = b->items[i].n_sites;
+        const long long mine = (long long)n_out(i) * ((n_sites + W - 1) / W);
+        if (k == 0 || (size_t)(records + mine) * sizeof(float4) > most) {
+            p.groups.push_back({(int)units.size(), 0, (int)blocks.size(), 0});
+            records = 0;
+        }
+        rec_off[i] = records;
+        records += mine;
+        p.n_records = std::max(p.n_records, (size_t)records);
         if (k == far) p.n_far = (int)units.size();
-        for (int t = 0; t < (b->items[order[k]].n_sites + tile - 1) / tile; ++t) units.push_back(make_int2(order[k], t));
+        for (int t = 0; t < (n_sites + tile - 1) / tile; ++t) units.push_back(make_int2(i, t));
+        for (int m = 0; m < n_out(i); m += 32) blocks.push_back(make_int2(i, m));
+        p.groups.back().unit1 = (int)units.size();
+        p.groups.back().block1 = (int)blocks.size();
     }
     if (far == n_items) p.n_far = (int)units.size();
     p.n_units = (int)units.size();
-    p.n_blocks = (int)blocks.size();
-    p.n_records = (size_t)std::max<long long>(records, 1);
     p.grid_near = std::min(p.n_units - p.n_far, occ * b->n_sms);
     p.grid_far = p.n_far == 0 ? 0 : std::min(p.n_far, std::max(1, down_occupancy(b->C, blen, false, z)) * b->n_sms);
     PLK_BCUDA(b, p.units.ensure(units.size() * sizeof(int2)), "allocate units");
@@ -1075,7 +1094,6 @@ plk_status enqueue_down(plk_batch* b, bool blen) {
     d.kids = b->d_kids.as<int4>();
     d.records = b->d_records.as<float4>();
     d.rec_off = p.rec_off.as<long long>();
-    d.reduce_blocks = p.blocks.as<int2>();
     d.nni_out = b->d_nni_out.as<double>();
     d.scratch_int = b->max_int;
     d.scr = b->d_scr.as<float4>();
@@ -1083,17 +1101,20 @@ plk_status enqueue_down(plk_batch* b, bool blen) {
     PLK_BCUDA(b, cudaMemcpyAsync(b->d_model.p, b->h_model, n_items * batch_model_stride(b->C) * sizeof(double),
                                  cudaMemcpyHostToDevice, b->stream), "upload models");
     PLK_BCUDA(b, launch_down_tables(d, bd, b->stream), "batch tables launch");
-    if (p.grid_far > 0) {
-        PLK_BCUDA(b, cudaMemsetAsync(b->d_counter.p, 0, sizeof(int), b->stream), "clear work queue");
-        PLK_BCUDA(b, launch_down(d, bd, blen, false, p.size, 0, p.n_far, p.grid_far, b->stream),
-                  "pre-order kernel launch");
+    for (const DownGroup& g : p.groups) {
+        // its units that read their tables through L1, then the others
+        const int cut = std::min(std::max(p.n_far, g.unit0), g.unit1);
+        for (const bool near : {false, true}) {
+            const int u0 = near ? cut : g.unit0, u1 = near ? g.unit1 : cut;
+            if (u0 == u1) continue;
+            PLK_BCUDA(b, cudaMemsetAsync(b->d_counter.p, 0, sizeof(int), b->stream), "clear work queue");
+            PLK_BCUDA(b, launch_down(d, bd, blen, near, p.size, u0, u1, std::min(near ? p.grid_near : p.grid_far, u1 - u0),
+                                     b->stream),
+                      "pre-order kernel launch");
+        }
+        d.reduce_blocks = p.blocks.as<int2>() + g.block0;
+        PLK_BCUDA(b, launch_down_reduce(d, bd, blen, g.block1 - g.block0, b->stream), "record fold launch");
     }
-    if (p.grid_near > 0) {
-        PLK_BCUDA(b, cudaMemsetAsync(b->d_counter.p, 0, sizeof(int), b->stream), "clear work queue");
-        PLK_BCUDA(b, launch_down(d, bd, blen, true, p.size, p.n_far, p.n_units, p.grid_near, b->stream),
-                  "pre-order kernel launch");
-    }
-    PLK_BCUDA(b, launch_down_reduce(d, bd, blen, p.n_blocks, b->stream), "record fold launch");
     return PLK_OK;
 }
 
