@@ -528,7 +528,7 @@ def run_protein(args):
              "5": "prune20u_kernel, tcgen05 tensor cores (split TF32, TMEM accumulators)",
              "6": "prune20v_kernel, tcgen05 tensor cores, compact form (three CTAs per SM)",
              "7": "prune20v_kernel, tcgen05 tensor cores, compact form, split BF16 (kind::f16)",
-             "fp64": "prune_generic_kernel, FP64 partials (the plain form)", "auto": "autotuned"}
+             "fp64": "prune_any_kernel, FP64 partials (the plain form)", "auto": "autotuned"}
     profiles = {"1": "prune20_kernel_protein_64x20k", "3": "prune20_kernel_protein_64x20k",
                 "5": "prune20u_kernel_protein_64x20k", "6": "prune20v_kernel_protein_64x20k",
                 "7": "prune20v_bf16_kernel_protein_64x20k"}

@@ -109,7 +109,7 @@ struct plk_handle {
     DevBuf d_P64, d_P32, d_tip64, d_tip32;
     // results and scratch
     DevBuf d_site_lnl, d_block, d_work, d_cond, d_outside, d_nodes_out;
-    DevBuf d_done;  // arrival counters (finish_grid_sum, then one per 128-site tile), zero between launches
+    DevBuf d_done;  // arrival counters (finish_grid_sum32 / 64, then one per 128-site tile), zero between launches
     bool paired_written = false;  // this evaluation's P(t) kernel also wrote prune4p's layouts
     bool stream_written = false;  // or the streamed forms' tables
     bool withhold_stage = false;  // plk_test_withhold_stage: armed for the next FP32 pass

@@ -625,7 +625,8 @@ constexpr int kFoldWarps = 32;
 // warp tiles, each every 32nd tile in order, a lane per output; then the
 // warps' sums in order.  Latency bound (a 50,000-site item has 3,125 tiles):
 // 32 warps with four loads in flight took the fold of the 24-item derivative
-// batch from 83 us (eight warps) to 30 us.
+// batch from 83 us (eight warps) to 30 us; with the third part of the
+// derivatives' sums it issues for 48 us.
 template <int MODE>
 __global__ void __launch_bounds__(32 * kFoldWarps) batch_down_reduce_kernel(BatchDev b, BlenDev bd, int W) {
     const int2 blk = b.reduce_blocks[blockIdx.x];

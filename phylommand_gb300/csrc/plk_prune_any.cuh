@@ -28,7 +28,7 @@
 // Operation order per value is prune_generic_kernel's, so are the bits.
 // Measured, pass alone, before (prune_generic_kernel / prune4_kernel) and here:
 // 20 states FP64 C = 4, 40 x 1,501: 6,540 -> 451 us; 5 states FP32 C = 4,
-// 77 x 5,000: 681 -> 33 us; 4 states FP64 C = 1, 103 x 694: 212 -> 63 us.
+// 77 x 5,000: 681 -> 37 us; 4 states FP64 C = 1, 103 x 694: 212 -> 65 us.
 #pragma once
 
 #include <type_traits>
