@@ -4,7 +4,7 @@
 //                             (src/sub_model.cpp:3-29, 99-114; get_freq :44-53)
 //  * pmat_taylor20_host     — marth::square_matrix::exponential(P, t, 20)
 //                             (src/marth/marth.cpp:129-140, multiply :50-61)
-//  * symmetric_eigen / reversible_eigen / pmat_series_host — exact exp(Qt),
+//  * jacobi_eigen / tridiagonal_eigen / reversible_eigen / pmat_series_host — exact exp(Qt),
 //                             which the reference lacks (cyclic Jacobi; tridiagonal QR,
 //                             Golub & Van Loan 4th ed. section 8.5; scaling and
 //                             squaring with a Taylor sum)
@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <numeric>
 
 #include "plk_internal.h"
 
@@ -228,11 +229,35 @@ static bool tridiagonal_eigen(int n, const double* Ain, double* w, double* V) {
     return true;
 }
 
-void symmetric_eigen(int n, const double* A, double* w, double* V) {
-    // up to 4 states the sweeps take a microsecond either way, with the smaller
-    // error (1.1e-15 against 3.6e-15 of |Q| = 1); above, the sweeps' n^3 counts:
-    // 20 states 77 -> 22 us
-    if (n < 5 || !tridiagonal_eigen(n, A, w, V)) jacobi_eigen(n, A, w, V);
+// Whether the tridiagonal method is as exact as the sweeps for B = D^1/2 Q D^-1/2.
+// Its vectors are exact to a rounding of their length, the sweeps' nearly to one
+// of each entry, and P(t) divides an entry by the square root of its state's
+// frequency.  So states that hang together by nothing (their P(t) is exactly zero
+// with the sweeps, rounding noise of either sign without) or weakly, and
+// frequencies far apart keep the sweeps.  20 states, the largest error of an
+// entry of P(0.001), sweeps and tridiagonal: frequencies over two decades 5.9e-15
+// and 3.4e-15, over six 8.0e-15 and 5.6e-14 (relative 2.5e-10 and 2.7e-7).
+static bool tridiagonal_suits(int n, const double* B, const double* pi) {
+    // up to 6 states the sweeps take 2 us more; above, their n^3 counts: 20
+    // states 77 -> 22 us
+    if (n <= 6 || !(*std::max_element(pi, pi + n) <= 100.0 * *std::min_element(pi, pi + n))) return false;
+    double top = 0.0;
+    for (int i = 0; i < n; ++i)
+        for (int j = 0; j < i; ++j) top = std::max(top, std::fabs(B[i * n + j]));
+    std::vector<int> seen(n, 0), todo(1, 0);  // states reached over entries of 1 % of the largest
+    seen[0] = 1;
+    int reached = 0;
+    while (!todo.empty()) {
+        const int i = todo.back();
+        todo.pop_back();
+        ++reached;
+        for (int j = 0; j < n; ++j)
+            if (!seen[j] && std::fabs(B[i * n + j]) >= 0.01 * top && top > 0.0) {
+                seen[j] = 1;
+                todo.push_back(j);
+            }
+    }
+    return reached == n;
 }
 
 bool reversible_eigen(int n, const double* Q, const double* pi, double* lam, double* L,
@@ -249,7 +274,19 @@ bool reversible_eigen(int n, const double* Q, const double* pi, double* lam, dou
             const double bji = sq[j] * Q[j * n + i] / sq[i];
             B[i * n + j] = 0.5 * (bij + bji);
         }
-    symmetric_eigen(n, B.data(), lam, V.data());
+    bool done = false;
+    if (tridiagonal_suits(n, B.data(), pi)) {
+        // common states first: the reduction then mixes least into the rare ones
+        std::vector<int> at(n);
+        std::iota(at.begin(), at.end(), 0);
+        std::stable_sort(at.begin(), at.end(), [&](int x, int y) { return pi[x] > pi[y]; });
+        std::vector<double> A((size_t)n * n), U((size_t)n * n);
+        for (int i = 0; i < n; ++i)
+            for (int j = 0; j < n; ++j) A[i * n + j] = B[at[i] * n + at[j]];
+        done = tridiagonal_eigen(n, A.data(), lam, U.data());
+        for (int i = 0; i < n && done; ++i) std::copy(&U[i * n], &U[i * n] + n, &V[at[i] * n]);
+    }
+    if (!done) jacobi_eigen(n, B.data(), lam, V.data());
     for (int i = 0; i < n; ++i)
         for (int m = 0; m < n; ++m) {
             L[i * n + m] = V[i * n + m] / sq[i];

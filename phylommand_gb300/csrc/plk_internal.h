@@ -67,8 +67,6 @@ void q_matrix(int n, bool tr, const unsigned* spec, const double* rates, const d
               double* Q);
 // Symmetric eigendecomposition by cyclic Jacobi rotations: A = V diag(w) V^T.
 void jacobi_eigen(int n, const double* A, double* w, double* V);
-// The same by the method that suits n.
-void symmetric_eigen(int n, const double* A, double* w, double* V);
 // Eigen system of a reversible Q with weights pi: Q = L diag(lam) R with
 // L = D^-1/2 V, R = V^T D^1/2 (D = diag(pi)).
 bool reversible_eigen(int n, const double* Q, const double* pi, double* lam, double* L,
