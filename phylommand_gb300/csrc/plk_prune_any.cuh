@@ -459,7 +459,10 @@ __global__ void __launch_bounds__(256) prune_any_kernel(PruneArgs a, AnyLaunch p
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             acc[r] = s1 == kSrcNone ? d0[r] : (EXACT ? mul_rn(d0[r], d1[r]) : d0[r] * d1[r]);
-            mx = fmax(mx, acc[r]);
+            // for the node states by magnitude: where rounding noise of P(0) is all a
+            // vector has, its larger entries may be negative, and scaled by the
+            // largest positive one they would overflow in the output
+            mx = fmax(mx, kNodes ? fabs(acc[r]) : acc[r]);
         }
         // ---- per-site power-of-two scaling (exact)
         const unsigned high = __ballot_sync(0xffffffffu, mx >= scale_threshold<T>());
@@ -640,11 +643,11 @@ __global__ void __launch_bounds__(256) down_any_kernel(PreorderArgs a, AnyLaunch
 #pragma unroll
         for (int r = 0; r < R; ++r) d[r] = src[row_of(r)];
     };
-    // x's rescale, as in prune_any_kernel
+    // x's rescale, as in prune_any_kernel's node passes
     auto rescale = [&](T (&x)[R]) {
         T mx = T(0);
 #pragma unroll
-        for (int r = 0; r < R; ++r) mx = fmax(mx, x[r]);
+        for (int r = 0; r < R; ++r) mx = fmax(mx, fabs(x[r]));
         const unsigned high = __ballot_sync(0xffffffffu, mx >= scale_threshold<T>());
         if (__any_sync(0xffffffffu, (high & site_mask) == 0u)) {
             T top = mx;
