@@ -10,6 +10,7 @@ namespace {
 
 constexpr size_t kAnySmem = 227 * 1024;  // of a CTA, the kernel's static bytes among them
 constexpr int kAnyWarps = 8;  // per CTA at most
+constexpr double kStoredBytes = 8e9;  // of vectors stored for node states where that is faster
 
 int any_sm_count() {
     static std::atomic<int> n{0};
@@ -30,9 +31,11 @@ struct AnyPlan {
 };
 
 // H, warps per CTA and the tables' place for these counts; H = 0 where
-// nothing fits.  smem(H, launch): the dynamic bytes of a CTA, fixed: its static ones.
+// nothing fits.  smem(H, launch): the dynamic bytes of a CTA, fixed: its static
+// ones; writes: the pass writes node states (NodeOut).
 template <class Smem>
-AnyPlan any_plan(int S, int C, bool fp64, int n_sites, int n_codes, int max_depth, int sms, size_t fixed, Smem smem) {
+AnyPlan any_plan(int S, int C, bool fp64, int n_sites, int n_codes, int max_depth, int sms, size_t fixed, bool writes,
+                 Smem smem) {
     AnyPlan best;
     const int tsz = fp64 ? 8 : 4;
     for (int H = 1; H <= 4; H *= 2) {
@@ -67,12 +70,27 @@ AnyPlan any_plan(int S, int C, bool fp64, int n_sites, int n_codes, int max_dept
                 fits = smem(H, p.launch) <= kAnySmem - fixed;
             }
         if (!fits) continue;
-        // FP64: the SM's FP64 pipe takes 16 cycles a warp instruction; FP32:
-        // four schedulers; either against the latency of one warp's op
-        p.cost = fp64 ? std::max(16.0 * per_sm * R * 2 * S, 300.0 + 16.0 * R * 2 * S)
-                      : std::max((per_sm + 3) / 4 * (1.5 * R * S + 100.0), 200.0 + 2.0 * R * S + 5.0 * S);
         p.blocks = (int)((warps + p.launch.warps - 1) / p.launch.warps);
-        if (best.H == 0 || p.cost < best.cost) best = p;
+        const int load = (p.blocks + sms - 1) / sms * p.launch.warps;  // warps of the fullest SM, whole CTAs
+        if (fp64) {
+            // the SM's FP64 pipe takes 16 cycles a warp instruction: the fullest SM's
+            // warps (157 CTAs on 152 SMs are two on five of them) with what they
+            // issue besides, against the latency of one warp's dependent ones.
+            // By per_sm alone a last wave's rounding chose
+            // four lanes a category for 90,000 sites (4 states, C = 4, 7 taxa: 646
+            // us of conditional vectors, one lane 285).
+            const double op = 16.0 * R * 2 * S;
+            const double out = writes ? 16.0 * ((2 * C + 12) * ((W * S + 31) / 32) + S) : 0.0;
+            const int beside = std::max(1, (int)((kAnySmem + 1024) / (smem(H, p.launch) + fixed + 1024)));  // CTAs an SM holds
+            const int rounds = (p.blocks + beside * sms - 1) / (beside * sms);
+            p.cost = std::max(rounds * (500.0 + 6.0 * op + out), load * (op + 100.0 + out));
+        } else {
+            // four schedulers, against the latency of one warp's op
+            p.cost = std::max((per_sm + 3) / 4 * (1.5 * R * S + 100.0), 200.0 + 2.0 * R * S + 5.0 * S);
+        }
+        // more lanes a site: while the SM's one CTA holds them all, else for a clear
+        // gain only (they cost instructions that are not counted)
+        if (best.H == 0 || p.cost < (fp64 ? (load <= kAnyWarps ? 1.15 : 0.95) : 1.0) * best.cost) best = p;
     }
     return best;
 }
@@ -80,7 +98,7 @@ AnyPlan any_plan(int S, int C, bool fp64, int n_sites, int n_codes, int max_dept
 // node_pass: a pass for the node states (of conditional vectors, or of messages)
 AnyPlan up_plan(const PruneArgs& a, int S, bool fp64, bool node_pass, bool cond_nodes, int sms) {
     return any_plan(S, a.C, fp64, a.n_sites, a.n_codes, a.max_depth, sms,
-                    dev::kSumStatic + (node_pass ? dev::kWeightStatic : 0),
+                    dev::kSumStatic + (node_pass ? dev::kWeightStatic : 0), cond_nodes,
                     [&](int H, dev::AnyLaunch p) {
                         static double some;
                         p.nodes = cond_nodes ? &some : nullptr;  // only its presence counts
@@ -88,7 +106,7 @@ AnyPlan up_plan(const PruneArgs& a, int S, bool fp64, bool node_pass, bool cond_
                     });
 }
 AnyPlan down_plan(const PreorderArgs& a, int S, bool fp64, int sms) {
-    return any_plan(S, a.C, fp64, a.n_sites, a.n_codes, 0, sms, dev::kWeightStatic,
+    return any_plan(S, a.C, fp64, a.n_sites, a.n_codes, 0, sms, dev::kWeightStatic, true,
                     [&](int H, const dev::AnyLaunch& p) { return dev::any_down_smem(S, H, fp64, p, a); });
 }
 
@@ -108,13 +126,29 @@ int prune_any_blocks(const PruneArgs& a, int S, int precision, bool nodes, bool 
         if (down_plan(d, S, fp64, sms).H == 0) return 0;
     }
     if (S == 4 && a.C <= 8 && !nodes) {
-        // prune4_kernel, a thread per site in 128-thread CTAs, issues the same
-        // FP64 instructions (32 per category and op) with less around them: it
-        // stays once its CTAs fill the SMs as evenly
-        const long long blocks = (a.n_sites + 127) / 128;
-        const double cost4 = (double)((blocks + sms - 1) / sms) * 4 * 16.0 * 32 * a.C;
-        if (p.cost > 0.9 * cost4) return 0;
+        // prune4_kernel, a thread per site in 128-thread CTAs (FP64 only: FP32 has
+        // other forms), issues the same FP64 instructions, 32 per category and op,
+        // with less around them once its CTAs fill the SMs.  Cycles an op of each,
+        // fitted to both over 4 to 50 taxa, 200 to 100,000 sites and 1 to 8
+        // categories (prune4_kernel pads those to 1, 4 or 8); `start`: what this
+        // kernel takes longer to start and end, in ops.  C = 1, 120 taxa x
+        // 30,625 sites: 332 us here and 411 there, 40,000 534 and 505.
+        const long long blocks4 = (a.n_sites + 127) / 128;
+        const double issue4 = (double)((blocks4 + sms - 1) / sms) * 4 * 16.0 * 32 * a.C;
+        const double cost4 = a.C == 1 ? 1.3 * issue4 + 1200.0 : (1.35 * issue4 + 1000.0 * a.C) * (a.C == 2 ? 1.2 : 1.0);
+        const double start = a.C / 8.0;
+        if ((a.n_ops + start) * 1.2 * p.cost > a.n_ops * cost4) return 0;
     }
+    // FP64 node states of few states: the output's divisions share the SM's FP64 pipe
+    // with the pass, and a CTA's few warps leave gaps.  Where the sites fill the SMs
+    // many times over, the kernels that store the vectors and normalise them after are
+    // faster: 4 states, 4 taxa x 100,000, C = 4, conditionals 240 us here and 216
+    // there, marginals 314 and 294; C = 8 439 and 317, 586 and 475.  At 16,000 sites
+    // (C = 4) 65 and 76, 79 and 100.  They hold all vectors, this pass none: up to 8 GB.
+    const double warps = (double)a.n_sites * a.C / 32 / sms;  // of an SM, a lane a category
+    if (fp64 && nodes && S <= 5 && a.C >= 4 && a.C <= 8 && 8.0 * a.n_ops * a.n_sites * a.C * S <= kStoredBytes &&
+        (marginal ? warps > 40 && a.n_ops <= 12 : warps > 20))
+        return 0;
     return p.blocks;
 }
 
