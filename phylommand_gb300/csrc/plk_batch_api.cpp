@@ -76,7 +76,7 @@ struct UnitSet {
 // Plan of NNI scoring or of the branch-length derivatives (plk_nni.cu) for
 // the current layout: warps per CTA, the units whose item's tables do not fit
 // in shared memory first, the records and the CTAs that fold them.  Items whose
-// records together pass kRecordBytes go in several groups, one after another
+// records together pass record_bytes() go in several groups, one after another
 // over the same records.
 struct DownGroup {
     int unit0, unit1, block0, block1;
@@ -133,9 +133,14 @@ struct plk_batch {
     // and plk_batch_nni_loglik (2, 3), and their elapsed times
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     double last_ms[2] = {0.0, 0.0};
+    // the down kernel of the items whose tables are in shared memory runs beside that
+    // of the others: its stream, begin and end
+    cudaStream_t beside = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
     ~plk_batch() {
-        for (cudaEvent_t e : ev)
+        for (cudaEvent_t e : {ev[0], ev[1], ev[2], ev[3], fork, join})
             if (e) cudaEventDestroy(e);
+        if (beside) cudaStreamDestroy(beside);
         if (exec) cudaGraphExecDestroy(exec);
         if (h_model) cudaFreeHost(h_model);
         if (h_lnl) cudaFreeHost(h_lnl);
@@ -329,7 +334,7 @@ plk_status build_layout(plk_batch* b) {
         }
     if (!stream_ok) b->d_stream.release();
     PLK_BCUDA(b, b->d_lnl.ensure(it.size() * sizeof(double)), "allocate lnL");
-    PLK_BCUDA(b, b->d_counter.ensure(sizeof(int)), "allocate counter");
+    PLK_BCUDA(b, b->d_counter.ensure(2 * sizeof(int)), "allocate counter");
     PLK_BCUDA(b, b->d_kids.ensure(kids.size() * sizeof(int4)), "allocate node table");
     PLK_BCUDA(b, cudaMemcpy(b->d_items.p, it.data(), it.size() * sizeof(BatchItemDev), cudaMemcpyHostToDevice), "upload table");
     size_t off = 0;
@@ -962,7 +967,10 @@ namespace {
 constexpr size_t kSmemLimit = 227 * 1024;
 // A record takes 16 bytes per output and warp tile, up to four times the tip codes
 // of its item: a batch whose codes fit has to fit with them.
-constexpr size_t kRecordBytes = (size_t)8 << 30;
+size_t record_bytes() {
+    const char* e = getenv("PLK_BATCH_RECORD_BYTES");
+    return e ? (size_t)std::max(0ll, atoll(e)) : (size_t)8 << 30;
+}
 
 // The trees NNI scoring and the derivatives take: those whose op list and
 // spill stack (of a staged tile of 128 sites) fit in a CTA's shared memory.
@@ -1024,8 +1032,7 @@ plk_status plan_down(plk_batch* b, DownPlan& p, bool blen) {
     p.n_far = 0;
     p.n_records = 1;
     p.groups.clear();
-    size_t most = kRecordBytes;
-    if (const char* e = getenv("PLK_BATCH_RECORD_BYTES")) most = (size_t)std::max(0ll, atoll(e));
+    const size_t most = record_bytes();
     long long records = 0;
     const int tile = z.warps * W;
     for (int k = 0; k < n_items; ++k) {
@@ -1071,9 +1078,6 @@ plk_status enqueue_down(plk_batch* b, bool blen) {
     plk_status s = plan_down(b, p, blen);
     if (s != PLK_OK) return s;
     const size_t KP = (b->C + 1) / 2, W = down_sites_per_warp(b->C), n_items = b->items.size();
-    const size_t gw = (size_t)std::max(p.grid_near, p.grid_far) * p.size.warps;
-    PLK_BCUDA(b, b->d_scr.ensure(gw * b->max_int * 128 * sizeof(float4)), "allocate scratch");
-    PLK_BCUDA(b, b->d_scr_e.ensure(gw * b->max_int * 2 * W * sizeof(int)), "allocate scratch");
     PLK_BCUDA(b, b->d_Pn.ensure((size_t)b->n_nodes_total * KP * 32 * sizeof(float)), "allocate P");
     PLK_BCUDA(b, b->d_tipn.ensure((size_t)b->tips_total * KP * 128 * sizeof(float)), "allocate tip tables");
     PLK_BCUDA(b, b->d_records.ensure(p.n_records * sizeof(float4)), "allocate records");
@@ -1086,6 +1090,25 @@ plk_status enqueue_down(plk_batch* b, bool blen) {
     } else {
         PLK_BCUDA(b, b->d_nni_out.ensure((size_t)p.total_out * sizeof(double)), "allocate NNI output");
     }
+    // Items that read their tables through L1 and the others are two launches.  Each
+    // lasts as long as its longest tree's chain, so they run side by side (25 items
+    // of up to 487 taxa, C = 1: derivatives 2430 us in turn, 1800 side by side), the first
+    // of them first; in turn where their scratch does not fit at once.
+    const size_t far = (size_t)p.grid_far * p.size.warps * b->max_int, near = (size_t)p.grid_near * p.size.warps * p.size.ints;
+    bool together = far > 0 && near > 0 && (far + near) * 128 * sizeof(float4) <= record_bytes();
+    for (;; together = false) {
+        const size_t n = together ? far + near : std::max(far, near);
+        cudaError_t e = b->d_scr.ensure(n * 128 * sizeof(float4));
+        if (e == cudaSuccess) e = b->d_scr_e.ensure(n * 2 * W * sizeof(int));
+        if (e == cudaSuccess) break;
+        if (!together) PLK_BCUDA(b, e, "allocate scratch");
+        cudaGetLastError();
+    }
+    if (together) {
+        if (!b->beside) PLK_BCUDA(b, cudaStreamCreateWithFlags(&b->beside, cudaStreamNonBlocking), "cudaStreamCreate");
+        for (cudaEvent_t* e : {&b->fork, &b->join})
+            if (!*e) PLK_BCUDA(b, cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate");
+    }
     BatchDev d = device_view(b, b->lnl_units);
     d.units = p.units.as<int2>();
     d.n_units = p.n_units;
@@ -1095,22 +1118,33 @@ plk_status enqueue_down(plk_batch* b, bool blen) {
     d.records = b->d_records.as<float4>();
     d.rec_off = p.rec_off.as<long long>();
     d.nni_out = b->d_nni_out.as<double>();
-    d.scratch_int = b->max_int;
-    d.scr = b->d_scr.as<float4>();
-    d.scr_e = b->d_scr_e.as<int>();
     PLK_BCUDA(b, cudaMemcpyAsync(b->d_model.p, b->h_model, n_items * batch_model_stride(b->C) * sizeof(double),
                                  cudaMemcpyHostToDevice, b->stream), "upload models");
     PLK_BCUDA(b, launch_down_tables(d, bd, b->stream), "batch tables launch");
     for (const DownGroup& g : p.groups) {
-        // its units that read their tables through L1, then the others
+        // its units that read their tables through L1, and the others
         const int cut = std::min(std::max(p.n_far, g.unit0), g.unit1);
-        for (const bool near : {false, true}) {
-            const int u0 = near ? cut : g.unit0, u1 = near ? g.unit1 : cut;
+        const bool both = together && g.unit0 < cut && cut < g.unit1;
+        PLK_BCUDA(b, cudaMemsetAsync(b->d_counter.p, 0, 2 * sizeof(int), b->stream), "clear work queues");
+        if (both) {
+            PLK_BCUDA(b, cudaEventRecord(b->fork, b->stream), "cudaEventRecord");
+            PLK_BCUDA(b, cudaStreamWaitEvent(b->beside, b->fork, 0), "cudaStreamWaitEvent");
+        }
+        for (const bool near_ones : {false, true}) {
+            const int u0 = near_ones ? cut : g.unit0, u1 = near_ones ? g.unit1 : cut;
             if (u0 == u1) continue;
-            PLK_BCUDA(b, cudaMemsetAsync(b->d_counter.p, 0, sizeof(int), b->stream), "clear work queue");
-            PLK_BCUDA(b, launch_down(d, bd, blen, near, p.size, u0, u1, std::min(near ? p.grid_near : p.grid_far, u1 - u0),
-                                     b->stream),
+            const size_t at = near_ones && both ? far : 0;  // ranks of all warps before its scratch
+            d.counter = b->d_counter.as<int>() + (near_ones ? 1 : 0);
+            d.scratch_int = near_ones ? p.size.ints : b->max_int;
+            d.scr = b->d_scr.as<float4>() + at * 128;
+            d.scr_e = b->d_scr_e.as<int>() + at * 2 * W;
+            const int grid = std::min(near_ones ? p.grid_near : p.grid_far, u1 - u0);
+            PLK_BCUDA(b, launch_down(d, bd, blen, near_ones, p.size, u0, u1, grid, near_ones && both ? b->beside : b->stream),
                       "pre-order kernel launch");
+        }
+        if (both) {
+            PLK_BCUDA(b, cudaEventRecord(b->join, b->beside), "cudaEventRecord");
+            PLK_BCUDA(b, cudaStreamWaitEvent(b->stream, b->join, 0), "cudaStreamWaitEvent");
         }
         d.reduce_blocks = p.blocks.as<int2>() + g.block0;
         PLK_BCUDA(b, launch_down_reduce(d, bd, blen, g.block1 - g.block0, b->stream), "record fold launch");
