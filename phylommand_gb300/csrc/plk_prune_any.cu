@@ -110,6 +110,33 @@ AnyPlan down_plan(const PreorderArgs& a, int S, bool fp64, int sms) {
                     [&](int H, const dev::AnyLaunch& p) { return dev::any_down_smem(S, H, fp64, p, a); });
 }
 
+// Whether the kernels that store every vector (a thread per site; node states are
+// normalised or formed by further kernels) are faster: where many sites meet few
+// ops or many idle lanes (11 categories leave a third), a warp's start, its sums and
+// its idle lanes here cost more than the vectors' way through L2.  Both times in
+// microseconds, fitted to 3 to 30 taxa, 5,000 to 100,000 sites, 2 to 24 states and 1
+// to 16 categories; FP32 up to 5 taxa, as this kernel is faster above.  lnL, FP64, 3
+// taxa x 100,000, 2 states, C = 11: 288 us here and 93 there; 9 states, C = 9, 1,212
+// and 495; 10 taxa x 100,000, 5 states, C = 4, 449 and 478.  By this rule the
+// mean over all those shapes is 0.6 % (node states 0.8) above the better of the two, by
+// this kernel alone 7 (16).  They hold all vectors, this pass none: up to 8 GB.
+bool stored_faster(const PruneArgs& a, int S, bool fp64, int kind, const AnyPlan& up, const AnyPlan* down, int sms) {
+    // [FP32, FP64][lnL, conditionals, marginals]: here: start, the plan's cost, warps,
+    // warps x ops x states; there: start, latency of an op and of a product, issue of both
+    static constexpr double kFit[2][3][9] = {
+        {{21, 1.2, 0.37, 0.071, 32, 0.78, 3.6, 3.1, 1.2}, {50, 1.4, 0.28, 0.31, 68, 0, 0, 16, 2.8}, {53, 0.98, 0.26, 0.49, 69, 0.64, 3.5, 25, 3.6}},
+        {{21, 0.35, 0.38, 0.31, 31, 0.99, 4.9, 6.2, 6.6}, {37, 0.42, 0.41, 0.39, 54, 0.74, 4.3, 16, 8.4}, {43, 0.33, 0.56, 0.65, 50, 2, 13, 22, 10}}};
+    const double stored = (fp64 ? 8.0 : 4.0) * (kind == 2 ? 2 : 1) * a.n_ops * a.n_sites * a.C * S;
+    if (stored > kStoredBytes || a.n_sites < 64 * sms || (!fp64 && a.n_ops > 4)) return false;
+    const double* f = kFit[fp64][kind];
+    const double ops = a.n_ops, products = a.n_ops - 1;
+    const double load = (up.blocks + sms - 1) / sms * up.launch.warps;
+    const double here = f[0] + f[1] * ops * (up.cost + (down ? down->cost : 0.0)) / 1e3 + f[2] * load + f[3] * ops * load * S / 10;
+    const double x = ((a.n_sites + 127) / 128 + sms - 1) / sms * a.C, SS = S * S / 100.0;
+    const double there = f[4] + f[5] * ops * a.C + f[6] * products * a.C * SS + f[7] * ops * x * S / 100 + f[8] * products * x * SS;
+    return here > 1.05 * there;
+}
+
 }  // namespace
 
 int prune_any_blocks(const PruneArgs& a, int S, int precision, bool nodes, bool marginal) {
@@ -119,11 +146,13 @@ int prune_any_blocks(const PruneArgs& a, int S, int precision, bool nodes, bool 
     const int sms = any_sm_count();
     const AnyPlan p = up_plan(a, S, fp64, nodes, nodes && !marginal, sms);
     if (p.H == 0) return 0;
+    AnyPlan down;
     if (marginal) {
         PreorderArgs d{};
         d.n_int = a.n_int; d.n_tips = a.n_tips; d.n_nodes = a.n_nodes; d.n_sites = a.n_sites; d.n_codes = a.n_codes;
         d.C = a.C;
-        if (down_plan(d, S, fp64, sms).H == 0) return 0;
+        down = down_plan(d, S, fp64, sms);
+        if (down.H == 0) return 0;
     }
     if (S == 4 && a.C <= 8 && !nodes) {
         // prune4_kernel, a thread per site in 128-thread CTAs (FP64 only: FP32 has
@@ -139,16 +168,15 @@ int prune_any_blocks(const PruneArgs& a, int S, int precision, bool nodes, bool 
         const double start = a.C / 8.0;
         if ((a.n_ops + start) * 1.2 * p.cost > a.n_ops * cost4) return 0;
     }
-    // FP64 node states of few states: the output's divisions share the SM's FP64 pipe
-    // with the pass, and a CTA's few warps leave gaps.  Where the sites fill the SMs
-    // many times over, the kernels that store the vectors and normalise them after are
-    // faster: 4 states, 4 taxa x 100,000, C = 4, conditionals 240 us here and 216
-    // there, marginals 314 and 294; C = 8 439 and 317, 586 and 475.  At 16,000 sites
-    // (C = 4) 65 and 76, 79 and 100.  They hold all vectors, this pass none: up to 8 GB.
+    // the stored forms of 4 states (prune4_kernel), up to 8 categories, padded to 4 or 8:
+    // 4 taxa x 100,000, C = 4, conditionals 240 us here and 216 there, marginals 314 and
+    // 294; C = 8 439 and 317, 586 and 475.  At 16,000 sites (C = 4) 65 and 76, 79 and 100
     const double warps = (double)a.n_sites * a.C / 32 / sms;  // of an SM, a lane a category
-    if (fp64 && nodes && S <= 5 && a.C >= 4 && a.C <= 8 && 8.0 * a.n_ops * a.n_sites * a.C * S <= kStoredBytes &&
+    if (fp64 && nodes && S == 4 && a.C >= 4 && a.C <= 8 && 8.0 * a.n_ops * a.n_sites * a.C * S <= kStoredBytes &&
         (marginal ? warps > 40 && a.n_ops <= 12 : warps > 20))
         return 0;
+    if (S != 4 || a.C > 8 || nodes)
+        if (stored_faster(a, S, fp64, nodes ? (marginal ? 2 : 1) : 0, p, down.H ? &down : nullptr, sms)) return 0;
     return p.blocks;
 }
 

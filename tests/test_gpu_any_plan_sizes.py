@@ -32,3 +32,25 @@ def test_few_states_many_sites(S, C, n_tips, n_sites):
             got = h.node_states(mode, plk.PLK_FP64)
             np.testing.assert_allclose(got[:, some], want, rtol=0, atol=tol)
             assert np.abs(got.sum(axis=-1) - 1.0).max() <= 1e-13
+
+
+@pytest.mark.parametrize("S, C, n_tips", [(2, 11, 3), (2, 5, 9), (3, 7, 3), (5, 6, 2), (9, 9, 4), (12, 2, 3), (20, 12, 3), (24, 1, 5)])
+@pytest.mark.parametrize("n_sites", [9727, 9728, 30001])
+def test_stored_or_not(S, C, n_tips, n_sites):
+    """Where the kernels that store the vectors take over: more categories, few taxa.
+    FP32 rounds each of the ~2 S operations of n ops at 2^-24, so a site of these
+    trees is within 9 * 2 * 24 * 6e-8 = 2.6e-5 of its likelihood (a marginal twice)."""
+    rng = np.random.default_rng(S * 100 + C * 10 + n_tips)
+    left, right, bl, masks, Q, f, cr, cw = _random_case(rng, n_tips, n_sites, S=S, C=C)
+    some = np.unique(np.r_[0, 31, n_sites - 1, rng.integers(0, n_sites, 12)])
+    teff = plk.effective_lengths(left, right, bl, False)
+    orc = O.loglik(left, right, masks[:, some], teff, Q, f, cr, cw, p_mode=O.P_TAYLOR20,
+                   want_cond_norm=True, want_marginal=True)
+    with _engine(left, right, bl, masks, S, Q, f, cr, cw, p_mode=plk.PLK_P_TAYLOR20) as h:
+        for precision, rel, tol in ((plk.PLK_FP64, 1e-14, 1e-13), (plk.PLK_FP32S, 0.0, 2.6e-5)):
+            lnl, site = h.loglik(precision), h.site_loglik()
+            np.testing.assert_allclose(site[some], orc.site_lnl, rtol=rel, atol=max(1e-14, tol if rel == 0.0 else 0.0))
+            assert lnl == pytest.approx(np.sum(site.astype(np.longdouble)), rel=1e-7 if rel == 0.0 else 1e-13)
+            for mode, want, k in ((plk.PLK_NODES_COND, orc.cond_norm, 1), (plk.PLK_NODES_MARGINAL, orc.marginal, 10 if rel else 2)):
+                got = h.node_states(mode, precision)
+                np.testing.assert_allclose(got[:, some], want, rtol=0, atol=k * tol)
