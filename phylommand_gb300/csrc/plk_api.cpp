@@ -578,8 +578,17 @@ plk_status run_prune(plk_handle* h, int precision, NodePass* store, cudaEvent_t*
     }
     const size_t tsz = precision == PLK_FP64 ? sizeof(double) : sizeof(float);
     const size_t vec_bytes = (size_t)h->post.size() * h->C * h->n_sites * h->S * tsz;
-    const int any_blocks =
-        prune_any_blocks(prune_args(h, precision), h->S, precision, store != nullptr, store && store->marginal);
+    const bool marginal = store && store->marginal, fused = fused_kernel_applies(h, precision);
+    int any_blocks = prune_any_blocks(prune_args(h, precision), h->S, precision, store != nullptr, marginal, true);
+    if (any_blocks == 0) {
+        // chosen for speed: not where the vectors cannot be allocated
+        const int without = prune_any_blocks(prune_args(h, precision), h->S, precision, store != nullptr, marginal, false);
+        if (without > 0 && ((fused && store ? h->d_cond : h->d_work).ensure(vec_bytes) != cudaSuccess ||
+                            (marginal && h->d_outside.ensure(vec_bytes) != cudaSuccess))) {
+            cudaGetLastError();
+            any_blocks = without;
+        }
+    }
     // the smallest tile elsewhere: 64 sites (prune4p, two threads per site)
     const int blocks = std::max((h->n_sites + 63) / 64, any_blocks);
     PLK_CUDA(h, h->d_site_lnl.ensure(sizeof(double) * h->n_sites), "allocate site lnL");
@@ -606,7 +615,6 @@ plk_status run_prune(plk_handle* h, int precision, NodePass* store, cudaEvent_t*
     a.withhold_arrival = (precision == PLK_FP32S && (h->withhold_stage || h->withhold_arrival)) ? 1 : 0;
     if (precision == PLK_FP32S) h->withhold_stage = h->withhold_arrival = false;
     a.use_any = any_blocks > 0 ? 1 : 0;
-    const bool fused = fused_kernel_applies(h, precision);
     std::vector<int> cands20;
     if (!store && precision == PLK_FP32S && h->S == 20)
         for (int v = 1; v <= 4; ++v)

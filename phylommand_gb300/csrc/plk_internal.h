@@ -366,8 +366,9 @@ cudaError_t launch_prune4s(const PruneArgs& a, int spt, int* n_blocks, cudaStrea
 // another kernel does (the tuned FP32 forms; 4 states once a thread per site
 // fills the chip; shapes whose matrices do not fit in shared memory).
 // nodes: a node-state pass, which it takes wherever its tables fit (with the
-// pre-order pass after it, where `marginal`).
-int prune_any_blocks(const PruneArgs& a, int S, int precision, bool nodes, bool marginal = false);
+// pre-order pass after it, where `marginal`).  may_store: 0 also where the kernels
+// that store every vector are estimated faster.
+int prune_any_blocks(const PruneArgs& a, int S, int precision, bool nodes, bool marginal, bool may_store);
 cudaError_t launch_prune_any(const PruneArgs& a, int S, int precision, int* n_blocks, cudaStream_t st);
 // Chooses the kernel for (S, C, precision); returns the number of blocks used
 // for the partial sums in *n_blocks.

@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cstdlib>
 
 namespace plk {
 
@@ -10,7 +11,12 @@ namespace {
 
 constexpr size_t kAnySmem = 227 * 1024;  // of a CTA, the kernel's static bytes among them
 constexpr int kAnyWarps = 8;  // per CTA at most
-constexpr double kStoredBytes = 8e9;  // of vectors stored for node states where that is faster
+
+// of vectors stored where that is faster
+double stored_limit() {
+    const char* e = getenv("PLK_STORED_BYTES");
+    return e ? atof(e) : 8e9;
+}
 
 int any_sm_count() {
     static std::atomic<int> n{0};
@@ -127,7 +133,7 @@ bool stored_faster(const PruneArgs& a, int S, bool fp64, int kind, const AnyPlan
         {{21, 1.2, 0.37, 0.071, 32, 0.78, 3.6, 3.1, 1.2}, {50, 1.4, 0.28, 0.31, 68, 0, 0, 16, 2.8}, {53, 0.98, 0.26, 0.49, 69, 0.64, 3.5, 25, 3.6}},
         {{21, 0.35, 0.38, 0.31, 31, 0.99, 4.9, 6.2, 6.6}, {37, 0.42, 0.41, 0.39, 54, 0.74, 4.3, 16, 8.4}, {43, 0.33, 0.56, 0.65, 50, 2, 13, 22, 10}}};
     const double stored = (fp64 ? 8.0 : 4.0) * (kind == 2 ? 2 : 1) * a.n_ops * a.n_sites * a.C * S;
-    if (stored > kStoredBytes || a.n_sites < 64 * sms || (!fp64 && a.n_ops > 4)) return false;
+    if (stored > stored_limit() || a.n_sites < 64 * sms || (!fp64 && a.n_ops > 4)) return false;
     const double* f = kFit[fp64][kind];
     const double ops = a.n_ops, products = a.n_ops - 1;
     const double load = (up.blocks + sms - 1) / sms * up.launch.warps;
@@ -139,7 +145,7 @@ bool stored_faster(const PruneArgs& a, int S, bool fp64, int kind, const AnyPlan
 
 }  // namespace
 
-int prune_any_blocks(const PruneArgs& a, int S, int precision, bool nodes, bool marginal) {
+int prune_any_blocks(const PruneArgs& a, int S, int precision, bool nodes, bool marginal, bool may_store) {
     const bool fp64 = precision == PLK_FP64;
     if (S < 2 || S > kMaxStates || a.C > kMaxCats || a.n_ops < 1) return 0;
     if (!fp64 && !nodes && ((S == 4 && a.C <= 8) || S == 20)) return 0;  // the tuned FP32 forms
@@ -168,11 +174,12 @@ int prune_any_blocks(const PruneArgs& a, int S, int precision, bool nodes, bool 
         const double start = a.C / 8.0;
         if ((a.n_ops + start) * 1.2 * p.cost > a.n_ops * cost4) return 0;
     }
+    if (!may_store) return p.blocks;
     // the stored forms of 4 states (prune4_kernel), up to 8 categories, padded to 4 or 8:
     // 4 taxa x 100,000, C = 4, conditionals 240 us here and 216 there, marginals 314 and
     // 294; C = 8 439 and 317, 586 and 475.  At 16,000 sites (C = 4) 65 and 76, 79 and 100
     const double warps = (double)a.n_sites * a.C / 32 / sms;  // of an SM, a lane a category
-    if (fp64 && nodes && S == 4 && a.C >= 4 && a.C <= 8 && 8.0 * a.n_ops * a.n_sites * a.C * S <= kStoredBytes &&
+    if (fp64 && nodes && S == 4 && a.C >= 4 && a.C <= 8 && 8.0 * a.n_ops * a.n_sites * a.C * S <= stored_limit() &&
         (marginal ? warps > 40 && a.n_ops <= 12 : warps > 20))
         return 0;
     if (S != 4 || a.C > 8 || nodes)
