@@ -182,6 +182,12 @@ int prune_any_blocks(const PruneArgs& a, int S, int precision, bool nodes, bool 
     if (fp64 && nodes && S == 4 && a.C >= 4 && a.C <= 8 && 8.0 * a.n_ops * a.n_sites * a.C * S <= stored_limit() &&
         (marginal ? warps > 40 && a.n_ops <= 12 : warps > 20))
         return 0;
+    // FP32 conditionals of one category: a long chain of ops with the output's division
+    // in each, 900 taxa x 50 961 us here and 802 there, x 500 1,044 and 881, x 3,000 1,438
+    // and 1,564; 300 taxa level
+    if (!fp64 && nodes && !marginal && S == 4 && a.C == 1 && a.n_ops > 300 && a.n_sites <= 8 * sms &&
+        4.0 * a.n_ops * a.n_sites * S <= stored_limit())
+        return 0;
     if (S != 4 || a.C > 8 || nodes)
         if (stored_faster(a, S, fp64, nodes ? (marginal ? 2 : 1) : 0, p, down.H ? &down : nullptr, sms)) return 0;
     return p.blocks;
